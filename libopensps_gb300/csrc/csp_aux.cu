@@ -12,23 +12,35 @@
 
 namespace sps {
 
+// The largest batch whose weight operand takes a CTA per model (run_weights_convert_sums).
+constexpr int WC_CTA_MODELS = 8192;
+
 // ---------------------------------------------------------------------------------------------- weights
 // The operand and, from the same FP64 weights, the FP64 sums of model_sums_zw (one warp per model, the sums in the
 // operand's column order; young ages by the column map's KMAP_YOUNG bit): the sums ride the FP64 pipe while the
 // conversion waits on memory, instead of a second pass over the weights bound by that pipe. Escaping-light columns
 // (KMAP_ION) carry the weight times the model's escaping fraction clamp(frac_obrun, 0, 1) (nebular_kernels step 2,
 // OpenSPS src/physics/opensps_csp_batch.f90:2726-2750, with fesc of batch_nebular_indices :1696) and join no sum.
-template <bool PARTS>
-__global__ void __launch_bounds__(256) weights_convert_sums_kernel(WeightsArgs a) {
-    const int m = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (m >= a.n_models) return;
+//
+// WPM warps share a model: one on large batches (the warps of the batch fill the GPU), the CTA's eight on small ones,
+// where a lane that walked 42 columns alone took 50 us of dependent loads whatever the batch (with eight warps 6.3 us
+// at one model and 15 at 1000).
+constexpr int WC_THREADS = 256, WC_WARPS = WC_THREADS / 32;
+
+template <bool PARTS, int WPM>
+__global__ void __launch_bounds__(WC_THREADS) weights_convert_sums_kernel(WeightsArgs a) {
+    constexpr int NSUM = PARTS ? 6 : 2;   // mass, L_bol; then mass young, old, L_bol young, old
+    const int m = (blockIdx.x * WC_WARPS + (threadIdx.x >> 5)) / WPM;
+    const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % WPM;
+    if (m >= a.n_models) return;          // (WPM = WC_WARPS: the whole CTA)
     const double *w = a.wz + (size_t)m * a.nt * a.nz;
     __nv_bfloat16 *hi = a.w_hi + (size_t)m * a.kpad, *lo = a.w_lo + (size_t)m * a.kpad;
-    double ms = 0.0, ls = 0.0, msy = 0.0, lsy = 0.0, mso = 0.0, lso = 0.0;
+    double s[NSUM];
+#pragma unroll
+    for (int i = 0; i < NSUM; ++i) s[i] = 0.0;
     const float fesc = a.mpar ? fminf(fmaxf(__ldg(a.mpar + (size_t)m * MODEL_PAR_FLOATS + MP_FO), 0.f), 1.f) : 0.f;
 #pragma unroll 4
-    for (int k = lane; k < a.kpad; k += 32) {
+    for (int k = part * 32 + lane; k < a.kpad; k += 32 * WPM) {
         const int code = __ldg(a.kmap + k);
         float wf = 0.f;
         if (code >= 0) {
@@ -39,11 +51,11 @@ __global__ void __launch_bounds__(256) weights_convert_sums_kernel(WeightsArgs a
                 wf *= fesc;
             } else if (__double_as_longlong(wv) > 0x0010000000000000LL) {   // wv > DBL_MIN (and not negative)
                 const double mk = __ldg(a.mass + idx), lk = __ldg(a.llin + idx);
-                ms = fma(wv, mk, ms);
-                ls = fma(wv, lk, ls);
-                if (PARTS) {
-                    if (code & KMAP_YOUNG) { msy = fma(wv, mk, msy); lsy = fma(wv, lk, lsy); }
-                    else { mso = fma(wv, mk, mso); lso = fma(wv, lk, lso); }
+                s[0] = fma(wv, mk, s[0]);
+                s[1] = fma(wv, lk, s[1]);
+                if constexpr (PARTS) {
+                    if (code & KMAP_YOUNG) { s[2] = fma(wv, mk, s[2]); s[4] = fma(wv, lk, s[4]); }
+                    else { s[3] = fma(wv, mk, s[3]); s[5] = fma(wv, lk, s[5]); }
                 }
             }
         }
@@ -52,28 +64,39 @@ __global__ void __launch_bounds__(256) weights_convert_sums_kernel(WeightsArgs a
         lo[k] = __float2bfloat16_rn(wf - __bfloat162float(h));
     }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        ms += __shfl_xor_sync(0xffffffffu, ms, off);
-        ls += __shfl_xor_sync(0xffffffffu, ls, off);
-        if (PARTS) {
-            msy += __shfl_xor_sync(0xffffffffu, msy, off);
-            lsy += __shfl_xor_sync(0xffffffffu, lsy, off);
-            mso += __shfl_xor_sync(0xffffffffu, mso, off);
-            lso += __shfl_xor_sync(0xffffffffu, lso, off);
+    for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+        for (int i = 0; i < NSUM; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
+    if constexpr (WPM > 1) {
+        __shared__ double part_sums[WC_WARPS][NSUM];
+        if (lane == 0)
+#pragma unroll
+            for (int i = 0; i < NSUM; ++i) part_sums[part][i] = s[i];
+        __syncthreads();
+        if (threadIdx.x < NSUM && a.sums) {
+            double v = 0.0;
+#pragma unroll
+            for (int p = 0; p < WPM; ++p) v += part_sums[p][threadIdx.x];
+            a.sums[(size_t)m * 6 + threadIdx.x] = v;
         }
-    }
-    if (lane == 0 && a.sums) {
+    } else if (lane == 0 && a.sums) {
         double *o = a.sums + (size_t)m * 6;
-        o[0] = ms; o[1] = ls;
-        if (PARTS) { o[2] = msy; o[3] = mso; o[4] = lsy; o[5] = lso; }
+#pragma unroll
+        for (int i = 0; i < NSUM; ++i) o[i] = s[i];
     }
+}
+
+template <bool PARTS>
+static void launch_weights_convert_sums(const WeightsArgs &a, cudaStream_t st) {
+    // a CTA per model up to the batch whose single warps would fill the SMs about once (152 x 8 CTAs of eight warps)
+    if (a.n_models <= WC_CTA_MODELS) weights_convert_sums_kernel<PARTS, WC_WARPS><<<a.n_models, WC_THREADS, 0, st>>>(a);
+    else weights_convert_sums_kernel<PARTS, 1><<<(a.n_models + WC_WARPS - 1) / WC_WARPS, WC_THREADS, 0, st>>>(a);
 }
 
 cudaError_t run_weights_convert_sums(const WeightsArgs &a, cudaStream_t st) {
     if (a.n_models <= 0) return cudaSuccess;
-    const int threads = 256, per_block = threads / 32, blocks = (a.n_models + per_block - 1) / per_block;
-    if (a.parts) weights_convert_sums_kernel<true><<<blocks, threads, 0, st>>>(a);
-    else weights_convert_sums_kernel<false><<<blocks, threads, 0, st>>>(a);
+    if (a.parts) launch_weights_convert_sums<true>(a, st);
+    else launch_weights_convert_sums<false>(a, st);
     return cudaGetLastError();
 }
 
