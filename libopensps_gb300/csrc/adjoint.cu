@@ -23,6 +23,7 @@
 #include <string>
 #include <vector>
 #include "context.h"
+#include "model_scalars.cuh"
 #include "sm103_ptx.cuh"
 
 namespace sps {
@@ -127,13 +128,13 @@ __global__ void __launch_bounds__(256) adjoint_prep_kernel(AdjointPrepArgs a) {
     for (int i = 0; i < AP_FLOATS; ++i) blk[i] = 0.f;
     const double z = pr[PF_ZRED];
     if (mp[MP_IGM_ON] != 0.f) {
-        const double pk[6] = {3.46, 1.68, 3.0 + 0.46, 1.5 + 0.18, 3.0 - 1.32, 1.68};
-        const double l1z = log1p(z);
+        // (1 + z)^p with p = 3.46 for k = 0 and 2, 1.68 for the others
+        const double l1z = log1p(z), inv = 1.0 / (1.0 + z), b0 = exp(3.46 * l1z), b1 = exp(1.68 * l1z);
+        const float f0 = (float)b0, f1 = (float)b1, g0 = (float)(3.46 * b0 * inv), g1 = (float)(1.68 * b1 * inv);
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
-            const double bk = exp(pk[k] * l1z);
-            blk[AP_B + k] = (float)bk;
-            blk[AP_DB + k] = (float)(pk[k] * bk / (1.0 + z));
+            blk[AP_B + k] = (k == 0 || k == 2) ? f0 : f1;
+            blk[AP_DB + k] = (k == 0 || k == 2) ? g0 : g1;
         }
     }
     const int R = __float_as_int(mp[MP_SMOOTH_R]);
@@ -160,7 +161,7 @@ __global__ void __launch_bounds__(256) adjoint_prep_kernel(AdjointPrepArgs a) {
         const int nsh = __float_as_int(zi.x) + ((zi.y > 0.f) ? 1 : 0);
         const double opz = 1.0 + z;
         kobs = -exp((double)nsh * a.dlnl) / (opz * opz * a.em1);
-        const int idx = max(0, min(find_interval0(a.zt, 500, z), 498));
+        const int idx = cosmology_interval(a.zt, z);
         const double slope = (a.dl[idx + 1] - a.dl[idx]) / (a.zt[idx + 1] - a.zt[idx]);
         const double dm = a.dl[idx] + slope * (z - a.zt[idx]);
         if (dm == dm && dm > SAFE_FLOOR) ddist = 5.0 / log(10.0) * slope / dm - 2.5 / (log(10.0) * opz);

@@ -8,100 +8,192 @@
 #include <vector>
 #include "context.h"
 #include "datalib.h"
+#include "model_scalars.cuh"
 
 namespace sps {
 
 // ---------------------------------------------------------------------------------------------- model params
 struct ModelParamArgs {
     int n, nspec, jtop, add_igm, smooth, i0;   // i0: the pixel whose smoothing row gives the model's taps
-    int mpw = 32;            // models per warp (1 .. 32)
+    int mpc = 32;            // models per CTA (1 .. 32)
     int dust_type = 0;       // the diffuse curve's scalars (MP_DUST_INDEX: its power, MP_CS1..: the tables' weights)
+    GridScalars grid;
     const double *par;       // PAR_DEVICE x n
     const float *igm_a;      // jtop x 6
     const double *lam;       // nspec
     const double *lnlam;     // nspec: ln lambda
     const double *zt, *dl;   // 500
-    double dlnl;
     float *mpar;             // n x MODEL_PAR_FLOATS
     float4 *zinfo;           // n: the observed-frame shift (band_gemm.cu)
     double *dist;            // n
 };
 
-// One thread per model for the FP64 scalars (GB300's FP64 rate is low: a warp instruction serves 32 models); the IGM
-// cap's search for the largest optical depth over the pixels below Lyman alpha is shared by the warp's lanes, model
-// after model.
-__global__ void __launch_bounds__(256) model_params_kernel(ModelParamArgs a) {
-    // a.mpw models per warp (lanes 0 .. mpw - 1): fewer than 32 when the batch is small, so that more warps share
-    // the cap searches
-    const int lane = threadIdx.x & 31;
-    const int m = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * a.mpw + lane;
-    const bool live = lane < a.mpw && m < a.n;
+// The velocity smoothing taps of one model: row i0 of build_velocity_kernel (src/spectra/opensps_smoothing.f90:
+// 553-633), normalised, offsets -4 .. 4; returns the half-width in pixels (-1: none).
+__device__ __forceinline__ int smoothing_taps(const ModelParamArgs &a, double sig, float *tap) {
+#pragma unroll
+    for (int d = 0; d < 9; ++d) tap[d] = 0.f;
+    if (!(a.smooth && sig > SAFE_FLOOR && a.i0 >= 0)) return -1;
+    const int n = a.nspec, i = a.i0;
+    const double sb = sig * (1.0 / (C_LIGHT * 1.0e-13)), inv2s2 = 0.5 / (sb * sb);
+    const double lli = __ldg(a.lnlam + i);
+    // the window in ln lambda: lambda_j vs lambda_i exp(-+4 sigma / c) compared as logarithms; il: first pixel >= vl,
+    // one lower when it lies above vl; ih: first pixel >= vh
+    const double vl = lli - 4.0 * sb, vh = lli + 4.0 * sb;
+    const int x = (int)(4.0 * sb * a.grid.inv_dlnl);
+    int il = min(lower_bound_from(a.lnlam, n, vl, i - x), n - 1);
+    if (il > 0 && __ldg(a.lnlam + il) > vl) il--;
+    int ih = min(lower_bound_from(a.lnlam, n, vh, i + x + 1), n - 1);
+    if (ih < il) ih = il;
+    if (!(ih - il + 1 >= 2 && i - il <= 4 && ih - i <= 4)) return -1;
+    // Gaussian weights / lambda_j times the trapezoid widths, normalised: the exponent is formed in FP64 (differences
+    // of ln lambda), the exponential and the normalisation in FP32 (the taps are stored so)
+    double lm[9], ll[9];
+#pragma unroll
+    for (int u = 0; u < 9; ++u) {
+        const int j = min(il + u, ih);
+        lm[u] = __ldg(a.lam + j);
+        ll[u] = __ldg(a.lnlam + j);
+    }
+    float w[9], tw = 0.f, dlft = 0.f;
+#pragma unroll
+    for (int u = 0; u < 9; ++u) {
+        const float drgt = (u < 8 && il + u < ih) ? (float)(lm[u < 8 ? u + 1 : 8] - lm[u]) : 0.f;
+        float wj = 0.f;
+        if (il + u <= ih) {
+            const double d = lli - ll[u];
+            wj = expf((float)(-inv2s2 * d * d)) / (float)lm[u] * 0.5f * (dlft + drgt);
+        }
+        w[u] = wj;
+        tw += wj;
+        dlft = drgt;
+    }
+    if (!(tw > 0.f)) return -1;
+    const float inv = 1.f / tw;
+#pragma unroll
+    for (int d = -4; d <= 4; ++d) {
+        const int u = i + d - il;
+        float v = 0.f;
+#pragma unroll
+        for (int q = 0; q < 9; ++q)
+            if (q == u && u <= ih - il) v = w[q] * inv;
+        tap[4 + d] = v;
+    }
+    return max(i - il, ih - i);
+}
+
+// A CTA of eight warps per mpc models. The FP64 scalars cost latency (the FP64 pipe takes a warp instruction every 64
+// cycles per SM sub-partition, whatever the lanes in use): warp 0 forms the models' IGM factors and later their dust
+// constants, warp 1 the smoothing taps, warp 2 the observed frame, one model per lane, side by side on three
+// sub-partitions. The IGM cap's search for the largest optical depth below Lyman alpha (apply_igm_z,
+// src/physics/opensps_csp_batch.f90:4272-4299: its first pixel) is shared by the CTA: each thread holds the wavelength
+// factors of its pixels in registers and takes the models in turn. With all of it on one thread per model, the table
+// staged in shared memory and the searches as bisections the kernel took 30 us at one model, 44 at 1000 and 168 at
+// 65536; now 7.8, 11.5 and 117.
+constexpr int MP_THREADS = 256, MP_WARPS = MP_THREADS / 32;
+constexpr int MP_PIX = 9;        // pixels per thread and pass: the 2218 below Lyman alpha in one pass
+
+__global__ void __launch_bounds__(MP_THREADS, 2) model_params_kernel(ModelParamArgs a) {
+    __shared__ __align__(16) float bsm[32][8];  // the redshift factors; [6]: 1 with IGM
+    __shared__ float red_t[MP_WARPS][32];
+    __shared__ int red_j[MP_WARPS][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int m0 = blockIdx.x * a.mpc, m = m0 + lane;
+    const bool live = lane < a.mpc && m < a.n;
     const double LOG2E = 1.4426950408889634;
     const double *p = a.par + (size_t)PAR_DEVICE * (live ? m : 0);
-    const double z = live ? p[PF_ZRED] : 0.0;
-    const bool igm = live && a.add_igm && z > SAFE_FLOOR && a.jtop > 0;
-    // redshift factors b_k = (1 + z)^p_k (igm_tau_z_terms, src/physics/opensps_cosmology.f90:497-508)
-    float b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    const double l1z = live ? log1p(z) : 0.0;   // (also the observed frame's shift below)
-    if (igm) {
-        // (1 + z)^p = 2^(p ln(1 + z) log2 e): the exponent formed and split in FP64 (x = n + r, |r| <= 1/2), 2^r
-        // by the SFU and 2^n exactly (the reference's exp_kp: FP64 argument, exponential at kernel precision; the
-        // factors are stored as FP32)
-        auto pw = [&](double pexp) {
-            const double x = pexp * l1z * LOG2E, n = rint(x);
-            float r;
-            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)(x - n)));
-            const int ni = (int)n;
-            return (ni > -126 && ni < 128) ? r * __int_as_float((ni + 127) << 23) : (float)exp(pexp * l1z);
-        };
-        b[0] = pw(3.46);
-        b[1] = pw(1.68);
-        b[2] = pw(3.0 + 0.46);
-        b[3] = pw(1.5 + 0.18);
-        b[4] = pw(3.0 - 1.32);
-        b[5] = b[1];
-    }
-    // the cap (apply_igm_z :4272-4299): the first pixel of the largest optical depth, searched by the whole warp for
-    // each of its models in turn, over the wavelength factors staged in shared memory (one array per factor)
-    extern __shared__ float4 sa4[];  // jtop float4 (factors 0..3), then jtop float2 (factors 4, 5)
+    float *o = a.mpar + (size_t)MODEL_PAR_FLOATS * (live ? m : 0);
     const int nj = a.add_igm ? a.jtop : 0;
-    float2 *sa2 = reinterpret_cast<float2 *>(sa4 + nj);
-    for (int j = threadIdx.x; j < nj; j += blockDim.x) {
-        const float *g = a.igm_a + 6 * (size_t)j;
-        sa4[j] = make_float4(g[0], g[1], g[2], g[3]);
-        sa2[j] = make_float2(g[4], g[5]);
+    red_t[warp][lane] = 0.f;
+    red_j[warp][lane] = 1;
+    float b[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    bool igm = false;
+    if (warp == 0) {
+        const double z = live ? p[PF_ZRED] : 0.0;
+        igm = live && a.add_igm && z > SAFE_FLOOR && a.jtop > 0;
+        // redshift factors b_k = (1 + z)^p_k (igm_tau_z_terms, src/physics/opensps_cosmology.f90:497-508; p = 3.46 for
+        // k = 0 and 2, 1.68 for the others)
+        if (igm) {
+            // (1 + z)^p = 2^(p ln(1 + z) log2 e): the exponent formed and split in FP64 (x = n + r, |r| <= 1/2), 2^r
+            // by the SFU and 2^n exactly (the reference's exp_kp: FP64 argument, exponential at kernel precision; the
+            // factors are stored as FP32)
+            const double l2z = log1p(z) * LOG2E;
+            auto pw = [&](double pexp) {
+                const double x = pexp * l2z, n = rint(x);
+                float r;
+                asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"((float)(x - n)));
+                const int ni = (int)n;
+                return (ni > -126 && ni < 128) ? r * __int_as_float((ni + 127) << 23) : (float)exp2(x);
+            };
+            b[0] = b[2] = pw(3.46);
+            b[1] = b[3] = b[4] = b[5] = pw(1.68);
+        }
+#pragma unroll
+        for (int k = 0; k < 6; ++k) bsm[lane][k] = b[k];
+        bsm[lane][6] = igm ? 1.f : 0.f;
+    } else if (warp == 1 && live) {
+        float tap[9];
+        const int R = smoothing_taps(a, p[PF_SIGMA_SMOOTH], tap);
+        float2 *o2 = reinterpret_cast<float2 *>(o);
+        o2[MP_SMOOTH_R / 2] = make_float2(__int_as_float(R), 0.f);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) o2[MP_TAPS / 2 + k] = make_float2(tap[2 * k], tap[2 * k + 1]);
+        o[MP_TAPS + 8] = tap[8];
+    } else if (warp == 2 && live) {
+        const double z = p[PF_ZRED];
+        float4 zi;
+        double dd;
+        observed_frame(z, log1p(z), a.grid, a.zt, a.dl, zi, dd);
+        a.zinfo[m] = zi;
+        a.dist[m] = dd;
     }
     __syncthreads();
-    float my_tmax = 0.f;
-    int my_jmax = 1;
-    const unsigned todo = __ballot_sync(0xffffffffu, igm);
-    for (int i = 0; i < a.mpw; ++i) {
-        if (!((todo >> i) & 1u)) continue;
-        float bb[6];
+    // the cap search
+    const int nm = min(a.mpc, a.n - m0);
+    for (int j0 = 0; j0 < nj; j0 += MP_PIX * MP_THREADS) {
+        float f[MP_PIX][6];
 #pragma unroll
-        for (int k = 0; k < 6; ++k) bb[k] = __shfl_sync(0xffffffffu, b[k], i);
-        float tmax = 0.f;
-        int jmax = 1;
-        for (int j = lane; j < nj; j += 32) {
-            const float4 f = sa4[j];
-            const float2 g = sa2[j];
-            const float t = f.x * bb[0] + f.y * bb[1] + f.z * bb[2] + f.w * bb[3] + g.x * bb[4] + g.y * bb[5];
-            if (t > tmax) { tmax = t; jmax = j + 1; }
-        }
+        for (int i = 0; i < MP_PIX; ++i) {
+            const int j = j0 + i * MP_THREADS + threadIdx.x;
+            const float2 *g = reinterpret_cast<const float2 *>(a.igm_a + 6 * (size_t)j);
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const float t2 = __shfl_xor_sync(0xffffffffu, tmax, off);
-            const int j2 = __shfl_xor_sync(0xffffffffu, jmax, off);
-            if (t2 > tmax || (t2 == tmax && j2 < jmax)) { tmax = t2; jmax = j2; }
+            for (int k = 0; k < 3; ++k) {
+                const float2 v = j < nj ? __ldg(g + k) : make_float2(0.f, 0.f);
+                f[i][2 * k] = v.x;
+                f[i][2 * k + 1] = v.y;
+            }
         }
-        if (lane == i) { my_tmax = tmax; my_jmax = tmax > 0.f ? jmax : 1; }
+        for (int i = 0; i < nm; ++i) {
+            const float4 b0 = *reinterpret_cast<const float4 *>(&bsm[i][0]), b1 = *reinterpret_cast<const float4 *>(&bsm[i][4]);
+            if (b1.z == 0.f) continue;
+            float tmax = 0.f;
+            int jmax = 0x7fffffff;
+#pragma unroll
+            for (int q = 0; q < MP_PIX; ++q) {
+                const float t = f[q][0] * b0.x + f[q][1] * b0.y + f[q][2] * b0.z + f[q][3] * b0.w + f[q][4] * b1.x + f[q][5] * b1.y;
+                if (t > tmax) { tmax = t; jmax = j0 + q * MP_THREADS + (int)threadIdx.x + 1; }
+            }
+            // (non-negative floats order as their bits)
+            const unsigned best = __reduce_max_sync(0xffffffffu, __float_as_uint(tmax));
+            const unsigned jb = __reduce_min_sync(0xffffffffu, __float_as_uint(tmax) == best ? (unsigned)jmax : 0x7fffffffu);
+            if (lane == 0 && __uint_as_float(best) > red_t[warp][i]) {
+                red_t[warp][i] = __uint_as_float(best);
+                red_j[warp][i] = (int)jb;
+            }
+        }
     }
-    if (!live) return;
-
-    float *o = a.mpar + (size_t)MODEL_PAR_FLOATS * m;
-    float blk[MODEL_PAR_FLOATS];
+    __syncthreads();
+    if (warp != 0 || !live) return;
+    float tmax = 0.f;
+    int jmax = 1;
 #pragma unroll
-    for (int i = 0; i < MODEL_PAR_FLOATS; ++i) blk[i] = 0.f;
+    for (int w = 0; w < MP_WARPS; ++w) {
+        const float t = red_t[w][lane];
+        const int j = red_j[w][lane];
+        if (t > tmax || (t == tmax && tmax > 0.f && j < jmax)) { tmax = t; jmax = j; }
+    }
+
+    float blk[18];
     // (dust_type 3: the diffuse optical depth is the curve itself, pixel_transmissions :3798-3801)
     const double d1 = p[PF_DUST1], d2 = a.dust_type == 3 ? 1.0 : p[PF_DUST2], d3 = p[PF_DUST3];
     const double fnd = p[PF_FRAC_NODUST], fo = p[PF_FRAC_OBRUN];
@@ -118,92 +210,29 @@ __global__ void __launch_bounds__(256) model_params_kernel(ModelParamArgs a) {
         else if (a.dust_type == 4) { ed = (float)di; s1 = (float)di; }
         else if (a.dust_type == 1) { const double ir = 1.0 / p[PF_MWR], u = p[PF_UVB]; s1 = (float)ir; s2 = (float)u; s3 = (float)(u * ir); }
         blk[MP_DUST_INDEX] = ed;
-        blk[MP_CS1] = s1; blk[MP_CS1 + 1] = s2; blk[MP_CS1 + 2] = s3;
+        o[MP_CS1] = s1; o[MP_CS1 + 1] = s2; o[MP_CS1 + 2] = s3;
     }
     blk[MP_KD1] = (d1 <= SAFE_FLOOR || 1.0 - fo <= SAFE_FLOOR) ? 0.f : (float)(-d1 * LOG2E);
     blk[MP_DUST1_INDEX] = (float)p[PF_DUST1_INDEX];
     blk[MP_ONE_M_FO] = (float)(1.0 - fo);
     blk[MP_FO] = (float)fo;
     blk[MP_KD3] = (fabs(d3) <= SAFE_FLOOR) ? 0.f : (float)(-d3 * LOG2E);
+    blk[MP_IGM_ON] = 0.f;
     blk[MP_IGM_JMAX] = __int_as_float(0);
+    blk[MP_IGM_KCAP] = 0.f;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) blk[MP_IGM_KB + k] = 0.f;
     if (igm) {
         const double kf = -p[PF_IGM_FACTOR] * LOG2E;
-#pragma unroll
-        for (int k = 0; k < 6; ++k) blk[MP_IGM_KB + k] = (float)((double)b[k] * kf);
-        blk[MP_IGM_KCAP] = (float)((double)my_tmax * kf);
-        blk[MP_IGM_JMAX] = __int_as_float(my_jmax);
+        const float kb0 = (float)((double)b[0] * kf), kb1 = (float)((double)b[1] * kf);
+        blk[MP_IGM_KB] = blk[MP_IGM_KB + 2] = kb0;
+        blk[MP_IGM_KB + 1] = blk[MP_IGM_KB + 3] = blk[MP_IGM_KB + 4] = blk[MP_IGM_KB + 5] = kb1;
+        blk[MP_IGM_KCAP] = (float)((double)tmax * kf);
+        blk[MP_IGM_JMAX] = __int_as_float(jmax);
         blk[MP_IGM_ON] = 1.f;
     }
-    // velocity smoothing taps: row i0 of build_velocity_kernel (src/spectra/opensps_smoothing.f90:553-633)
-    blk[MP_SMOOTH_R] = __int_as_float(-1);
-    const double sig = p[PF_SIGMA_SMOOTH];
-    if (a.smooth && sig > SAFE_FLOOR && a.i0 >= 0) {
-        const int n = a.nspec, i = a.i0;
-        const double sb = sig / (C_LIGHT * 1.0e-13);
-        const double inv2s2 = 0.5 * (1.0 / sb) * (1.0 / sb);
-        // the window in ln lambda: lambda_j vs lambda_i exp(-+4 sigma / c) compared as logarithms
-        const double vl = a.lnlam[i] - 4.0 * sb, vh = a.lnlam[i] + 4.0 * sb;
-        // il: first pixel >= vl, one lower when it lies above vl; ih: first pixel >= vh
-        int lo = 0, hi = n;
-        while (lo < hi) { const int md = (lo + hi) / 2; if (a.lnlam[md] < vl) lo = md + 1; else hi = md; }
-        int il = lo < n ? lo : n - 1;
-        if (il > 0 && a.lnlam[il] > vl) il--;
-        lo = il; hi = n;
-        while (lo < hi) { const int md = (lo + hi) / 2; if (a.lnlam[md] < vh) lo = md + 1; else hi = md; }
-        int ih = lo < n ? lo : n - 1;
-        if (ih < il) ih = il;
-        if (ih - il + 1 >= 2 && i - il <= 4 && ih - i <= 4) {
-            // Gaussian weights / lambda_j times the trapezoid widths, normalised: the exponent is formed in FP64
-            // (differences of ln lambda), the exponential and the normalisation in FP32 (the taps are stored so)
-            float w[9], tw = 0.f;
-            const double lli = a.lnlam[i];
 #pragma unroll
-            for (int u = 0; u < 9; ++u) {
-                const int j = il + u;
-                float wj = 0.f;
-                if (j <= ih) {
-                    const double d = lli - a.lnlam[j];
-                    const float dlft = (j > il) ? (float)(a.lam[j] - a.lam[j - 1]) : 0.f;
-                    const float drgt = (j < ih) ? (float)(a.lam[j + 1] - a.lam[j]) : 0.f;
-                    wj = expf((float)(-inv2s2 * d * d)) / (float)a.lam[j] * 0.5f * (dlft + drgt);
-                }
-                w[u] = wj;
-                tw += wj;
-            }
-            if (tw > 0.f) {
-                const float inv = 1.f / tw;
-#pragma unroll
-                for (int d = -4; d <= 4; ++d) {
-                    const int u = i + d - il;
-                    blk[MP_TAPS + 4 + d] = (u >= 0 && u <= ih - il && u < 9) ? w[u] * inv : 0.f;
-                }
-                blk[MP_SMOOTH_R] = __int_as_float(max(i - il, ih - i));
-            }
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < MODEL_PAR_FLOATS; i += 4)
-        reinterpret_cast<float4 *>(o)[i / 4] = make_float4(blk[i], blk[i + 1], blk[i + 2], blk[i + 3]);
-    // observed frame: the shift of lambda / (1 + z) on the log-uniform grid, in pixels
-    // (observed pixel j reads rest pixels j - n0 - 1 and j - n0 at t, the same t for every interior pixel)
-    float4 zi = make_float4(__int_as_float(0), 0.f, 0.f, 0.f);
-    double dd = 0.0;
-    if (fabs(z) > SAFE_FLOOR) {
-        const double s = l1z / a.dlnl;
-        const double n0 = floor(s), phi = s - n0;
-        zi.x = __int_as_float((int)n0);
-        zi.y = phi > 0.0 ? (float)(expm1((1.0 - phi) * a.dlnl) / expm1(a.dlnl)) : 0.f;
-        zi.z = (float)s;
-        zi.w = 1.f;
-        // distance term (distance_term, src/spectra/opensps_batch_photometry.f90:784-794)
-        int idx = find_interval0(a.zt, 500, z);
-        idx = max(0, min(idx, 498));
-        const double slope = (a.dl[idx + 1] - a.dl[idx]) / (a.zt[idx + 1] - a.zt[idx]);
-        const double dm = a.dl[idx] + slope * (z - a.zt[idx]);
-        if (dm == dm && dm > SAFE_FLOOR) dd = 5.0 * log10(dm / 10.0) - 2.5 * log10(1.0 + z);
-    }
-    a.zinfo[m] = zi;
-    a.dist[m] = dd;
+    for (int i = 0; i < 18; i += 2) reinterpret_cast<float2 *>(o)[i / 2] = make_float2(blk[i], blk[i + 1]);
 }
 
 // ---------------------------------------------------------------------------------------------- basis operand
@@ -929,24 +958,18 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     // ---- the per-model parameters, then the weight operand (one stream: run side by side they took longer than in
     // turn)
     prof_mark(c, 0);
-    const int smem_mp = (c.add_igm_absorption == 1 ? c.jtop : 0) * 6 * (int)sizeof(float);
-    if (smem_mp > 48 * 1024 &&
-        (e = cudaFuncSetAttribute(model_params_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_mp)) != cudaSuccess) {
-        err = cuda_msg("model parameter kernel", e);
-        return ST_DATA_MISSING;
-    }
     // per-model parameters of models [off, off + nk)
     auto model_params = [&](int off, int nk) -> cudaError_t {
         ModelParamArgs ma;
         ma.n = nk; ma.nspec = ns; ma.jtop = c.jtop; ma.add_igm = c.add_igm_absorption == 1; ma.smooth = any_smooth ? 1 : 0;
-        ma.i0 = i0; ma.dust_type = c.dust_type; ma.par = d_par + (size_t)PAR_DEVICE * off; ma.igm_a = c.d_igm_a.p; ma.lam = c.d_lam.p;
-        ma.zt = c.d_zt.p; ma.dl = c.d_dl.p; ma.dlnl = c.dlnl; ma.mpar = c.d_mpar.p + (size_t)MODEL_PAR_FLOATS * off;
-        ma.zinfo = c.d_zinfo.p + off; ma.dist = c.d_dist.p + off; ma.lnlam = c.d_lnlam.p;
-        int mpw = 32;
-        while (mpw > 4 && (nk + mpw - 1) / mpw < 8 * c.num_sms) mpw >>= 1;
-        ma.mpw = mpw;
-        const long long warps = (nk + mpw - 1) / mpw;
-        model_params_kernel<<<(unsigned)((warps * 32 + 255) / 256), 256, smem_mp, st>>>(ma);
+        ma.i0 = i0; ma.dust_type = c.dust_type; ma.grid = grid_scalars(c.dlnl); ma.par = d_par + (size_t)PAR_DEVICE * off;
+        ma.igm_a = c.d_igm_a.p; ma.lam = c.d_lam.p; ma.lnlam = c.d_lnlam.p; ma.zt = c.d_zt.p; ma.dl = c.d_dl.p;
+        ma.mpar = c.d_mpar.p + (size_t)MODEL_PAR_FLOATS * off; ma.zinfo = c.d_zinfo.p + off; ma.dist = c.d_dist.p + off;
+        // (fewer models per CTA while that gives every SM one)
+        int mpc = 32;
+        while (mpc > 1 && (nk + mpc - 1) / mpc < c.num_sms) mpc >>= 1;
+        ma.mpc = mpc;
+        model_params_kernel<<<(nk + mpc - 1) / mpc, MP_THREADS, 0, st>>>(ma);
         return cudaGetLastError();
     };
     int launches = 0;
