@@ -342,6 +342,11 @@ static BasisOperand *get_basis(Context &c, int nacc, int itesc, bool neb, double
     op->kion_y = pad(ty_end * nz);
     op->kion_o = pad(n_ion_old * nz);
     op->kpad = op->kmain + op->kion_y + op->kion_o;
+    {
+        const int cols[4] = {nacc == 1 ? nt * nz : itesc * nz, nacc == 1 ? 0 : (nt - itesc) * nz, ty_end * nz, n_ion_old * nz};
+        for (int r = 0; r < 4; ++r)
+            if (cols[r] > 0) op->ktail |= (unsigned)(((cols[r] - 1) % BK) / 16 + 1) << (8 * r);
+    }
     const int kpad = op->kpad;
     std::vector<uint16_t> hi((size_t)ns * kpad, 0), lo((size_t)ns * kpad, 0);
     std::vector<int> kmap(kpad, -1);   // operand column -> source index t + nt z with the KMAP_ flags
@@ -833,8 +838,6 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     c.geom.neb_table = neb_table;
 
     // ---- scratch
-    const int bn = contract_models_per_tile(nacc);
-    const int n_mtiles = (n + bn - 1) / bn;
     const int kpad = ops ? 64 : bop->kpad;
     cudaError_t e;
     const size_t nwz = (size_t)n * nt * nz;
@@ -1082,6 +1085,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
                 return ST_DATA_MISSING;
             }
             if (marks) prof_mark(c, 2);
+            const int n_ptiles = (ns + contract_out_rows() - 1) / contract_out_rows();
+            const int bn = contract_tile_models(nacc, nk, n_ptiles, c.num_sms);
             ContractPlan pl;
             pl.tm_a_hi = bop->tm_hi;
             pl.tm_a_lo = bop->tm_lo;
@@ -1093,7 +1098,9 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             }
             ContractArgs ca;
             ca.nspec = ns; ca.n_models = nk;
-            ca.n_ptiles = (ns + contract_out_rows() - 1) / contract_out_rows();
+            ca.n_ptiles = n_ptiles;
+            ca.bn = bn;
+            ca.ktail = bop->ktail;
             ca.n_mtiles = (nk + bn - 1) / bn;
             ca.nkb_young = (nacc == 1) ? bop->kmain / contract_bk() : bop->ky_pad / contract_bk();
             ca.nkb_old = (nacc == 1) ? 0 : (bop->kmain - bop->ky_pad) / contract_bk();

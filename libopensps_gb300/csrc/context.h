@@ -57,6 +57,7 @@ struct BasisOperand {
     // K columns: [young block (ky_pad) | old block | escaping-light young block (kion_y) | escaping-light old block
     // (kion_o)]; kmain = the young and old blocks, kpad = all (the blocks padded to the contraction's K step)
     int nacc = 0, itesc = 0, kpad = 0, ky_pad = 0, nty = 0, kmain = 0, kion_y = 0, kion_o = 0;
+    unsigned ktail = 0;   // the K steps in each range's last block (ContractArgs::ktail)
     bool ion = false;
     DevBuf<__nv_bfloat16> hi, lo;
     DevBuf<int> kmap;            // operand column -> source (age, metallicity) of the weights with the KMAP_ flags

@@ -11,7 +11,9 @@
 // Matrix form: D(pixels x models) = basis(pixels x K) . W(models x K)^T, both operands K-major bf16 split into hi and
 // lo parts (x = x_hi + x_lo); D = A_hi B_hi + A_hi B_lo + A_lo B_hi, accumulated in f32 in tensor memory. Tile: 128
 // pixels x BN models x 64 K per stage; the 128 pixel rows of a tile are 120 output pixels with a halo of 4 on each
-// side for the smoothing. One CTA per SM, persistent over tiles (model tile outer, pixel tile inner, so that the
+// side for the smoothing; BN is the largest tile (256 models, 128 with two accumulators) or a narrower one of a smaller
+// batch, with the stages that fit (contract_tile_models). The 16-column K steps past a range's last column are left out
+// (81 steps of 84 for 107 ages x 12 metallicities). One CTA per SM, persistent over tiles (model tile outer, pixel tile inner, so that the
 // CTAs running together share the weights of a model tile in L2). Warp roles: warp 0 = TMA producer, warp 1 = MMA
 // issuer (and TMEM owner), warps 2..9 = epilogue in two groups of four (group g takes the models of column half g;
 // in a group, warp w reads TMEM lanes 32 (w % 4) ..). Accumulators are double-buffered in TMEM so that the
@@ -30,6 +32,7 @@
 // ones. Only the pixel tiles that reach an ionizing pixel run them.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <cstdint>
 #include "sm103_ptx.cuh"
 #include "csp_kernels.h"
@@ -40,7 +43,7 @@ constexpr int BM = 128;          // pixel rows per tile (MMA M)
 constexpr int BK = 64;           // K per stage (one 128-byte swizzled row of bf16)
 constexpr int HALO = 4;          // smoothing halo (taps -4 .. 4)
 constexpr int OUT_ROWS = BM - 2 * HALO;
-constexpr int NSTAGE = 2;
+constexpr int MAX_STAGES = 4;    // stages of a tile of few models (2 at the full tile)
 constexpr int EPI_GROUPS = 2;
 constexpr int EPI_WARPS = 4 * EPI_GROUPS;
 constexpr int NTHREADS = (2 + EPI_WARPS) * 32;
@@ -49,18 +52,20 @@ constexpr int TROW = BM + 4;     // staging row (floats): 16-byte aligned rows, 
 
 template <int NACC>
 struct ContractCfg {
-    static constexpr int BN = (NACC == 1) ? 256 : 128;           // models per tile (MMA N)
+    static constexpr int BN = (NACC == 1) ? 256 : 128;           // most models per tile (MMA N)
     static constexpr int A_BYTES = BM * BK * 2;                   // one of A_hi / A_lo
-    static constexpr int B_BYTES = BN * BK * 2;
-    static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
+    static constexpr int STAGE_SMEM = 2 * (2 * A_BYTES + 2 * BN * BK * 2);   // the stages' shared memory
     static constexpr int ACC_COLS = NACC * BN;                    // TMEM columns of one accumulator set
     static constexpr int TMEM_COLS = 2 * ACC_COLS;                // double-buffered (= 512)
-    static constexpr int GROUP_COLS = BN / EPI_GROUPS;            // models per epilogue group
     static constexpr int STAGE_T_FLOATS = CHUNK * TROW;           // per group
     static constexpr int PAR_FLOATS = 2 * CHUNK * MODEL_PAR_FLOATS;   // per group, double-buffered
     static constexpr int EPI_BYTES = EPI_GROUPS * (STAGE_T_FLOATS + PAR_FLOATS) * 4;
-    static constexpr int SMEM_BYTES = NSTAGE * STAGE_BYTES + EPI_BYTES + 256 + 1024;
-    static constexpr uint32_t IDESC = idesc_bf16_f32(BM, BN);
+    static constexpr int SMEM_BYTES = STAGE_SMEM + EPI_BYTES + 256 + 1024;
+    // a stage of tiles of bn models, and the stages that fit
+    static constexpr __host__ __device__ int stage_bytes(int bn) { return 2 * A_BYTES + 2 * bn * BK * 2; }
+    static constexpr __host__ __device__ int stages(int bn) {
+        return STAGE_SMEM / stage_bytes(bn) < MAX_STAGES ? STAGE_SMEM / stage_bytes(bn) : MAX_STAGES;
+    }
 };
 
 // 2^x by the SFU (relative error ~2^-22; flushes results below the smallest normal to zero).
@@ -92,14 +97,16 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint8_t *stage_base = smem;
-    float *epi_base = reinterpret_cast<float *>(smem + NSTAGE * C::STAGE_BYTES);
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + NSTAGE * C::STAGE_BYTES + C::EPI_BYTES);
-    uint64_t *full = bars;                 // [NSTAGE]
-    uint64_t *empty = bars + NSTAGE;       // [NSTAGE]
-    uint64_t *tfull = bars + 2 * NSTAGE;   // [2]
-    uint64_t *tempty = bars + 2 * NSTAGE + 2;
-    uint64_t *mma_done = bars + 2 * NSTAGE + 4;
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NSTAGE + 5);
+    float *epi_base = reinterpret_cast<float *>(smem + C::STAGE_SMEM);
+    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + C::STAGE_SMEM + C::EPI_BYTES);
+    uint64_t *full = bars;                     // [MAX_STAGES]
+    uint64_t *empty = bars + MAX_STAGES;       // [MAX_STAGES]
+    uint64_t *tfull = bars + 2 * MAX_STAGES;   // [2]
+    uint64_t *tempty = bars + 2 * MAX_STAGES + 2;
+    uint64_t *mma_done = bars + 2 * MAX_STAGES + 4;
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * MAX_STAGES + 5);
+    const int bn = args.bn, nstage = C::stages(bn);
+    const uint32_t stage_bytes = (uint32_t)C::stage_bytes(bn), b_bytes = (uint32_t)(bn * BK * 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_ptiles = args.n_ptiles;
@@ -111,7 +118,7 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
     int *status = args.status;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < NSTAGE; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < nstage; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], EPI_WARPS); }
         mbar_init(mma_done, 1);
         fence_mbar_init();
@@ -130,27 +137,31 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
         // ------------------------------------------------------------------ TMA producer
         if (lane == 0) {
             int s = 0; uint32_t ph = 0;
-            int last_fill[NSTAGE];              // parity of the last fill issued into each stage, -1: none
-            for (int i = 0; i < NSTAGE; ++i) last_fill[i] = -1;
+            int last_fill[MAX_STAGES];          // parity of the last fill issued into each stage, -1: none
+#pragma unroll
+            for (int i = 0; i < MAX_STAGES; ++i) last_fill[i] = -1;
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 const int mt = tile / n_ptiles, pt = tile % n_ptiles;
-                const int p0 = pt * OUT_ROWS - HALO, m0 = mt * C::BN;
+                const int p0 = pt * OUT_ROWS - HALO, m0 = mt * bn;
                 const int kbn = tile_nkb(pt);
                 for (int kb = 0; kb < kbn; ++kb) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, status, ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
-                    uint8_t *st = stage_base + s * C::STAGE_BYTES;
-                    mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
+                    uint8_t *st = stage_base + s * stage_bytes;
+                    mbar_arrive_expect_tx(&full[s], stage_bytes);
                     tma_load_2d(st, &tm_a_hi, kb * BK, p0, &full[s]);
                     tma_load_2d(st + C::A_BYTES, &tm_a_lo, kb * BK, p0, &full[s]);
                     tma_load_2d(st + 2 * C::A_BYTES, &tm_b_hi, kb * BK, m0, &full[s]);
-                    tma_load_2d(st + 2 * C::A_BYTES + C::B_BYTES, &tm_b_lo, kb * BK, m0, &full[s]);
-                    last_fill[s] = (int)ph;
-                    if (++s == NSTAGE) { s = 0; ph ^= 1u; }
+                    tma_load_2d(st + 2 * C::A_BYTES + b_bytes, &tm_b_lo, kb * BK, m0, &full[s]);
+#pragma unroll
+                    for (int i = 0; i < MAX_STAGES; ++i)
+                        if (i == s) last_fill[i] = (int)ph;
+                    if (++s == nstage) { s = 0; ph ^= 1u; }
                 }
             }
             // Drain: every copy this thread issued must have landed before the CTA may exit.
-            for (int i = 0; i < NSTAGE; ++i)
+#pragma unroll
+            for (int i = 0; i < MAX_STAGES; ++i)
                 if (last_fill[i] >= 0) mbar_wait(&full[i], (uint32_t)last_fill[i], status, ERR_TIMEOUT_PRODUCER, false);
         }
     } else if (warp == 1) {
@@ -158,6 +169,7 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
         if (lane == 0) {
             int s = 0; uint32_t ph = 0;
             int acc = 0; uint32_t aph = 0;
+            const uint32_t idesc = idesc_bf16_f32(BM, bn);
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 if (!mbar_wait(&tempty[acc], aph ^ 1u, status, ERR_TIMEOUT_MMA)) { ok = false; break; }
@@ -174,19 +186,28 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
                     const int which = (NACC == 2 && ((kb >= args.nkb_young && kb < nkb) || ion_old)) ? 1 : 0;
                     const uint32_t d = d_base + which * C::BN;
                     const int kfirst = kb >= nkb ? -1 : (which == 0) ? 0 : args.nkb_young;
-                    const uint32_t sa = smem_u32(stage_base + s * C::STAGE_BYTES);
+                    const uint32_t sa = smem_u32(stage_base + s * stage_bytes);
                     const uint32_t a_hi = sa, a_lo = sa + C::A_BYTES;
-                    const uint32_t b_hi = sa + 2 * C::A_BYTES, b_lo = b_hi + C::B_BYTES;
-#pragma unroll
-                    for (int k = 0; k < BK / 16; ++k) {
+                    const uint32_t b_hi = sa + 2 * C::A_BYTES, b_lo = b_hi + b_bytes;
+                    // (the last block of a range holds only its last columns' K steps)
+                    const int r = kb < args.nkb_young ? 0 : kb < nkb ? 1 : kb < nkb + args.nkb_ion_young ? 2 : 3;
+                    const int rend = r == 0 ? args.nkb_young : r == 1 ? nkb : r == 2 ? nkb + args.nkb_ion_young : nkb + nkb_ion;
+                    const int ksteps = kb + 1 == rend ? (int)((args.ktail >> (8 * r)) & 0xffu) : BK / 16;
+                    auto step = [&](int k) {
                         const uint32_t off = k * 32;
                         const uint32_t accum = (kb > kfirst || k > 0) ? 1u : 0u;
-                        mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_hi + off), C::IDESC, accum);
-                        mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_lo + off), C::IDESC, 1u);
-                        mma_bf16(d, sw128_desc(a_lo + off), sw128_desc(b_hi + off), C::IDESC, 1u);
+                        mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_hi + off), idesc, accum);
+                        mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_lo + off), idesc, 1u);
+                        mma_bf16(d, sw128_desc(a_lo + off), sw128_desc(b_hi + off), idesc, 1u);
+                    };
+                    if (ksteps == BK / 16) {
+#pragma unroll
+                        for (int k = 0; k < BK / 16; ++k) step(k);
+                    } else {
+                        for (int k = 0; k < ksteps; ++k) step(k);
                     }
                     mma_commit(&empty[s]);          // frees the stage once these MMAs have read it
-                    if (++s == NSTAGE) { s = 0; ph ^= 1u; }
+                    if (++s == nstage) { s = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
                 mma_commit(&tfull[acc]);            // accumulator ready for the epilogue
@@ -208,11 +229,12 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
         float *stageT = epi_base + g * (C::STAGE_T_FLOATS + C::PAR_FLOATS);
         float *parbuf = stageT + C::STAGE_T_FLOATS;
         const bool vec_store = (args.ld_spec & 1) == 0;
+        const int group_cols = bn / EPI_GROUPS;          // models per epilogue group
         int acc = 0; uint32_t aph = 0;
         int pb = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
             const int mt = tile / n_ptiles, pt = tile % n_ptiles;
-            const int p0 = pt * OUT_ROWS - HALO, m0 = mt * C::BN;
+            const int p0 = pt * OUT_ROWS - HALO, m0 = mt * bn;
             const int p = p0 + r;
             const bool inpix = (p >= 0 && p < args.nspec);
             // per-pixel data of this thread's row (phase 1)
@@ -234,8 +256,8 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
             tc_fence_after();
             const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + acc * C::ACC_COLS;
 
-            for (int c = 0; c < C::GROUP_COLS / CHUNK; ++c) {
-                const int col0 = g * C::GROUP_COLS + c * CHUNK;      // first model of the chunk in the tile
+            for (int c = 0; c < group_cols / CHUNK; ++c) {
+                const int col0 = g * group_cols + c * CHUNK;      // first model of the chunk in the tile
                 // model parameters of the chunk (double-buffered)
                 float *par = parbuf + pb * CHUNK * MODEL_PAR_FLOATS;
                 for (int i = et; i < CHUNK * MODEL_PAR_FLOATS / 4; i += 128) {
@@ -259,7 +281,7 @@ csp_contract_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_co
                         for (int j = 0; j < 16; ++j) o[j] = 0.f;
                     }
                 }
-                if (c == C::GROUP_COLS / CHUNK - 1) {
+                if (c == group_cols / CHUNK - 1) {
                     // all of this group's accumulator columns have been read: hand them back to the MMA warp
                     tc_fence_before();
                     __syncwarp();
@@ -378,7 +400,26 @@ static cudaError_t launch_contract(const ContractPlan &pl, const ContractArgs &a
     return cudaGetLastError();
 }
 
-int contract_models_per_tile(int nacc) { return nacc == 1 ? ContractCfg<1>::BN : ContractCfg<2>::BN; }
+// The tile width by its measured cost: a first wave of tiles takes 18 + 0.135 bn us (one accumulator; 23.5 + 0.135 bn
+// with two: the K loop's latency and the epilogue, which nothing overlaps), a further wave what the table gives (us at
+// bn = 32, 64 ..; the narrow ones pay the epilogue and the K loop's latency). The widest tile is not always the
+// cheapest: a batch may fill its last wave badly, or hold fewer models than a tile. Measured, 256 (128) models a tile
+// before -> with the rule: 38.7 -> 20.5 us at one model, 80 -> 64 at 1000, 110 -> 97 at 2000, 1951 -> 1927 at 65536.
+// Every width gives the same bits: an output's products are summed in the same order.
+int contract_tile_models(int nacc, int n_models, int n_ptiles, int num_sms) {
+    static const double further1[8] = {13.2, 13.4, 13.9, 14.4, 15.8, 17.4, 19.9, 23.0};
+    static const double further2[4] = {14.7, 15.5, 17.2, 17.6};
+    const int most = nacc == 1 ? ContractCfg<1>::BN : ContractCfg<2>::BN;
+    int best = most;
+    double best_t = 1e300;
+    for (int bn = most; bn >= 32; bn -= 32) {
+        const long long tiles = (long long)((n_models + bn - 1) / bn) * n_ptiles, waves = (tiles + num_sms - 1) / num_sms;
+        const double t = (nacc == 1 ? 18.0 : 23.5) + 0.135 * bn +
+                         (double)(waves - 1) * (nacc == 1 ? further1 : further2)[bn / 32 - 1];
+        if (t < best_t) { best_t = t; best = bn; }
+    }
+    return best;
+}
 int contract_out_rows() { return OUT_ROWS; }
 int contract_halo() { return HALO; }
 int contract_bk() { return BK; }

@@ -99,6 +99,10 @@ struct ContractArgs {
     // young accumulator, then ion old blocks into the old one), run only by the pixel tiles that reach a pixel below
     // ion_pix (the ionizing pixels; the basis holds those columns' unabsorbed spectra there and zeros above)
     int nkb_ion_young = 0, nkb_ion_old = 0, ion_pix = 0;
+    // models per tile (a multiple of 32, contract_tile_models), and the 16-column K steps of the last block of the
+    // young, old, ion young and ion old ranges, a byte each
+    int bn = 0;
+    unsigned ktail = 0;
     int sm_lo, sm_hi;    // pixels smoothed (lambda within [min_wave_smooth, max_wave_smooth]); sm_lo > sm_hi: none
     int uniform_index;   // every model has the pixel table's curve
     int tab_curve = 0;   // not uniform: each model's curve from the pixel table's T0..T3 (else its power law)
@@ -114,7 +118,8 @@ struct ContractPlan {
     int num_sms;
 };
 
-int contract_models_per_tile(int nacc);
+// Models per tile for a batch of n_models over n_ptiles pixel tiles.
+int contract_tile_models(int nacc, int n_models, int n_ptiles, int num_sms);
 int contract_out_rows();
 int contract_halo();
 int contract_bk();
