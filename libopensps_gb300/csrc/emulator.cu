@@ -21,6 +21,11 @@
 // deviation over the members, the largest over the bands that are less than `faint` mag fainter than the
 // brightest) and flag are formed from there.
 //
+// A batch of few tiles leaves most SMs without one (four CTAs took 220 us for 500 models): there a CTA takes one member
+// of a tile at a time (SPLIT), its outputs go to the tile's place in the scratch, and emu_reduce_kernel forms the
+// ensemble's results from them, in the order of members the fused kernel sums them in: 224 -> 47 us at 500 models,
+// 441 -> 227 at 20000.
+//
 // Every mbarrier wait is bounded (status word, no hang); drains wait for the copies and MMAs in flight.
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -82,11 +87,23 @@ __device__ __forceinline__ float emu_distance(float z, const float *zt, const fl
     return 5.f * log10f(dm * 0.1f) - 2.5f * log10f(1.f + z);
 }
 
-// The member a CTA runs at step mem of each tile: the order is rotated by the CTA index, so that the CTAs stream
-// different members' weights at a time instead of all reading the same tiles from the same L2 lines.
-__device__ __forceinline__ int emu_member(int mem) { return (mem + (int)blockIdx.x) % EMU_MEMBERS; }
-// Tiles per CTA: the same count in every CTA, the ones past the last tile are run with no valid model.
-__device__ __forceinline__ int emu_iters(int ntiles) { return (ntiles + (int)gridDim.x - 1) / (int)gridDim.x; }
+// The work of a CTA: iteration it's tile, and the members it runs there (all of them, or with SPLIT one: unit
+// blockIdx + it gridDim is member unit % EMU_MEMBERS of tile unit / EMU_MEMBERS). The member at step mem is rotated by
+// the CTA index, so that the CTAs stream different members' weights at a time instead of all reading the same tiles
+// from the same L2 lines. The same count of iterations in every CTA, the ones past the last tile are run with no valid
+// model.
+template <bool SPLIT>
+struct EmuWork {
+    static constexpr int STEPS = SPLIT ? 1 : EMU_MEMBERS;
+    static __device__ __forceinline__ int unit(int it) { return (int)blockIdx.x + it * (int)gridDim.x; }
+    static __device__ __forceinline__ int tile(int it) { return SPLIT ? unit(it) / EMU_MEMBERS : unit(it); }
+    static __device__ __forceinline__ int member(int it, int mem) {
+        return SPLIT ? unit(it) % EMU_MEMBERS : (mem + (int)blockIdx.x) % EMU_MEMBERS;
+    }
+    static __device__ __forceinline__ int iters(int ntiles) {
+        return ((SPLIT ? ntiles * EMU_MEMBERS : ntiles) + (int)gridDim.x - 1) / (int)gridDim.x;
+    }
+};
 
 // A warp-uniform bounded wait (every lane polls; the warp goes on only if all saw the phase complete).
 __device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, int *status, int code) {
@@ -110,6 +127,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 
 // The epilogue warps: lane quarter q (TMEM lanes 32q..32q+31, model rows), column slice cs (64 of a hidden chunk's
 // 256 columns; 32 of the output chunk's 128).
+template <bool SPLIT>
 __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, uint64_t *bars, uint32_t tmem_base,
                                              int q, int cs, int lane) {
     uint64_t *afull = bars + 2 * EI_NS, *aempty = afull + 1, *hrdy = aempty + 1, *inrdy = hrdy + 2;
@@ -118,13 +136,14 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
     const uint32_t s_base = smem_u32(S);
     const float *par = a.par;
     const int ntiles = (a.n + 127) / 128;
-    const int iters = emu_iters(ntiles);
+    using Work = EmuWork<SPLIT>;
+    const int iters = Work::iters(ntiles);
     int *status = a.status;
-    // this row's outputs of each member: scratch[cta][member][row][128]; then, per CTA, two slots x 128 rows x 16
-    // words of tile inputs (the input row's 12 f16 words, zred, the flags)
-    float *scr_row = a.scratch + ((size_t)blockIdx.x * EMU_SCRATCH_CTA + (size_t)r * EMU_NOUT);
-    uint4 *in_row = reinterpret_cast<uint4 *>(a.scratch + (size_t)blockIdx.x * EMU_SCRATCH_CTA +
-                                             (size_t)EMU_MEMBERS * 128 * EMU_NOUT) + (size_t)r * 4;
+    // per CTA, two slots x 128 rows x 16 words of tile inputs (the input row's 12 f16 words, zred, the flags); this
+    // row's outputs of each member: scratch[cta][step][row][128], with SPLIT scratch[unit][row][128]
+    uint4 *in_row = reinterpret_cast<uint4 *>(a.scratch + (size_t)blockIdx.x * EMU_SCRATCH_IN) + (size_t)r * 4;
+    float *scr_row = a.scratch + (size_t)gridDim.x * EMU_SCRATCH_IN +
+                     (SPLIT ? 0 : (size_t)blockIdx.x * EMU_MEMBERS * 128 * EMU_NOUT) + (size_t)r * EMU_NOUT;
     constexpr size_t SCR_MEM = (size_t)128 * EMU_NOUT;
     uint32_t g = 0;
     bool ok = true;
@@ -178,13 +197,15 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
         __syncwarp();
         if (lane == 0) mbar_arrive(inrdy);
     };
-    prepare_input(blockIdx.x, 0);
+    prepare_input(Work::tile(0), 0);
     put_input(0);
     for (int it = 0; it < iters && ok; ++it) {
-        const int tile = blockIdx.x + it * gridDim.x;
-        const int m = tile * 128 + r;
-        for (int mem = 0; mem < EMU_MEMBERS && ok; ++mem) {
-            const float *bm = a.bias + (size_t)emu_member(mem) * EMU_NBIAS;
+        const int m = Work::tile(it) * 128 + r;
+        if (SPLIT && it > 0) scr_row += (size_t)gridDim.x * 128 * EMU_NOUT;
+        if (SPLIT && it == 0) scr_row += (size_t)blockIdx.x * 128 * EMU_NOUT;
+        const bool stored = !SPLIT || Work::tile(it) < ntiles;
+        for (int mem = 0; mem < Work::STEPS && ok; ++mem) {
+            const float *bm = a.bias + (size_t)Work::member(it, mem) * EMU_NBIAS;
             for (int L = 0; L < 5 && ok; ++L) {
                 const int nch = L == 4 ? 1 : 2;
                 for (int c = 0; c < nch; ++c) {
@@ -235,7 +256,7 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&hrdy[c]);
                         // the next tile's inputs, where the epilogue has time to spare
-                        if (mem == 0 && L == 1 && c == 0 && it + 1 < iters) prepare_input(tile + gridDim.x, (it + 1) & 1);
+                        if (mem == 0 && L == 1 && c == 0 && it + 1 < iters) prepare_input(Work::tile(it + 1), (it + 1) & 1);
                     } else {
                         // the output chunk (128 columns): this slice's 32
                         uint32_t v[32];
@@ -246,12 +267,12 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
                         if (lane == 0) mbar_arrive(aempty);
                         // S is free (the output layer's MMAs are done): the next member's input row, or the next
                         // tile's after the last member
-                        if (mem + 1 < EMU_MEMBERS) put_input(it & 1);
+                        if (mem + 1 < Work::STEPS) put_input(it & 1);
                         else if (it + 1 < iters) put_input((it + 1) & 1);
                         const float4 *b4 = reinterpret_cast<const float4 *>(bm + 4 * EMU_H + cs * 32);
                         float4 *dst = reinterpret_cast<float4 *>(scr_row + mem * SCR_MEM + cs * 32);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) {
+                        for (int i = 0; stored && i < 8; ++i) {
                             const float4 t = __ldg(b4 + i);
                             dst[i] = make_float4(__uint_as_float(v[4 * i]) + t.x, __uint_as_float(v[4 * i + 1]) + t.y,
                                                  __uint_as_float(v[4 * i + 2]) + t.z, __uint_as_float(v[4 * i + 3]) + t.w);
@@ -260,6 +281,7 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
                 }
             }
         }
+        if (SPLIT) continue;
         // ---- the ensemble's outputs of the quarter's rows: the four slices' scratch writes are in. The barrier is
         // passed by all four warps whatever happened, and they stop together if any of them, or the status word,
         // says so (a wait that gave up)
@@ -333,6 +355,7 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
     }
 }
 
+template <bool SPLIT>
 __global__ void __launch_bounds__(EI_THREADS, 1)
 emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constant__ CUtensorMap tm_wh,
                  const __grid_constant__ CUtensorMap tm_w4, EmuInferArgs a) {
@@ -363,7 +386,8 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    const int iters = emu_iters(ntiles);
+    using Work = EmuWork<SPLIT>;
+    const int iters = Work::iters(ntiles);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -372,14 +396,14 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
             for (int i = 0; i < EI_NS; ++i) last_fill[i] = -1;
             bool ok = true;
             for (int it = 0; it < iters && ok; ++it)
-                for (int mem = 0; mem < EMU_MEMBERS && ok; ++mem)
+                for (int mem = 0; mem < Work::STEPS && ok; ++mem)
                     for (int L = 0; L < 5 && ok; ++L) {
                         const int nch = L == 4 ? 1 : 2, nkb = L == 0 ? 1 : 8;
                         for (int c = 0; c < nch && ok; ++c)
                             for (int kb = 0; kb < nkb; ++kb) {
                                 // the stage is free once the MMAs that read it have completed
                                 if (!mbar_wait(&empty[s], ph ^ 1u, status, ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
-                                const int mw = emu_member(mem);
+                                const int mw = Work::member(it, mem);
                                 uint8_t *st = W + s * EI_STAGE;
                                 if (L < 4) {
                                     mbar_arrive_expect_tx(&full[s], EI_STAGE);
@@ -407,7 +431,7 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
             const uint32_t s_base = smem_u32(S);
             const uint32_t d = tmem_base + EI_ACC_COL;
             for (int it = 0; it < iters && ok; ++it)
-                for (int mem = 0; mem < EMU_MEMBERS && ok; ++mem) {
+                for (int mem = 0; mem < Work::STEPS && ok; ++mem) {
                     if (!mbar_wait(inrdy, icnt & 1u, status, ERR_TIMEOUT_MMA)) { ok = false; break; }
                     ++icnt;
                     tc_fence_after();
@@ -455,7 +479,7 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
             mbar_wait(mma_done, 0, status, ERR_TIMEOUT_MMA, false);
         }
     } else {
-        emu_epilogue(a, S, bars, tmem_base, warp & 3, (warp - 2) >> 2, lane);
+        emu_epilogue<SPLIT>(a, S, bars, tmem_base, warp & 3, (warp - 2) >> 2, lane);
     }
     tc_fence_before();
     __syncthreads();
@@ -463,6 +487,90 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }
+}
+
+// The ensemble's results of a SPLIT batch, one warp per model: four outputs per lane, the members in the fused kernel's
+// order (member (k + tile) % EMU_MEMBERS at step k, the order of a CTA's first tile).
+__global__ void __launch_bounds__(256) emu_reduce_kernel(EmuInferArgs a, const float *out) {
+    const int m = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (m >= a.n) return;
+    const float *par = a.par;
+    const int tile = m >> 7, r = m & 127;
+    const float invm = 1.f / (float)EMU_MEMBERS;
+    float z[EMU_MEMBERS][4];
+#pragma unroll
+    for (int k = 0; k < EMU_MEMBERS; ++k) {
+        const int unit = tile * EMU_MEMBERS + (k + tile) % EMU_MEMBERS;
+        const float4 t = *reinterpret_cast<const float4 *>(out + ((size_t)unit * 128 + r) * EMU_NOUT + 4 * lane);
+        z[k][0] = t.x; z[k][1] = t.y; z[k][2] = t.z; z[k][3] = t.w;
+    }
+    float x[EMU_NIN], xs[EMU_NFEAT];
+#pragma unroll
+    for (int i = 0; i < EMU_NIN; ++i) x[i] = __ldg(a.x + (size_t)m * EMU_NIN + i);
+    const bool outside = !emu_features(x, par, xs);
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < EMU_NFEAT; ++i) bad = bad || !isfinite(xs[i]);
+    // (the fused kernel's distance of a model that is not finite is zred's too)
+    const float dd = emu_distance(x[5], par + EMU_P_ZT, par + EMU_P_DL);
+    float v[4], sd[4];
+    float mmin = INFINITY;
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int col = 4 * lane + i, band = col - EMU_NPC;
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < EMU_MEMBERS; ++k) sum += z[k][i];
+        v[i] = par[EMU_P_OMU + col] + par[EMU_P_OSIG + col] * sum * invm;
+        sd[i] = 0.f;
+        if (band < 0) continue;
+        v[i] += dd;
+        const float mean = sum * invm;
+        float var = 0.f;
+#pragma unroll
+        for (int k = 0; k < EMU_MEMBERS; ++k) var += (z[k][i] - mean) * (z[k][i] - mean);
+        sd[i] = par[EMU_P_OSIG + col] * sqrtf(var * invm);
+        if (band < a.nb) {
+            if (!isfinite(v[i]) || !isfinite(sd[i])) finite = false;
+            mmin = fminf(mmin, v[i]);
+            a.mags[(size_t)m * a.nb + band] = v[i];
+        }
+    }
+    if (a.coef && 4 * lane < EMU_NPC)
+        *reinterpret_cast<float4 *>(a.coef + (size_t)m * EMU_NPC + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mmin = fminf(mmin, __shfl_xor_sync(0xffffffffu, mmin, off));
+    float spread = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int band = 4 * lane + i - EMU_NPC;
+        if (band >= 0 && band < a.nb && v[i] < mmin + a.faint) spread = fmaxf(spread, sd[i]);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) spread = fmaxf(spread, __shfl_xor_sync(0xffffffffu, spread, off));
+    finite = __all_sync(0xffffffffu, finite);
+    if (lane == 0) {
+        const int f = outside ? 1 : (bad || !finite) ? 3 : (spread > a.spread_max) ? 2 : 0;
+        if (a.spread) a.spread[m] = spread;
+        a.flag[m] = f;
+        if (f) a.flagged[atomicAdd(a.nflag, 1)] = m;
+    }
+}
+
+// One member per CTA while that shortens the longest CTA: members (tiles x 5) in rounds of num_sms against five members
+// for each round of tiles; up to two tiles per SM (its scratch is 64 KB a member).
+static bool emu_split(int n, int num_sms) {
+    const int ntiles = (n + 127) / 128;
+    if (ntiles > 2 * num_sms) return false;
+    const int rounds = (ntiles * EMU_MEMBERS + num_sms - 1) / num_sms, fused = (ntiles + num_sms - 1) / num_sms * EMU_MEMBERS;
+    return rounds < fused;
+}
+size_t emu_scratch_floats(int n, int num_sms) {
+    const int ntiles = (n + 127) / 128, units = ntiles * EMU_MEMBERS;
+    const size_t cta = (size_t)128 * EMU_NOUT;
+    return emu_split(n, num_sms) ? (size_t)std::min(num_sms, units) * EMU_SCRATCH_IN + units * cta
+                                 : (size_t)std::min(num_sms, ntiles) * (EMU_SCRATCH_IN + EMU_MEMBERS * cta);
 }
 
 int emu_infer_smem() { return EI_SMEM; }
@@ -473,19 +581,15 @@ int emu_weight_box_rows4() { return EI_ROWS4; }
 cudaError_t run_emu_infer(const Emulator &e, const EmuInferArgs &a, int num_sms, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
     if (a.nb < 1 || a.nb > EMU_MAX_BANDS) return cudaErrorInvalidValue;
-    cudaError_t err = cudaFuncSetAttribute(emu_infer_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, EI_SMEM);
-    if (err != cudaSuccess) return err;
-    cudaLaunchConfig_t cfg = {};
-    cfg.blockDim = dim3(EI_THREADS);
-    cfg.dynamicSmemBytes = EI_SMEM;
-    cfg.stream = st;
-    cfg.attrs = nullptr;
-    cfg.numAttrs = 0;
-    // persistent: one CTA per SM (its shared memory allows no more), no more CTAs than tiles
     const int ntiles = (a.n + 127) / 128;
-    cfg.gridDim = dim3(std::min(num_sms, ntiles));
-    err = cudaLaunchKernelEx(&cfg, emu_infer_kernel, e.tm_w0, e.tm_wh, e.tm_w4, a);
+    const bool split = emu_split(a.n, num_sms);
+    auto kern = split ? emu_infer_kernel<true> : emu_infer_kernel<false>;
+    cudaError_t err = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, EI_SMEM);
     if (err != cudaSuccess) return err;
+    // persistent: one CTA per SM (its shared memory allows no more), no more CTAs than tiles (members with split)
+    const int grid = std::min(num_sms, split ? ntiles * EMU_MEMBERS : ntiles);
+    kern<<<grid, EI_THREADS, EI_SMEM, st>>>(e.tm_w0, e.tm_wh, e.tm_w4, a);
+    if (split) emu_reduce_kernel<<<(a.n + 7) / 8, 256, 0, st>>>(a, a.scratch + (size_t)grid * EMU_SCRATCH_IN);
     return cudaGetLastError();
 }
 

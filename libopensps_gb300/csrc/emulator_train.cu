@@ -28,6 +28,7 @@
 namespace sps {
 
 cudaError_t run_emu_infer(const Emulator &e, const EmuInferArgs &a, int num_sms, cudaStream_t st);
+size_t emu_scratch_floats(int n, int num_sms);
 int emu_weight_box_rows();
 int emu_weight_box_rows4();
 int csp_batch_mags(Context &c, int n, int n_params, const char *const *names, const double *const *values,
@@ -61,6 +62,7 @@ void Emulator::release() {
     wht = w4t = nullptr;
     bias = d_par = d_pca_mean = d_pca_basis = master = adam_m = adam_v = nullptr;
     d_x = d_mags = d_coef = d_spread = d_scratch = nullptr;
+    scratch_cap = 0;
     d_flag = d_nflag = d_flagged = nullptr;
     cap = 0;
     ready = trainable = false;
@@ -776,9 +778,14 @@ int emu_infer_device(Context &c, int n, const float *d_x, float *d_mags, float *
     Emulator &e = c.emu;
     if (!e.ready) { err = "no emulator on the context (opensps_gb300_emulator_load / _train)"; return ST_NO_OPERATOR; }
     if (e.nb != c.nbands) { err = "the emulator was trained for another band set"; return ST_UNSUPPORTED; }
-    if (!e.d_scratch) {
-        const cudaError_t r = dalloc(&e.d_scratch, (size_t)c.num_sms * EMU_SCRATCH_CTA);
+    const size_t need = emu_scratch_floats(n, c.num_sms);
+    if (e.scratch_cap < need) {
+        cudaFree(e.d_scratch);
+        e.d_scratch = nullptr;
+        e.scratch_cap = 0;
+        const cudaError_t r = dalloc(&e.d_scratch, need);
         if (r != cudaSuccess) { err = cmsg("emulator scratch", r); return ST_DATA_MISSING; }
+        e.scratch_cap = need;
     }
     EmuInferArgs a;
     a.n = n; a.nb = e.nb; a.x = d_x; a.bias = e.bias; a.par = e.d_par; a.spread_max = e.spread_max; a.faint = e.faint;
