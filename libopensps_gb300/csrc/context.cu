@@ -770,6 +770,8 @@ int context_setup_grid(Context &c, std::string &err) {
     std::vector<double> lzv(c.nz);
     for (int z = 0; z < c.nz; ++z) lzv[z] = std::log10(c.zlegend[z] / c.zsol);
     cosmology_table(c.h0, c.om0, c.ol0, c.zt, c.dl);
+    std::vector<double> ages(c.log_age);   // log10 of the grid's ages, then the ages (yr)
+    for (int t = 0; t < c.nt; ++t) ages.push_back(std::pow(10.0, c.log_age[t]));
     if ((e = upload(c.d_wl, wl.data(), wl.size())) != cudaSuccess ||
         (e = upload(c.d_igm_a, igm_a.data(), igm_a.size())) != cudaSuccess ||
         (e = upload(c.d_igm_a64, igm_a64.data(), igm_a64.size())) != cudaSuccess ||
@@ -777,7 +779,7 @@ int context_setup_grid(Context &c, std::string &err) {
         (e = upload(c.d_lnlam, lnlam.data(), lnlam.size())) != cudaSuccess ||
         (e = upload(c.d_mass, c.mass.data(), c.mass.size())) != cudaSuccess ||
         (e = upload(c.d_llin, c.llin.data(), c.llin.size())) != cudaSuccess ||
-        (e = upload(c.d_logage, c.log_age.data(), c.log_age.size())) != cudaSuccess ||
+        (e = upload(c.d_logage, ages.data(), ages.size())) != cudaSuccess ||
         (e = upload(c.d_lz, lzv.data(), lzv.size())) != cudaSuccess ||
         (e = upload(c.d_lbol, c.lbol.data(), c.lbol.size())) != cudaSuccess ||
         (e = upload(c.d_zt, c.zt.data(), c.zt.size())) != cudaSuccess ||

@@ -278,6 +278,7 @@ enum { PB_LOGZSOL = 15, PB_TAGE = 16, PB_TAU = 17, PB_CONST = 18, PB_FBURST = 19
 struct SfhArgs {
     int n, nt, nz, sfh, itesc;
     const double *tf;        // nt: log10(age / yr) of the grid
+    const double *t10;       // nt: the ages (yr)
     const double *lz;        // nz: log10(Z / Zsun)
     const double *lbol;      // nz x nt: log10 L_bol of the SSPs (age fastest)
     const double *par;       // n x SFH_NCOL
@@ -287,8 +288,8 @@ struct SfhArgs {
     double *wz;              // n x nt x nz: the weights over ages and metallicities
     double *lblend;          // n x 3: log-blended L_bol (total, young, old)
     double *sfr;             // n, or null
-    double2 *mtab = nullptr; // n x nt: the main component's moments at the grid ages (sfh 1, 4, and 5's delayed
-                             // tau; null: formed serially per model)
+    double2 *mtab = nullptr; // n x (nt + 1): the main component's moments at the interval limits (sfh 1, 4, and 5's
+                             // delayed tau)
     int ntab = 0;            // the tabular SFH (sfh 2, 3): ntab rows, tab = ages (years since the start,
     const double *tab = nullptr;   // non-decreasing) then SFRs, each with one zero entry past the table
 };

@@ -102,7 +102,7 @@ __device__ __forceinline__ Dual chain(const Dual &x, double f, double df) {
 template <class T> __device__ __forceinline__ T sexp(const T &x) { const double e = exp(val(x)); return chain(x, e, e); }
 template <class T> __device__ __forceinline__ T sexpm1(const T &x) { return chain(x, expm1(val(x)), exp(val(x))); }
 template <class T> __device__ __forceinline__ T spow10(const T &x) {
-    const double e = pow(10.0, val(x));
+    const double e = exp10(val(x));
     return chain(x, e, e * SFH_LN10);
 }
 template <class T> __device__ __forceinline__ T slog10(const T &x) {
@@ -111,33 +111,60 @@ template <class T> __device__ __forceinline__ T slog10(const T &x) {
 template <class T> __device__ __forceinline__ T smax(const T &a, const T &b) { return val(a) >= val(b) ? a : b; }
 template <class T> __device__ __forceinline__ T smin(const T &a, const T &b) { return val(a) <= val(b) ? a : b; }
 
-// 1 / (k + 1)^2, k = 0 .. 1000: the power series' term ratio without an FP64 division per term (GB300's FP64 pipe is
-// narrow and the series' terms form one dependent chain)
-constexpr int SFH_NSER = 1001;
-__constant__ double c_inv_sq[SFH_NSER];
+// Ei's power series sum_k x^k / (k k!) for 0 < x <= 40 (expi, src/math/opensps_special_functions.f90:62-122) as a
+// Horner form with a fixed count of terms by the size of x: one FP64 multiply-add per term (a term's recurrence, its sum
+// and its convergence test took seven FP64 instructions, and GB300's FP64 pipe takes one every 64 cycles per SM
+// sub-partition). c_ei[k] = 1 / (k k!); c_ei_x[i]: the largest x that 8 (i + 1) terms sum to within 1e-17 of itself.
+constexpr int EI_BLOCKS = 18, EI_TERMS = 8 * EI_BLOCKS;
+__device__ double d_ei[EI_TERMS + 1];
+__device__ float d_ei_x[EI_BLOCKS];
 
-// Ei(x) (expi, src/math/opensps_special_functions.f90:62-122): the power series about 0 for x <= 40, the
-// asymptotic series (20 terms) beyond; d Ei / dx = e^x / x.
+static void ei_tables(double *c, float *xs) {
+    c[0] = 0.0;
+    double f = 1.0;
+    for (int k = 1; k <= EI_TERMS; ++k) {
+        f /= (double)k;
+        c[k] = f / (double)k;
+    }
+    for (int i = 0; i < EI_BLOCKS; ++i) {
+        const int terms = 8 * (i + 1);
+        double lo = 0.0, hi = 64.0;
+        for (int it = 0; it < 60; ++it) {
+            const double x = 0.5 * (lo + hi);
+            double t = 1.0, sum = 0.0, rest = 0.0;   // t = x^k / k!
+            for (int k = 1; k <= 400; ++k) {
+                t *= x / (double)k;
+                (k <= terms ? sum : rest) += t / (double)k;
+            }
+            (rest <= 1e-17 * sum ? lo : hi) = x;
+        }
+        xs[i] = (float)(lo * 0.999999);
+    }
+}
+
+// Ei(x): the power series about 0 for x <= 40, the asymptotic series (20 terms) beyond; d Ei / dx = e^x / x.
 __device__ double expi_d(double x) {
     if (x == 0.0) return -INFINITY;
     if (x < 0.0) return NAN;
     if (fabs(x) <= 40.0) {
-        double res = 1.0, r = 1.0;
-        for (int k = 1; k <= 1000; ++k) {
-            r = (r * (double)k * x) * c_inv_sq[k];
-            res += r;
-            if (fabs(r) <= 1.0e-20 * fabs(res)) break;
-            if (k == 1000) return NAN;
+        const float xf = (float)x;
+        int blocks = 1;
+        while (blocks < EI_BLOCKS && xf > __ldg(d_ei_x + blocks - 1)) ++blocks;
+        double r = 0.0;
+        for (int i = blocks - 1; i >= 0; --i) {
+            double c[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) c[k] = __ldg(d_ei + 8 * i + 1 + k);
+#pragma unroll
+            for (int k = 7; k >= 0; --k) r = fma(r, x, c[k]);
         }
-        return SFH_EULER_GAMMA + log(x) + x * res;
+        return SFH_EULER_GAMMA + log(x) + x * r;
     }
-    double res = 1.0, r = 1.0;
     const double inv = 1.0 / x;
-    for (int k = 1; k <= 20; ++k) {
-        r *= (double)k * inv;
-        res += r;
-    }
-    return exp(x) * inv * res;
+    double r = 1.0;
+#pragma unroll
+    for (int k = 20; k >= 1; --k) r = fma(r, (double)k * inv, 1.0);
+    return exp(x) * inv * r;
 }
 template <class T> __device__ __forceinline__ T sexpi(const T &x, bool &finite) {
     const double e = expi_d(val(x));
@@ -219,22 +246,8 @@ __device__ void moments_log(const T &log_t, const SfhT<T> &s, T &m0, T &m1) {
 
 // compute_ssp_weights (src/physics/opensps_sfh.f90:97-257) with log-age interpolation: w (nt, strided) += the hat
 // kernel masses; idx_min / idx_max 1-based as the reference's. w must start at zero.
-// The moments at limit lim = the grid age tf[j] clamped to [lts, lte]: from the table when tf[j] lies strictly
-// inside (the table's entries are moments_log at tf[j] itself), else formed here.
 template <class T>
-__device__ __forceinline__ void moments_at(const T &lim, int j, const double *tf, const T &lts, const T &lte,
-                                           const SfhT<T> &s, const double2 *mtab, T &m0, T &m1) {
-    if (mtab && val(lim) == tf[j] && tf[j] > val(lts) && tf[j] < val(lte)) {
-        m0 = lift<T>(mtab[j].x);
-        m1 = lift<T>(mtab[j].y);
-        return;
-    }
-    moments_log(lim, s, m0, m1);
-}
-
-template <class T>
-__device__ __forceinline__ void ssp_weights(const double *tf, int nt, const SfhT<T> &s, int idx_min, int idx_max, T *w, int ws,
-                            const double2 *mtab = nullptr) {
+__device__ __forceinline__ void ssp_weights(const double *tf, int nt, const SfhT<T> &s, int idx_min, int idx_max, T *w, int ws) {
     const double tiny_logt = 0.0;
     if (s.type == -1) {
         if (val(s.tb) < 0.0) return;
@@ -256,12 +269,12 @@ __device__ __forceinline__ void ssp_weights(const double *tf, int nt, const SfhT
     if (je > hi_bound) je = hi_bound;
     T lim_prev = smin(smax(lift<T>(tf[js - 1]), lts), lte);
     T m0p, m1p;
-    moments_at(lim_prev, js - 1, tf, lts, lte, s, mtab, m0p, m1p);
+    moments_log(lim_prev, s, m0p, m1p);
     for (int j = js; j <= je; ++j) {
         const T lim2 = smin(smax(lift<T>(tf[j]), lts), lte);
         if (val(lim2) <= val(lim_prev)) { lim_prev = lim2; continue; }
         T m0c, m1c;
-        moments_at(lim2, j, tf, lts, lte, s, mtab, m0c, m1c);
+        moments_log(lim2, s, m0c, m1c);
         const T m0 = m0c - m0p, m1 = m1c - m1p;
         m0p = m0c;
         m1p = m1c;
@@ -356,8 +369,7 @@ __device__ __forceinline__ void sfh_props(const double *tf, int nt, int sfh, con
 // p: tage, tau, const, fburst, tburst, sf_start, sf_trunc (Gyr), sf_slope (per Gyr). w, t1, t2: nt entries at stride
 // ws, zeroed here.
 template <class T>
-__device__ __forceinline__ void sfh_weights_core(const double *tf, int nt, int sfh, const T *p, T *w, T *t1, T *t2, int ws,
-                                 const double2 *mtab = nullptr) {
+__device__ __forceinline__ void sfh_weights_core(const double *tf, int nt, int sfh, const T *p, T *w, T *t1, T *t2, int ws) {
     for (int i = 0; i < nt; ++i) { w[i * ws] = lift<T>(0.0); t1[i * ws] = lift<T>(0.0); t2[i * ws] = lift<T>(0.0); }
     SfhT<T> s;
     sfh_setup(sfh, p, s);
@@ -371,7 +383,7 @@ __device__ __forceinline__ void sfh_weights_core(const double *tf, int nt, int s
     }
     if (sfh == 5) {
         s.type = 4;
-        ssp_weights(tf, nt, s, 0, imax, t1, ws, mtab);
+        ssp_weights(tf, nt, s, 0, imax, t1, ws);
         s.type = 5;
         s.simha = 1;
         ssp_weights(tf, nt, s, 0, imax, t2, ws);
@@ -386,7 +398,7 @@ __device__ __forceinline__ void sfh_weights_core(const double *tf, int nt, int s
         return;
     }
     s.type = sfh;
-    ssp_weights(tf, nt, s, 0, imax, w, ws, mtab);
+    ssp_weights(tf, nt, s, 0, imax, w, ws);
     T mass1 = lift<T>(0.0);
     for (int i = 0; i < imax; ++i) mass1 = mass1 + w[i * ws];
     if (val(mass1) < SAFE_FLOOR) mass1 = lift<T>(1.0);
@@ -427,32 +439,110 @@ __device__ __forceinline__ void zinterval(const double *lz, int nz, double x, in
     dz = (x - lz[zlo]) / (lz[zlo + 1] - lz[zlo]);
 }
 
-// One thread per (model, grid age): the main component's moments (sfh 1, 4; the delayed tau of sfh 5) at the grid
-// ages strictly inside the model's [log t_start, log t_age], the SFH set up as sfh_weights_core sets it, for
-// sfh_forward_kernel's table.
+// The main component's moments (sfh 1, 4; the delayed tau of sfh 5, set up as sfh_weights_core sets it) at the limits
+// sfh_forward_kernel's intervals end at, one thread per (model, limit): the grid ages clamped to the model's window
+// [max(tq, 1 yr), max(tage, 1 yr)], then the window's start (the youngest edge's lower limit), nt + 1 per model; limits
+// that no interval of positive width ends at are left out. t10 = 10^(log age) from the host. After them one thread per
+// model for the SFR, which one lane of a warp per model would take as long for as 32.
+// Bound by the FP64 pipe: about 110 instructions per limit, 612 with the series term by term, pow and logarithms per
+// limit: 116 us at 4001 models, 454 before (sfh_forward_kernel 116, 526 before).
+__device__ double sfh_sfr(const double *tf, int nt, int sfh, const double *p);
+
 __global__ void __launch_bounds__(128) sfh_moments_kernel(SfhArgs a) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)a.n * a.nt) return;
-    const int m = (int)(i / a.nt), j = (int)(i % a.nt);
+    const int nl = a.nt + 1;
+    const size_t nmom = (size_t)a.n * nl;
+    if (i >= nmom) {
+        const size_t m = i - nmom;
+        if (m < (size_t)a.n && a.sfr) a.sfr[m] = sfh_sfr(a.tf, a.nt, a.sfh, a.par + (size_t)SFH_NCOL * m);
+        return;
+    }
+    const int m = (int)(i / nl), j = (int)(i % nl);
     const double *p = a.par + (size_t)SFH_NCOL * m;
     SfhT<double> s;
     sfh_setup(a.sfh, p, s);
-    s.type = a.sfh == 5 ? 4 : a.sfh;
-    double lts, lte;
-    sfh_window(s, lts, lte);
-    const double x = a.tf[j];
+    const double tlo = smax(s.tq, 1.0), thi = smax(s.tage, 1.0);
+    double t, lt;
+    bool need = true;
+    const double tj = j < a.nt ? __ldg(a.t10 + j) : 0.0;
+    if (j == a.nt || tj <= tlo) {
+        t = fmin(tlo, thi);
+        lt = t == 1.0 ? 0.0 : log10(t);
+        need = j == a.nt || (j + 1 < a.nt && __ldg(a.t10 + j + 1) * (1.0 + 1e-9) > tlo);
+    } else if (tj >= thi) {
+        t = thi;
+        need = j == 0 || __ldg(a.t10 + j - 1) < thi * (1.0 + 1e-9);
+        lt = need ? log10(thi) : 0.0;
+    } else {
+        t = tj;
+        lt = __ldg(a.tf + j);
+    }
     double2 r = make_double2(0.0, 0.0);
-    if (x > lts && x < lte) moments_log(x, s, r.x, r.y);
+    if (need && !(s.tau <= SAFE_FLOOR)) {
+        // eval_indefinite_moments_log's types 1 and 4
+        const double tt = fmax(t / s.tau, SAFE_FLOOR);
+        bool fin;
+        const double ei = sexpi(tt, fin), e = exp(tt);
+        if (a.sfh == 1) {
+            r.x = e;
+            r.y = lt * e - SFH_LOG_E * ei;
+        } else {
+            const double q = t - s.tage - s.tau;
+            r.x = -(q * e);
+            r.y = -((q * lt - s.tau * SFH_LOG_E) * e) - (s.tage + s.tau) * SFH_LOG_E * ei;
+        }
+    }
     a.mtab[i] = r;
 }
 
+// find_interval0 of an ascending table by a warp: the entries <= v counted by ballots, with its end case.
+__device__ __forceinline__ int warp_find(const double *a, int n, double v, int lane) {
+    int c = 0;
+    for (int i = 0; i < n; i += 32) c += __popc(__ballot_sync(0xffffffffu, i + lane < n && v >= __ldg(a + i + lane)));
+    return v == __ldg(a + n - 1) ? n - 2 : c - 1;
+}
+
+// The main component's weights over ages by a warp from its moments at every limit (mtab, nt + 1 entries): interval
+// j = 1 .. nt - 1's shares A_j = (hi d0 - d1) / dt to w[j - 1] and B_j = (d1 - lo d0) / dt to w[j] (d0, d1 the moments'
+// differences over the interval; intervals of zero width skipped), then w[i] = B_i + A_(i+1) and the youngest edge, the
+// sums of the reference's loop in its order. lte: log10 of the model's age. A, B: the warp's scratch.
+__device__ __forceinline__ void warp_main_component(const double *tf, int nt, const SfhT<double> &s, int imax, double lts,
+                                                    double lte, const double2 *mtab, double *A, double *B, double *wout,
+                                                    int lane) {
+    const int hi_bound = imax < nt - 1 ? imax : nt - 1;
+    const int js = max(warp_find(tf, nt, lts, lane) + 1, 1), je = min(warp_find(tf, nt, lte, lane) + 2, hi_bound);
+    for (int j = lane; j <= nt; j += 32) {
+        double av = 0.0, bv = 0.0;
+        if (j >= js && j <= je) {
+            const double lo = __ldg(tf + j - 1), hi = __ldg(tf + j);
+            if (fmin(fmax(hi, lts), lte) > fmin(fmax(lo, lts), lte)) {
+                const double2 c = __ldg(mtab + j), q = __ldg(mtab + j - 1);
+                const double d0 = c.x - q.x, d1 = c.y - q.y, inv = 1.0 / (hi - lo);
+                av = (hi * d0 - d1) * inv;
+                bv = (d1 - lo * d0) * inv;
+            }
+        }
+        A[j] = av;
+        B[j] = bv;
+    }
+    __syncwarp();
+    for (int i = lane; i < nt; i += 32) {
+        double v = B[i] + A[i + 1];
+        if (i == 0) {
+            const double l2 = fmin(fmax(__ldg(tf), lts), lte);
+            if (fmin(lts, lte) < l2) v += __ldg(&mtab[0].x) - __ldg(&mtab[nt].x);
+        }
+        wout[i] = v;
+    }
+    __syncwarp();
+}
+
 // One component's weights over ages by a warp (ssp_weights for T = double, idx_min 0 or the SSP's window): the
-// moments at every boundary of its intervals (the table's, or formed here at the clamped ends), then per age
+// moments at every boundary of its intervals, then per age
 // w[i] = B_i + A_(i+1), interval j's shares A_j = (hi d0 - d1) / dt to w[j - 1] and B_j = (d1 - lo d0) / dt to w[j]
 // (d0, d1 the moments' differences over the interval; intervals of zero width skipped): the sums the serial loop
 // forms, in its order. wout[0 .. nt) is written in full; M0s / M1s are the warp's scratch.
-__device__ void warp_component(const double *tf, int nt, const SfhT<double> &s, int idx_min, int idx_max,
-                               const double2 *mtab, double *M0s, double *M1s, double *wout, int lane) {
+__device__ void warp_component(const double *tf, int nt, const SfhT<double> &s, int idx_min, int idx_max, double *M0s, double *M1s, double *wout, int lane) {
     for (int i = lane; i < nt; i += 32) wout[i] = 0.0;
     __syncwarp();
     if (s.type == -1) {
@@ -482,7 +572,7 @@ __device__ void warp_component(const double *tf, int nt, const SfhT<double> &s, 
         if (j >= js - 1 && j <= je) {
             const double lim = fmin(fmax(tf[j], lts), lte);
             double m0, m1;
-            moments_at(lim, j, tf, lts, lte, s, mtab, m0, m1);
+            moments_log(lim, s, m0, m1);
             M0s[j] = m0;
             M1s[j] = m1;
         }
@@ -535,7 +625,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 constexpr int SFH_WARPS = 4;
 constexpr int SFH_WMAXT = 128;
 __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) {
-    __shared__ double sm[SFH_WARPS][5][SFH_WMAXT];
+    __shared__ double sm[SFH_WARPS][5][SFH_WMAXT + 1];
     const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
     const int m = blockIdx.x * SFH_WARPS + wi;
     if (m >= a.n) return;
@@ -551,20 +641,23 @@ __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) 
         const int sfh = a.sfh;
         SfhT<double> s;
         sfh_setup(sfh, p, s);
-        int imax = find_interval0(a.tf, nt, log10(s.tage)) + 1 + 2;
+        // the window in log10 lookback years (sfh_window); below 1 yr the index of log10(tage) is the grid's start
+        const double lte = log10(smax(s.tage, 1.0)), lts = s.tq > 1.0 ? log10(s.tq) : 0.0;
+        int imax = (s.tage >= 1.0 ? warp_find(a.tf, nt, lte, lane) : find_interval0(a.tf, nt, log10(s.tage))) + 1 + 2;
         imax = imax < 1 ? 1 : (imax > nt ? nt : imax);
+        const double2 *mt = a.mtab ? a.mtab + (size_t)(nt + 1) * m : nullptr;
         if (sfh == 0) {
             s.type = -1;
             s.tb = s.tage;
-            warp_component(a.tf, nt, s, imax - 2 > 1 ? imax - 2 : 1, imax, nullptr, M0s, M1s, w, lane);
+            warp_component(a.tf, nt, s, imax - 2 > 1 ? imax - 2 : 1, imax, M0s, M1s, w, lane);
         } else if (sfh == 5) {
             // the delayed tau over [tq, tage] and the ramp over [t0, tq], each normalised, mixed by the ramp's
             // mass fraction at tage
             s.type = 4;
-            warp_component(a.tf, nt, s, 0, imax, a.mtab ? a.mtab + (size_t)nt * m : nullptr, M0s, M1s, t1, lane);
+            warp_main_component(a.tf, nt, s, imax, lts, lte, mt, M0s, M1s, t1, lane);
             s.type = 5;
             s.simha = 1;
-            warp_component(a.tf, nt, s, 0, imax, nullptr, M0s, M1s, t2, lane);
+            warp_component(a.tf, nt, s, 0, imax, M0s, M1s, t2, lane);
             double p1 = 0.0, p2 = 0.0;
             for (int i = lane; i < imax; i += 32) { p1 += t1[i]; p2 += t2[i]; }
             double mass1 = warp_sum(p1), mass2 = warp_sum(p2);
@@ -577,17 +670,18 @@ __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) 
             __syncwarp();
         } else {
             s.type = sfh;
-            warp_component(a.tf, nt, s, 0, imax, a.mtab ? a.mtab + (size_t)nt * m : nullptr, M0s, M1s, w, lane);
+            warp_main_component(a.tf, nt, s, imax, lts, lte, mt, M0s, M1s, w, lane);
             double part = 0.0;
             for (int i = lane; i < imax; i += 32) part += w[i];
             double mass1 = warp_sum(part);
             if (mass1 < SAFE_FLOOR) mass1 = 1.0;
-            for (int i = lane; i < nt; i += 32) w[i] = w[i] / mass1;
+            const double inv_mass = 1.0 / mass1;
+            for (int i = lane; i < nt; i += 32) w[i] *= inv_mass;
             __syncwarp();
             const double cst = p[SFH_CONST], fb_in = p[SFH_FBURST];
             if (cst > 0.0 || fb_in > SAFE_FLOOR) {
                 s.type = 0;
-                warp_component(a.tf, nt, s, 0, imax, nullptr, M0s, M1s, t1, lane);
+                warp_component(a.tf, nt, s, 0, imax, M0s, M1s, t1, lane);
                 part = 0.0;
                 for (int i = lane; i < imax; i += 32) part += t1[i];
                 double m1 = warp_sum(part);
@@ -595,7 +689,7 @@ __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) 
                 double fb = 0.0;
                 if (s.tb >= 0.0) {
                     s.type = -1;
-                    warp_component(a.tf, nt, s, 0, imax, nullptr, M0s, M1s, t2, lane);
+                    warp_component(a.tf, nt, s, 0, imax, M0s, M1s, t2, lane);
                     fb = fb_in;
                 } else {
                     for (int i = lane; i < nt; i += 32) t2[i] = 0.0;
@@ -605,13 +699,13 @@ __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) 
                 __syncwarp();
             }
         }
-        if (lane == 0 && a.sfr) a.sfr[m] = sfh_sfr(a.tf, nt, sfh, p);
+        if (!a.mtab && lane == 0 && a.sfr) a.sfr[m] = sfh_sfr(a.tf, nt, sfh, p);
     }
     double *wg = a.w + (size_t)nt * m;
     for (int i = lane; i < nt; i += 32) wg[i] = w[i];
-    int zlo;
-    double dz;
-    zinterval(a.lz, nz, p[SFH_LOGZSOL], zlo, dz);
+    const double lzs = p[SFH_LOGZSOL];
+    const int zi = warp_find(a.lz, nz, lzs, lane) + 1, zlo = (zi < 1 ? 1 : (zi > nz - 1 ? nz - 1 : zi)) - 1;
+    const double dz = (lzs - a.lz[zlo]) / (a.lz[zlo + 1] - a.lz[zlo]);
     double *wz = a.wz + (size_t)nt * nz * m;
     for (int k = lane; k < nt * nz; k += 32) {
         const int z = k / nt, t = k - z * nt;
@@ -626,7 +720,7 @@ __global__ void __launch_bounds__(SFH_WARPS * 32) sfh_forward_kernel(SfhArgs a) 
     for (int t = lane; t < nt; t += 32) {
         const double wt = w[t];
         if (!(wt > SAFE_FLOOR)) continue;
-        const double lk = wt * pow(10.0, (1.0 - dz) * a.lbol[t + (size_t)nt * zlo] + dz * a.lbol[t + (size_t)nt * (zlo + 1)]);
+        const double lk = wt * exp10((1.0 - dz) * a.lbol[t + (size_t)nt * zlo] + dz * a.lbol[t + (size_t)nt * (zlo + 1)]);
         ls += lk;
         if (t < a.itesc) ly += lk; else lo += lk;
     }
@@ -751,9 +845,12 @@ static cudaError_t sfh_init_tables(cudaStream_t st) {
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> lk(mu);
     if (dev < 64 && done[dev]) return cudaSuccess;
-    static double h[SFH_NSER];
-    for (int k = 0; k < SFH_NSER; ++k) h[k] = 1.0 / (((double)k + 1.0) * ((double)k + 1.0));
-    if ((e = cudaMemcpyToSymbolAsync(c_inv_sq, h, sizeof(h), 0, cudaMemcpyHostToDevice, st)) != cudaSuccess) return e;
+    static double c[EI_TERMS + 1];
+    static float xs[EI_BLOCKS];
+    ei_tables(c, xs);
+    if ((e = cudaMemcpyToSymbolAsync(d_ei, c, sizeof(c), 0, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+        (e = cudaMemcpyToSymbolAsync(d_ei_x, xs, sizeof(xs), 0, cudaMemcpyHostToDevice, st)) != cudaSuccess)
+        return e;
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return e;
     if (dev < 64) done[dev] = true;
     return cudaSuccess;
@@ -766,7 +863,7 @@ cudaError_t run_sfh_forward(const SfhArgs &a, cudaStream_t st) {
     SfhArgs b = a;
     if (a.given || (a.sfh != 1 && a.sfh != 4 && a.sfh != 5)) b.mtab = nullptr;
     if (b.mtab) {
-        const size_t tot = (size_t)a.n * a.nt;
+        const size_t tot = (size_t)a.n * (a.nt + 2);   // limits, then the models' SFRs
         sfh_moments_kernel<<<(unsigned)((tot + 127) / 128), 128, 0, st>>>(b);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -813,7 +910,7 @@ __global__ void __launch_bounds__(64) sfh_reverse_kernel(SfhRevArgs a) {
         gz += w[t] * (b1 - b0);
         if (lbar != 0.0 && w[t] > SAFE_FLOOR) {
             const double l0 = a.lbol[t + (size_t)nt * zlo], l1 = a.lbol[t + (size_t)nt * (zlo + 1)];
-            const double lt = pow(10.0, (1.0 - dz) * l0 + dz * l1);
+            const double lt = exp10((1.0 - dz) * l0 + dz * l1);
             g += lbar * lt;
             gz += lbar * w[t] * lt * SFH_LN10 * (l1 - l0);
         }
