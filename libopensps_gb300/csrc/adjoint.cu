@@ -761,6 +761,8 @@ cudaError_t run_transpose_bf16(const __nv_bfloat16 *src, __nv_bfloat16 *dst, int
 // (ln 10 L_bol) plus the AGN's (backward_age_sums_w; the ssp_weights_z branch of compute_csp_batch's reverse pass).
 struct WzbArgs {
     int n_models, ntz, ldd;
+    int ky = 0, ks_young = 1, ks_old = 1;   // columns below ky in ks_young partial sums, the others in ks_old, each
+    size_t d_split = 0;                     // d_split elements after the one before
     const float *D;
     const int *col_of;
     const double *cscale, *mass_bar, *lbol_bar, *sums, *mass, *llin;
@@ -772,7 +774,13 @@ __global__ void wzbar_kernel(WzbArgs a) {
     if (i >= (size_t)a.n_models * a.ntz) return;
     const int m = (int)(i / a.ntz), k = (int)(i % a.ntz);
     double v = 0.0;
-    if (a.D) v = a.cscale[m] * (double)a.D[(size_t)m * a.ldd + a.col_of[k]];
+    if (a.D) {
+        const int col = a.col_of[k], ks = col < a.ky ? a.ks_young : a.ks_old;
+        const float *d = a.D + (size_t)m * a.ldd + col;
+        float f = 0.f;
+        for (int s = 0; s < ks; ++s) f += __ldg(d + (size_t)s * a.d_split);
+        v = a.cscale[m] * (double)f;
+    }
     if (a.mass_bar) v += a.mass_bar[m] * a.mass[k];
     if (a.lbol_bar) {
         const double ls = a.sums[(size_t)6 * m + 1];
@@ -1018,7 +1026,12 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         // then the reverse fold: the weights' cotangent at every grid point (when wanted) and the slopes' rows
         const SspOps &o = c.ops;
         const bool want_wzb = weights_z_bar || sfh_rev;
-        if ((e = c.d_vbar.reserve((size_t)2 * n * o.ntpad)) != cudaSuccess ||
+        // (few output tiles: the K blocks split over the SMs, the partial sums added with the bf16 split: 38 us instead of
+        // 213 at 100 models; the exact fold's reverse reads whole sums)
+        const int tiles = ((n + gemm_bm() - 1) / gemm_bm()) * ((o.ntpad + gemm_bn() - 1) / gemm_bn());
+        const int ks = c.ops_last_interp ? gemm_choose_ksplit(tiles, ppad / gemm_bk(), c.num_sms) : 1;
+        const size_t vper = (size_t)n * o.ntpad;
+        if ((e = c.d_vbar.reserve(2 * ks * vper)) != cudaSuccess ||
             (e = c.d_apart.reserve((size_t)c.nz * n * 3)) != cudaSuccess ||
             (want_wzb && (e = c.d_wzbar.reserve((size_t)n * ntz)) != cudaSuccess)) {
             err = msg("device memory", e);
@@ -1027,7 +1040,7 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         for (int part = 0; part < 2; ++part) {
             GemmArgs g;
             g.M = n; g.N = o.ntpad; g.K = ppad; g.ldd = o.ntpad; g.b_row0 = 0; g.status = c.d_status.p;
-            g.D = c.d_vbar.p + (size_t)part * n * o.ntpad;
+            g.D = c.d_vbar.p + (size_t)part * ks * vper; g.ksplit = ks; g.d_split = (long long)vper;
             GemmPlan pl;
             pl.num_sms = c.num_sms;
             pl.tm_b_hi = o.tm_lib_thi;
@@ -1046,7 +1059,7 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         r.n = n; r.nt = c.nt; r.nz = c.nz; r.npt = o.npt; r.ntpad = o.ntpad; r.itesc = c.geom.itesc; r.imf_type = c.imf_type;
         if (int rc = ops_imf_limits(c, c.imf_type, r.lim, err)) return rc;   // (the forward's limits and user IMF)
         r.wz = c.geom.wz; r.alpha = c.d_alpha.p; r.pts = o.pts.p; r.pidx = o.pidx.p; r.pcoef = o.pcoef.p;
-        r.vbar = c.d_vbar.p; r.cscale = c.d_cscale.p;
+        r.vbar = c.d_vbar.p; r.vsplit = ks; r.cscale = c.d_cscale.p;
         r.mass_bar = mass_bar ? c.d_mass_bar.p : nullptr;
         r.lbol_bar = lbol_bar ? c.d_lbol_bar.p : nullptr;   // (L_bol with the operators: the linear row, always)
         r.lsum_bar = c.geom.agn ? c.d_lsum_bar.p : nullptr;
@@ -1069,7 +1082,16 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
             return ST_DATA_MISSING;
         }
     } else if (weights_z_bar || sfh_rev) {
-        if ((e = c.d_wzb32.reserve((size_t)n * kpad)) != cudaSuccess || (e = c.d_wzbar.reserve((size_t)n * ntz)) != cudaSuccess) {
+        // (few output tiles: the K blocks split over the SMs, the partial sums added by wzbar_kernel: at 2000 models 131 us
+        // for the two GEMMs and the sum, 239 without)
+        int ks[2];
+        for (int part = 0; part < 2; ++part) {
+            const int cols = part == 0 ? bop->ky_pad : kpad - bop->ky_pad;
+            const int tiles = ((n + gemm_bm() - 1) / gemm_bm()) * ((cols + gemm_bn() - 1) / gemm_bn());
+            ks[part] = cols > 0 ? gemm_choose_ksplit(tiles, ppad / gemm_bk(), c.num_sms) : 1;
+        }
+        const size_t dper = (size_t)n * kpad;
+        if ((e = c.d_wzb32.reserve(std::max(ks[0], ks[1]) * dper)) != cudaSuccess || (e = c.d_wzbar.reserve((size_t)n * ntz)) != cudaSuccess) {
             err = msg("device memory", e);
             return ST_DATA_MISSING;
         }
@@ -1079,6 +1101,8 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
             g.N = part == 0 ? bop->ky_pad : kpad - bop->ky_pad;
             g.b_row0 = part == 0 ? 0 : bop->ky_pad;
             g.D = c.d_wzb32.p + (part == 0 ? 0 : bop->ky_pad);
+            g.ksplit = ks[part];
+            g.d_split = (long long)dper;
             if (g.N <= 0) continue;
             GemmPlan pl;
             pl.num_sms = c.num_sms;
@@ -1095,7 +1119,7 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         }
         prof_mark(c, 8);
         WzbArgs w;
-        w.n_models = n; w.ntz = ntz; w.ldd = kpad; w.D = c.d_wzb32.p; w.col_of = bop->col_of.p;
+        w.n_models = n; w.ntz = ntz; w.ldd = kpad; w.D = c.d_wzb32.p; w.ky = bop->ky_pad; w.ks_young = ks[0]; w.ks_old = ks[1]; w.d_split = dper; w.col_of = bop->col_of.p;
         w.cscale = c.d_cscale.p; w.mass_bar = mass_bar ? c.d_mass_bar.p : nullptr;
         // (the log-blended L_bol of weights formed on the device has its own cotangent, in the SFH reverse pass)
         w.lbol_bar = (lbol_bar && !dev_blend) ? c.d_lbol_bar.p : nullptr;

@@ -304,6 +304,7 @@ struct Context {
     DevBuf<__nv_bfloat16> d_ix_hi, d_ix_lo;   // the interpolated fold's operand: node values x SFH weights
     DevBuf<float> d_ipart;       // and its GEMM's split-K partial sums
     DevBuf<double2> d_ix_const;  // and each model's 1 / T and c2
+    DevBuf<double> d_ix_dln;     // and d ln T / d alpha (the reverse pass)
     DevBuf<DustEmModel> d_dem;   // the batch's dust emission cells (one per model)
     DevBuf<float> d_bpart;       // the band GEMM's partial fluxes when it splits the pixels (few models)
     DevBuf<float> d_vbar;        // reverse pass with operators: 2n x ntpad template cotangents (young, old)

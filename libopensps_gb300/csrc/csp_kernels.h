@@ -202,6 +202,7 @@ struct GemmPlan {
 int gemm_bk();
 int gemm_bm();
 int gemm_bn();
+int gemm_choose_ksplit(int tiles_mn, int nkb, int num_sms);
 cudaError_t run_gemm_bf16x3(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st);   // three products (hi / lo)
 cudaError_t run_gemm_bf16(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st);     // one product (hi only)
 
@@ -375,7 +376,8 @@ struct OpsRevArgs {
     const OpsPoint *pts;      // (nt x nz) x npt
     const ushort4 *pidx;      // (nt x nz) x npt: each point's four templates
     const float4 *pcoef;      // and their coefficients
-    const float *vbar;        // 2n x ntpad: the template weights' cotangents / cscale (young rows, then old)
+    const float *vbar;        // 2n x ntpad: the template weights' cotangents / cscale (young rows, then old); with
+    int vsplit = 1;           // vsplit > 1 that many partial sums of the young rows, then of the old (interpolated only)
     const double *cscale;     // n: the reverse pass's cotangent scale
     const double *mass_bar, *lbol_bar;   // n each, or null
     const double *lsum_bar = nullptr;    // n: the AGN's cotangent of the linear L_bol row (absolute), or null

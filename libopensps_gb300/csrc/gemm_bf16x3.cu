@@ -18,6 +18,7 @@
 // four of 48 KB (plain). Every mbarrier wait is bounded (status word, no hang).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
+#include <algorithm>
 #include <cstdint>
 #include "sm103_ptx.cuh"
 #include "csp_kernels.h"
@@ -198,6 +199,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
 int gemm_bk() { return G_BK; }
 int gemm_bm() { return G_BM; }
 int gemm_bn() { return G_BN; }
+
+// K splits for a GEMM of tiles_mn output tiles over nkb K blocks: the fewest giving at least two waves over the SMs
+// with the last wave at least 85% full (else the fullest last wave), each split keeping 8 or more K blocks.
+int gemm_choose_ksplit(int tiles_mn, int nkb, int num_sms) {
+    int best = 1;
+    double best_eff = -1.0;
+    const int cap = std::max(1, std::min(64, nkb / 8));
+    for (int ks = 1; ks <= cap; ++ks) {
+        const long long tiles = (long long)tiles_mn * ks, waves = (tiles + num_sms - 1) / num_sms;
+        const double eff = (double)tiles / (double)(waves * num_sms);
+        if (tiles >= 2LL * num_sms && eff >= 0.85) return ks;
+        if (eff > best_eff + 1e-9) { best_eff = eff; best = ks; }
+    }
+    return best;
+}
 
 template <int NPROD>
 static cudaError_t launch_gemm(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) {

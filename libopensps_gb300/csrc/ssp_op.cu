@@ -655,22 +655,48 @@ constexpr int OPS_IMAXR = 256;                       // nodes per grid point (R 
 // point gp = q / (R / 8) (by a multiply-high with rg_magic = 2^32 / (R / 8) rounded up; exact for q < 2^20).
 constexpr int OPS_IMAXG = 4096;                      // grid points (nt nz <= OPS_IMAXG)
 
-// One thread per model: 1 / T (the IMF's mass between its limits, FP64) and c2 = 0.5^(alpha2 - alpha1), for
-// ops_interp_x_kernel (formed there by one thread per CTA, the FP64 work ran as one-lane warps).
-__global__ void ops_interp_const_kernel(const double *alpha, int n, float lim_lo, float lim_hi, double fixed_inv_total,
-                                        double2 *out) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= n) return;
-    if (fixed_inv_total > 0.0) {   // an IMF without per-model parameters (Chabrier): its 1 / T, formed on the host
-        out[m] = make_double2(fixed_inv_total, 0.0);
+// Per model: 1 / T (the IMF's mass between its limits, FP64) and c2 = 0.5^(alpha2 - alpha1), for ops_interp_x_kernel,
+// and with dln the derivatives d ln T / d alpha_j for the reverse pass. Four lanes per model, a Kroupa segment each: a
+// chain of FP64 powers on one thread per model took 24 us at 1024 models (the FP64 pipe takes a warp instruction every
+// 64 cycles), this 5. ll, dl: the segments' ln(lower mass) and ln(upper / lower).
+struct OpsConstArgs {
+    int n;
+    double ll[3], dl[3], fixed_inv_total;
+    const double *alpha;
+    double2 *out;
+    double *dln;              // n x 3, or null
+};
+__global__ void __launch_bounds__(128) ops_interp_const_kernel(OpsConstArgs a) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, m = i >> 2, sg = min(i & 3, 2);
+    const bool live = m < a.n;
+    if (a.fixed_inv_total > 0.0) {   // an IMF without per-model parameters (Chabrier): its 1 / T, formed on the host
+        if (live && (i & 3) == 0) a.out[m] = make_double2(a.fixed_inv_total, 0.0);
+        if (live && (i & 3) < 3 && a.dln) a.dln[3 * (size_t)m + sg] = 0.0;
         return;
     }
-    KroupaSeg ks;
-    float itf;
-    double total;
-    const double *al = alpha + 3 * (size_t)m;
-    kroupa_setup(al, lim_lo, lim_hi, ks, itf, nullptr, &total);
-    out[m] = make_double2(total > 0.0 ? 1.0 / total : 1.0, pow(0.5, -al[0] + al[1]));
+    const double *al = a.alpha + 3 * (size_t)(live ? m : 0);
+    const double al_s = al[sg], em = 2.0 - al_s, c2 = exp2(al[0] - al[1]);   // mass-weighted: int c m^(1 - alpha) dm
+    const double ll = a.ll[sg], dl = a.dl[sg], x = em * dl;
+    const double f = (sg > 0 ? c2 : 1.0) * exp(em * ll) * dl, piece = f * kr_g1(x);
+    const unsigned base = (threadIdx.x & 31) & ~3u;
+    const double p0 = __shfl_sync(0xffffffffu, piece, base), p1 = __shfl_sync(0xffffffffu, piece, base + 1),
+                 p2 = __shfl_sync(0xffffffffu, piece, base + 2);
+    const double total = p0 + p1 + p2;
+    if (live && (i & 3) == 0) a.out[m] = make_double2(total > 0.0 ? 1.0 / total : 1.0, c2);
+    if (a.dln && live && (i & 3) < 3) {
+        const double dp = f * (ll * kr_g1(x) + dl * kr_g2(x)), t12 = p1 + p2, it = total > 0.0 ? 1.0 / total : 0.0;
+        a.dln[3 * (size_t)m + sg] = (sg == 0 ? KR_LN2 * t12 - dp : sg == 1 ? -dp - KR_LN2 * t12 : -dp) * it;
+    }
+}
+static cudaError_t run_ops_interp_const(int n, const double *alpha, double fixed_inv_total, double2 *out, double *dln,
+                                        cudaStream_t st) {
+    OpsConstArgs a;
+    a.n = n;
+    const double lo[3] = {0.08, 0.5, 1.0}, hi[3] = {0.5, 1.0, 120.0};
+    for (int s = 0; s < 3; ++s) { a.ll[s] = std::log(lo[s]); a.dl[s] = std::log(hi[s] / lo[s]); }
+    a.fixed_inv_total = fixed_inv_total; a.alpha = alpha; a.out = out; a.dln = dln;
+    ops_interp_const_kernel<<<(4 * n + 127) / 128, 128, 0, st>>>(a);
+    return cudaGetLastError();
 }
 // A node's value for the fold: the IMF per unit mass at mu = e^x of segment q, over T (it = 1 / T). Kroupa (and
 // Salpeter as Kroupa with equal slopes): c_q mu^-alpha_q (c = 1, c2, c2). Chabrier 2003 (imf_integral case 1,
@@ -1029,54 +1055,49 @@ struct OpsInterpRevArgs {
     size_t ktot;
     int noff[3], nn[3];
     double x0[3], h[3];
-    float lim_lo, lim_hi;
     const double *wz, *alpha, *cscale, *mass_bar, *lbol_bar, *lsum_bar, *sums;
     const double2 *kconst;                   // n: 1 / T and c2 (the forward's)
+    const double *dln;                       // n x 3: d ln T / d alpha_j
     const float *xbar;                       // rows x ktot: Vbar B of the chunk
     const float *mrow, *lrow;
     double *wzb;                             // n x nt x nz, or null
     double *params_bar;                      // n x rows, or null
     int rows, row_imf1;
 };
-constexpr int OPS_IR_THREADS = 256, OPS_IR_WARPS = OPS_IR_THREADS / 32, OPS_IR_RI = OPS_IMAXR / 32;
-
-// One model per CTA: the node values and their log-derivatives in shared memory; warp w takes grid points w, w + 8,
-// ..., lane l the nodes l + 32 i of each (the row of Xbar read once, coalesced): wz_bar(g) by a warp sum, Y(r) in
-// FP32 per lane over 64 grid points at a time (GB300's FP64 pipe is narrow), then FP64; the slopes' sums over the
-// nodes by a block reduction.
-__global__ void __launch_bounds__(OPS_IR_THREADS) ops_interp_rev_kernel(OpsInterpRevArgs a) {
-    __shared__ float ct[OPS_IMAXR];
-    __shared__ float dlc[3][OPS_IMAXR];
+// One model per CTA: the node values and their log-derivatives in shared memory; warp w takes grid points w, w + WARPS,
+// ..., four at a time, lane l the nodes l + 32 i of each (the row of Xbar read once, coalesced): wz_bar(g) by a warp
+// sum, Y(r) in FP32 per lane over 64 grid points at a time (GB300's FP64 pipe is narrow), then FP64; the slopes' sums
+// over the nodes by a block reduction. RI = ceil(R / 32) loads per grid point; with 80 nodes 32 warps, so that a small
+// batch's CTAs cover the row's latency (100 models: 194 us with eight warps, a grid point at a time and d ln T on one
+// thread, now 55).
+template <int RI, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) ops_interp_rev_kernel(OpsInterpRevArgs a) {
+    constexpr int THREADS = WARPS * 32, MAXR = RI * 32, GS = 4;
+    __shared__ float ct[MAXR];
+    __shared__ float dlc[3][MAXR];
     __shared__ float sws[OPS_IMAXG];
-    __shared__ double ypart[OPS_IR_WARPS][OPS_IMAXR];
-    __shared__ double red[OPS_IR_WARPS][3];
-    __shared__ double dlnT_s[3];
-    __shared__ float qm_s, ql_s;
+    __shared__ double ypart[WARPS][MAXR];
+    __shared__ double red[WARPS][3];
     const int row = blockIdx.x, m = a.m0 + row, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int ng = a.nt * a.nz;
-    const double *al = a.alpha + 3 * (size_t)m;
+    const double *al = a.alpha + 3 * (size_t)m, *dln = a.dln + 3 * (size_t)m;
     const double *wzm = a.wz + (size_t)ng * m;
-    for (int g = tid; g < ng; g += OPS_IR_THREADS) {
+    for (int g = tid; g < ng; g += THREADS) {
         const int t = g % a.nt, z = g / a.nt;                 // the weights' order: age fastest
         const double sw = wzm[g];
         sws[t * a.nz + z] = sw > SAFE_FLOOR ? (float)sw : 0.f;   // the columns' order: (t nz + z)
     }
     const double cs = a.cscale[m];
-    if (tid == 0) {
-        KroupaSeg ks;
-        float itf;
-        double dl[3];
-        kroupa_setup(al, a.lim_lo, a.lim_hi, ks, itf, dl);
-        for (int j = 0; j < 3; ++j) dlnT_s[j] = dl[j];
+    const float qm = a.mass_bar ? (float)(a.mass_bar[m] / cs) : 0.f;
+    float ql = 0.f;
+    if (a.lbol_bar || a.lsum_bar) {
         const double ls = a.sums[(size_t)6 * m + 1];
-        qm_s = a.mass_bar ? (float)(a.mass_bar[m] / cs) : 0.f;
         double qlv = (a.lbol_bar && ls > SAFE_FLOOR) ? a.lbol_bar[m] / (ls * 2.302585092994046) : 0.0;
         if (a.lsum_bar) qlv += a.lsum_bar[m];   // (the AGN's L_bol scale)
-        ql_s = (float)(qlv / cs);
+        ql = (float)(qlv / cs);
     }
-    __syncthreads();
     const double2 kc = a.kconst[m];                  // 1 / T, c2
-    for (int r = tid; r < OPS_IMAXR; r += OPS_IR_THREADS) {
+    for (int r = tid; r < MAXR; r += THREADS) {
         float v = 0.f, d[3] = {0.f, 0.f, 0.f};
         if (r < a.R) {
 #pragma unroll
@@ -1086,7 +1107,7 @@ __global__ void __launch_bounds__(OPS_IR_THREADS) ops_interp_rev_kernel(OpsInter
                     const double x = a.x0[q] + (double)(j - OPS_IDEG / 2) * a.h[q];
                     v = (float)ops_node_value(a.imf_type, q, x, al, kc.x, kc.y);
                     if (a.imf_type == 2) {   // (the slopes act with Kroupa only)
-                        double g3[3] = {-dlnT_s[0], -dlnT_s[1], -dlnT_s[2]};
+                        double g3[3] = {-dln[0], -dln[1], -dln[2]};
                         g3[q] -= x;
                         if (q > 0) { g3[0] += KR_LN2; g3[1] -= KR_LN2; }
                         d[0] = (float)g3[0]; d[1] = (float)g3[1]; d[2] = (float)g3[2];
@@ -1098,78 +1119,133 @@ __global__ void __launch_bounds__(OPS_IR_THREADS) ops_interp_rev_kernel(OpsInter
         dlc[0][r] = d[0]; dlc[1][r] = d[1]; dlc[2][r] = d[2];
     }
     __syncthreads();
-    const float qm = qm_s, ql = ql_s;
+    const bool rows_in = qm != 0.f || ql != 0.f;     // the mass and L_bol rows' shares (read only then)
     const float *xr = a.xbar + (size_t)row * a.ktot;
-    float y[OPS_IR_RI];
-    double yd[OPS_IR_RI];
+    float y[RI], c[RI];
+    double yd[RI];
 #pragma unroll
-    for (int i = 0; i < OPS_IR_RI; ++i) { y[i] = 0.f; yd[i] = 0.0; }
+    for (int i = 0; i < RI; ++i) { y[i] = 0.f; yd[i] = 0.0; c[i] = ct[lane + 32 * i]; }
     int nstep = 0;
-    for (int g = warp; g < ng; g += OPS_IR_WARPS) {
-        const float sw = sws[g];
-        const size_t base = (size_t)g * a.R;
-        float ws = 0.f;
+    for (int g0 = warp; g0 < ng; g0 += GS * WARPS) {
+        float x[GS][RI], sw[GS];
 #pragma unroll
-        for (int i = 0; i < OPS_IR_RI; ++i) {
-            const int r = lane + 32 * i;
-            if (r < a.R) {
-                const float xt = fmaf(qm, __ldg(a.mrow + base + r), fmaf(ql, __ldg(a.lrow + base + r), __ldg(xr + base + r)));
-                ws = fmaf(xt, ct[r], ws);
-                y[i] = fmaf(sw, xt, y[i]);
+        for (int k = 0; k < GS; ++k) {
+            const int g = g0 + k * WARPS;
+            const bool in = g < ng;
+            sw[k] = in ? sws[g] : 0.f;
+#pragma unroll
+            for (int i = 0; i < RI; ++i) {
+                const int r = lane + 32 * i;
+                x[k][i] = in && r < a.R ? __ldg(xr + (size_t)g * a.R + r) : 0.f;
+            }
+        }
+        if (rows_in) {
+#pragma unroll
+            for (int k = 0; k < GS; ++k) {
+                const int g = g0 + k * WARPS;
+#pragma unroll
+                for (int i = 0; i < RI; ++i) {
+                    const int r = lane + 32 * i;
+                    if (g < ng && r < a.R) {
+                        const size_t q = (size_t)g * a.R + r;
+                        x[k][i] = fmaf(qm, __ldg(a.mrow + q), fmaf(ql, __ldg(a.lrow + q), x[k][i]));
+                    }
+                }
+            }
+        }
+        float ws[GS];
+#pragma unroll
+        for (int k = 0; k < GS; ++k) {
+            ws[k] = 0.f;
+#pragma unroll
+            for (int i = 0; i < RI; ++i) {
+                ws[k] = fmaf(x[k][i], c[i], ws[k]);
+                y[i] = fmaf(sw[k], x[k][i], y[i]);
             }
         }
         if (a.wzb) {
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) ws += __shfl_xor_sync(0xffffffffu, ws, off);
-            if (lane == 0) {
-                const int t = g / a.nz, z = g - t * a.nz;
-                a.wzb[(size_t)ng * m + t + (size_t)a.nt * z] = cs * (double)ws;
+            for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+                for (int k = 0; k < GS; ++k) ws[k] += __shfl_xor_sync(0xffffffffu, ws[k], off);
+#pragma unroll
+            for (int k = 0; k < GS; ++k) {
+                const int g = g0 + k * WARPS;
+                if (lane == k && g < ng) {
+                    const int t = g / a.nz, z = g - t * a.nz;
+                    a.wzb[(size_t)ng * m + t + (size_t)a.nt * z] = cs * (double)ws[k];
+                }
             }
         }
-        if (++nstep == 64) {
+        if ((nstep += GS) == 64) {
 #pragma unroll
-            for (int i = 0; i < OPS_IR_RI; ++i) { yd[i] += (double)y[i]; y[i] = 0.f; }
+            for (int i = 0; i < RI; ++i) { yd[i] += (double)y[i]; y[i] = 0.f; }
             nstep = 0;
         }
     }
 #pragma unroll
-    for (int i = 0; i < OPS_IR_RI; ++i) {
-        const int r = lane + 32 * i;
-        ypart[warp][r] = yd[i] + (double)y[i];
-    }
+    for (int i = 0; i < RI; ++i) ypart[warp][lane + 32 * i] = yd[i] + (double)y[i];
     __syncthreads();
     double s[3] = {0.0, 0.0, 0.0};
-    for (int r = tid; r < a.R; r += OPS_IR_THREADS) {
+    for (int r = tid; r < a.R; r += THREADS) {
         double yv = 0.0;
-        for (int w = 0; w < OPS_IR_WARPS; ++w) yv += ypart[w][r];
+        for (int w = 0; w < WARPS; ++w) yv += ypart[w][r];
         const double yc = yv * (double)ct[r];
 #pragma unroll
         for (int j = 0; j < 3; ++j) s[j] += yc * (double)dlc[j][r];
     }
+    if (warp * 32 < a.R) {                           // (the warps that hold a node)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) {
+        for (int j = 0; j < 3; ++j) {
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], off);
-        if (lane == 0) red[warp][j] = s[j];
+            for (int off = 16; off > 0; off >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], off);
+            if (lane == 0) red[warp][j] = s[j];
+        }
     }
     __syncthreads();
     if (tid < 3 && a.params_bar) {
         double v = 0.0;
-        for (int w = 0; w < OPS_IR_WARPS; ++w) v += red[w][tid];
+        for (int w = 0; w < WARPS && w * 32 < a.R; ++w) v += red[w][tid];
         a.params_bar[(size_t)a.rows * m + a.row_imf1 + tid] = cs * v;
     }
 }
 
-// FP32 -> bf16 hi / lo, element-wise (count a multiple of 2).
+// FP32 -> bf16 hi / lo, element-wise: dst(part, i) from the sum of ks partial products src(part, split, i), two parts of
+// per elements (a multiple of 2).
 __global__ void split_bf16_kernel(const float *__restrict__ src, __nv_bfloat16 *__restrict__ hi,
-                                  __nv_bfloat16 *__restrict__ lo, size_t count) {
-    for (size_t i = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x); i < count; i += 2 * (size_t)gridDim.x * blockDim.x) {
-        const float2 v = *reinterpret_cast<const float2 *>(src + i);
+                                  __nv_bfloat16 *__restrict__ lo, size_t per, int ks) {
+    for (size_t i = 2 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x); i < 2 * per; i += 2 * (size_t)gridDim.x * blockDim.x) {
+        const size_t part = i >= per ? 1 : 0;
+        const float *q = src + part * (size_t)ks * per + (i - part * per);
+        float2 v = make_float2(0.f, 0.f);
+        for (int s = 0; s < ks; ++s) {
+            const float2 t = *reinterpret_cast<const float2 *>(q + (size_t)s * per);
+            v.x += t.x;
+            v.y += t.y;
+        }
         const __nv_bfloat162 h = __floats2bfloat162_rn(v.x, v.y);
         const float2 hf = __bfloat1622float2(h);
         *reinterpret_cast<__nv_bfloat162 *>(hi + i) = h;
         *reinterpret_cast<__nv_bfloat162 *>(lo + i) = __floats2bfloat162_rn(v.x - hf.x, v.y - hf.y);
     }
+}
+
+// Chabrier 2003's mass between m1 and m2 (imf_integral case 1, mass-weighted: src/physics/opensps_imf.f90:234-242):
+// the lognormal per unit ln m, exp(-(log10 m - log10 0.08)^2 / (2 sigma^2)) with sigma = 0.69, below 1 M_sun (times m:
+// a lognormal of centre log10 0.08 + ln 10 sigma^2, scale exp(ln 10 log10 0.08 + (ln 10 sigma)^2 / 2), in closed form
+// with erf), and the power law exp(-(log10 0.08)^2 / (2 sigma^2)) m^-2.3 above. FP64, host.
+static double chabrier_mass(double m1, double m2) {
+    const double K = std::log(10.0), lmc = std::log10(0.08), s2 = 0.69 * 0.69, sig = 0.69;
+    double v = 0.0;
+    const double a = m1, b = std::min(m2, 1.0);
+    if (b > a) {
+        const double centre = lmc + K * s2, scale = std::exp(K * lmc + 0.5 * K * K * s2);
+        const double z1 = (std::log10(a) - centre) / (sig * std::sqrt(2.0)), z2 = (std::log10(b) - centre) / (sig * std::sqrt(2.0));
+        v += scale * K * sig * std::sqrt(0.5 * M_PI) * (std::erf(z2) - std::erf(z1));
+    }
+    const double lo = std::max(m1, 1.0);
+    if (m2 > lo) v += std::exp(-lmc * lmc / (2.0 * s2)) * (std::pow(m2, -0.3) - std::pow(lo, -0.3)) / -0.3;
+    return v;
 }
 
 static std::string cmsg(const char *what, cudaError_t e);
@@ -1197,11 +1273,18 @@ int run_ops_interp_reverse(Context &c, const OpsRevArgs &r, std::string &err) {
     const size_t nv = (size_t)2 * n * o.ntpad;
     const int chunk = std::min(n, 2048);
     if ((e = c.d_vbh.reserve(nv)) != cudaSuccess || (e = c.d_vbl.reserve(nv)) != cudaSuccess ||
-        (e = c.d_xbar.reserve((size_t)chunk * ktot)) != cudaSuccess) {
+        (e = c.d_xbar.reserve((size_t)chunk * ktot)) != cudaSuccess || (e = c.d_ix_dln.reserve((size_t)3 * n)) != cudaSuccess) {
         err = cmsg("device memory", e);
         return ST_DATA_MISSING;
     }
-    split_bf16_kernel<<<(unsigned)std::min<size_t>((nv / 2 + 255) / 256, 8192), 256, 0, st>>>(r.vbar, c.d_vbh.p, c.d_vbl.p, nv);
+    // (the constants again, with d ln T / d alpha)
+    if ((e = run_ops_interp_const(n, r.alpha, r.imf_type == 1 ? 1.0 / chabrier_mass(0.08, 120.0) : 0.0, c.d_ix_const.p,
+                                  c.d_ix_dln.p, st)) != cudaSuccess) {
+        err = cmsg("interpolated fold constants kernel", e);
+        return ST_DATA_MISSING;
+    }
+    split_bf16_kernel<<<(unsigned)std::min<size_t>((nv / 2 + 255) / 256, 8192), 256, 0, st>>>(r.vbar, c.d_vbh.p, c.d_vbl.p, nv / 2,
+                                                                                              r.vsplit);
     if ((e = cudaGetLastError()) != cudaSuccess) { err = cmsg("template cotangent operand kernel", e); return ST_DATA_MISSING; }
     for (int m0 = 0; m0 < n; m0 += chunk) {
         const int rows = std::min(chunk, n - m0);
@@ -1226,11 +1309,11 @@ int run_ops_interp_reverse(Context &c, const OpsRevArgs &r, std::string &err) {
         OpsInterpRevArgs a;
         a.m0 = m0; a.nt = nt; a.nz = nz; a.R = R; a.ktot = ktot; a.imf_type = r.imf_type;
         for (int s = 0; s < 3; ++s) { a.noff[s] = o.interp_noff[s]; a.nn[s] = o.interp_nn[s]; a.x0[s] = o.interp_x0[s]; a.h[s] = o.interp_h[s]; }
-        a.lim_lo = (float)r.lim.lim_lo; a.lim_hi = (float)r.lim.lim_hi;
         a.wz = r.wz; a.alpha = r.alpha; a.cscale = r.cscale; a.mass_bar = r.mass_bar; a.lbol_bar = r.lbol_bar; a.lsum_bar = r.lsum_bar; a.sums = r.sums;
-        a.kconst = c.d_ix_const.p; a.xbar = c.d_xbar.p; a.mrow = o.i_mrow.p; a.lrow = o.i_lrow.p;
+        a.kconst = c.d_ix_const.p; a.dln = c.d_ix_dln.p; a.xbar = c.d_xbar.p; a.mrow = o.i_mrow.p; a.lrow = o.i_lrow.p;
         a.wzb = r.wzb; a.params_bar = r.params_bar; a.rows = r.rows; a.row_imf1 = r.row_imf1;
-        ops_interp_rev_kernel<<<rows, OPS_IR_THREADS, 0, st>>>(a);
+        if (R <= 96) ops_interp_rev_kernel<3, 32><<<rows, 1024, 0, st>>>(a);
+        else ops_interp_rev_kernel<OPS_IMAXR / 32, 8><<<rows, 256, 0, st>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) { err = cmsg("interpolated reverse fold kernel", e); return ST_DATA_MISSING; }
     }
     return 0;
@@ -2061,41 +2144,8 @@ static bool ops_interp_ok(const Context &c, const double *h_alpha, int n) {
     return true;
 }
 
-// K splits for a GEMM of tiles_mn output tiles over nkb K blocks: the fewest giving at least two waves over the SMs
-// with the last wave at least 85% full (else the fullest last wave), each split keeping 8 or more K blocks.
-static int choose_ksplit(int tiles_mn, int nkb, int num_sms) {
-    int best = 1;
-    double best_eff = -1.0;
-    const int cap = std::max(1, std::min(64, nkb / 8));
-    for (int ks = 1; ks <= cap; ++ks) {
-        const long long tiles = (long long)tiles_mn * ks, waves = (tiles + num_sms - 1) / num_sms;
-        const double eff = (double)tiles / (double)(waves * num_sms);
-        if (tiles >= 2LL * num_sms && eff >= 0.85) return ks;
-        if (eff > best_eff + 1e-9) { best_eff = eff; best = ks; }
-    }
-    return best;
-}
-
 // The interpolated fold of n models into the template GEMM's operand (d_vhi / d_vlo) and the sums: per chunk of
 // models the operand X, the young and old split-K GEMMs against the operator basis, their reduction.
-// Chabrier 2003's mass between m1 and m2 (imf_integral case 1, mass-weighted: src/physics/opensps_imf.f90:234-242):
-// the lognormal per unit ln m, exp(-(log10 m - log10 0.08)^2 / (2 sigma^2)) with sigma = 0.69, below 1 M_sun (times m:
-// a lognormal of centre log10 0.08 + ln 10 sigma^2, scale exp(ln 10 log10 0.08 + (ln 10 sigma)^2 / 2), in closed form
-// with erf), and the power law exp(-(log10 0.08)^2 / (2 sigma^2)) m^-2.3 above. FP64, host.
-static double chabrier_mass(double m1, double m2) {
-    const double K = std::log(10.0), lmc = std::log10(0.08), s2 = 0.69 * 0.69, sig = 0.69;
-    double v = 0.0;
-    const double a = m1, b = std::min(m2, 1.0);
-    if (b > a) {
-        const double centre = lmc + K * s2, scale = std::exp(K * lmc + 0.5 * K * K * s2);
-        const double z1 = (std::log10(a) - centre) / (sig * std::sqrt(2.0)), z2 = (std::log10(b) - centre) / (sig * std::sqrt(2.0));
-        v += scale * K * sig * std::sqrt(0.5 * M_PI) * (std::erf(z2) - std::erf(z1));
-    }
-    const double lo = std::max(m1, 1.0);
-    if (m2 > lo) v += std::exp(-lmc * lmc / (2.0 * s2)) * (std::pow(m2, -0.3) - std::pow(lo, -0.3)) / -0.3;
-    return v;
-}
-
 static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d_alpha, int itesc, std::string &err) {
     SspOps &o = c.ops;
     cudaStream_t st = c.stream;
@@ -2106,8 +2156,8 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
     const int chunk = std::min(n, 4096);
     const int ky = itesc * nz * R, ko = (nt - itesc) * nz * R;
     const int tiles_mn = ((chunk + gemm_bm() - 1) / gemm_bm()) * ((o.ntempl + gemm_bn() - 1) / gemm_bn());
-    const int ks_y = ky > 0 ? choose_ksplit(tiles_mn, (ky + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
-    const int ks_o = ko > 0 ? choose_ksplit(tiles_mn, (ko + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
+    const int ks_y = ky > 0 ? gemm_choose_ksplit(tiles_mn, (ky + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
+    const int ks_o = ko > 0 ? gemm_choose_ksplit(tiles_mn, (ko + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
     if ((e = c.d_ix_hi.reserve((size_t)chunk * ktot)) != cudaSuccess || (e = c.d_ix_lo.reserve((size_t)chunk * ktot)) != cudaSuccess ||
         (e = c.d_ix_const.reserve((size_t)n)) != cudaSuccess ||
         (e = c.d_ipart.reserve((size_t)std::max(ks_y + ks_o, 1) * chunk * o.ntpad)) != cudaSuccess) {
@@ -2115,8 +2165,7 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
         return ST_DATA_MISSING;
     }
     const double fixed_it = c.imf_type == 1 ? 1.0 / chabrier_mass(0.08, 120.0) : 0.0;
-    ops_interp_const_kernel<<<(n + 127) / 128, 128, 0, st>>>(d_alpha, n, 0.08f, 120.f, fixed_it, c.d_ix_const.p);
-    if ((e = cudaGetLastError()) != cudaSuccess) { err = cmsg("interpolated fold constants kernel", e); return ST_DATA_MISSING; }
+    if ((e = run_ops_interp_const(n, d_alpha, fixed_it, c.d_ix_const.p, nullptr, st)) != cudaSuccess) { err = cmsg("interpolated fold constants kernel", e); return ST_DATA_MISSING; }
     c.ops_launches += 1;
     for (int m0 = 0; m0 < n; m0 += chunk) {
         const int rows = std::min(chunk, n - m0);
