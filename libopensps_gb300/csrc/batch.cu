@@ -1086,22 +1086,23 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             }
             if (marks) prof_mark(c, 2);
             const int n_ptiles = (ns + contract_out_rows() - 1) / contract_out_rows();
-            const int bn = contract_tile_models(nacc, nk, n_ptiles, c.num_sms);
+            const ContractTile ct = contract_tile(nacc, nk, n_ptiles, c.num_sms);
             ContractPlan pl;
             pl.tm_a_hi = bop->tm_hi;
             pl.tm_a_lo = bop->tm_lo;
             pl.num_sms = c.num_sms;
-            if ((e = encode_tmap_2d_bf16(&pl.tm_b_hi, w.w_hi, kpad, nk, contract_bk(), bn)) != cudaSuccess ||
-                (e = encode_tmap_2d_bf16(&pl.tm_b_lo, w.w_lo, kpad, nk, contract_bk(), bn)) != cudaSuccess) {
+            if ((e = encode_tmap_2d_bf16(&pl.tm_b_hi, w.w_hi, kpad, nk, contract_bk(), ct.bn / ct.ctas)) != cudaSuccess ||
+                (e = encode_tmap_2d_bf16(&pl.tm_b_lo, w.w_lo, kpad, nk, contract_bk(), ct.bn / ct.ctas)) != cudaSuccess) {
                 err = cuda_msg("weights tensor map", e);
                 return ST_DATA_MISSING;
             }
             ContractArgs ca;
             ca.nspec = ns; ca.n_models = nk;
             ca.n_ptiles = n_ptiles;
-            ca.bn = bn;
+            ca.bn = ct.bn;
+            ca.ctas = ct.ctas;
             ca.ktail = bop->ktail;
-            ca.n_mtiles = (nk + bn - 1) / bn;
+            ca.n_mtiles = (nk + ct.bn - 1) / ct.bn;
             ca.nkb_young = (nacc == 1) ? bop->kmain / contract_bk() : bop->ky_pad / contract_bk();
             ca.nkb_old = (nacc == 1) ? 0 : (bop->kmain - bop->ky_pad) / contract_bk();
             ca.nkb_ion_young = bop->kion_y / contract_bk();

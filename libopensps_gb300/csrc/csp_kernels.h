@@ -99,9 +99,9 @@ struct ContractArgs {
     // young accumulator, then ion old blocks into the old one), run only by the pixel tiles that reach a pixel below
     // ion_pix (the ionizing pixels; the basis holds those columns' unabsorbed spectra there and zeros above)
     int nkb_ion_young = 0, nkb_ion_old = 0, ion_pix = 0;
-    // models per tile (a multiple of 32, contract_tile_models), and the 16-column K steps of the last block of the
+    // models per tile and CTAs per tile (contract_tile), and the 16-column K steps of the last block of the
     // young, old, ion young and ion old ranges, a byte each
-    int bn = 0;
+    int bn = 0, ctas = 1;
     unsigned ktail = 0;
     int sm_lo, sm_hi;    // pixels smoothed (lambda within [min_wave_smooth, max_wave_smooth]); sm_lo > sm_hi: none
     int uniform_index;   // every model has the pixel table's curve
@@ -118,8 +118,10 @@ struct ContractPlan {
     int num_sms;
 };
 
-// Models per tile for a batch of n_models over n_ptiles pixel tiles.
-int contract_tile_models(int nacc, int n_models, int n_ptiles, int num_sms);
+// The tile of a batch of n_models over n_ptiles pixel tiles: models (a multiple of 32) and CTAs (2: a CTA pair takes two
+// pixel tiles in one MMA, each CTA loading half of the models' weights).
+struct ContractTile { int bn, ctas; };
+ContractTile contract_tile(int nacc, int n_models, int n_ptiles, int num_sms);
 int contract_out_rows();
 int contract_halo();
 int contract_bk();

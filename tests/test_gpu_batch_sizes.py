@@ -21,7 +21,7 @@ def setup(data, built_lib):
     ctx.close()
 
 
-@pytest.mark.parametrize("n", [1, 2, 31, 33, 65, 153, 305, 609, 1217, 8192, 8193])
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 65, 153, 305, 609, 1217, 3011, 8192, 8193])
 @pytest.mark.parametrize("birth_cloud", [False, True])
 def test_batch_sizes(setup, n, birth_cloud):
     ctx, oracle = setup
