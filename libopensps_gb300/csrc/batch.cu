@@ -434,6 +434,30 @@ void prof_mark(Context &c, int k) {
     c.prof_pending[s] = k > 0;
 }
 
+// Batches whose per-model host loops are spread over the host threads: a fork and join takes some tens of us, what 8192
+// models of the light loops take (with 1024 a batch of that size lost 120 us in four loops), and 2048 of the emission
+// cells' (40 ns a model).
+constexpr int OMP_MODELS = 8192, OMP_CELL_MODELS = 2048;
+// Batches whose weight operand runs on a stream of its own beside the model parameters.
+constexpr int FORK_MODELS = 4096;
+
+// A page-locked buffer kept by the context, at least count doubles.
+static cudaError_t reserve_pinned(double *&p, size_t &n, size_t count) {
+    if (n >= count) return cudaSuccess;
+    if (p) cudaFreeHost(p);
+    p = nullptr;
+    n = 0;
+    const cudaError_t e = cudaMallocHost(&p, sizeof(double) * count);
+    if (e == cudaSuccess) n = count;
+    return e;
+}
+static bool page_locked(const void *p) {
+    cudaPointerAttributes a;
+    const bool yes = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+    cudaGetLastError();
+    return yes;
+}
+
 static std::string cuda_msg(const char *what, cudaError_t e) { return std::string(what) + ": " + cudaGetErrorString(e); }
 
 int run_batch(Context &c, const BatchIO &io, std::string &err) {
@@ -579,15 +603,73 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             }
         }
     }
-    // smoothing rows must keep their whole window inside the grid
+    // the smoothed pixels, lambda within [min_wave_smooth, max_wave_smooth] (kept until the range changes); smoothing
+    // rows must keep their whole window inside the grid
+    if (c.sm_range[0] != minl || c.sm_range[1] != maxl) {
+        c.sm_first = ns;
+        c.sm_last = -1;
+        for (int j = 0; j < ns; ++j)
+            if (c.lam[j] >= minl && c.lam[j] <= maxl) { c.sm_first = std::min(c.sm_first, j); c.sm_last = j; }
+        c.sm_range[0] = minl;
+        c.sm_range[1] = maxl;
+    }
+    const int sm_lo = c.sm_first, sm_hi = c.sm_last;
     int i0 = -1;
     if (any_smooth) {
-        for (int j = 0; j < ns; ++j)
-            if (c.lam[j] >= minl && c.lam[j] <= maxl) { i0 = j; break; }
+        if (sm_hi >= 0) i0 = sm_lo;
         if (i0 >= 0 && (minl <= c.lam[contract_halo()] || maxl >= c.lam[ns - 1 - contract_halo()])) {
             err = "the smoothing range must lie inside the wavelength grid's interior";
             return ST_UNSUPPORTED;
         }
+    }
+    cudaError_t e;
+    cudaStream_t st = c.stream;
+    // the weights over ages (the SFH's, or the caller's) and their blend at logzsol, formed on the device: queued here,
+    // so that they run beside the checks that follow
+    struct SfhInFlight {   // (a batch refused after this point waits: the next one reuses the staging buffer)
+        cudaStream_t st = nullptr;
+        ~SfhInFlight() { if (st) cudaStreamSynchronize(st); }
+    } sfh_in_flight;
+    if (io.sfh_par) {
+        const size_t np = (size_t)SFH_NCOL * n;
+        if ((e = reserve_pinned(c.pinned_sfh, c.pinned_sfh_n, np)) != cudaSuccess) {
+            err = cuda_msg("page-locked SFH parameters", e);
+            return ST_DATA_MISSING;
+        }
+        sfh_in_flight.st = st;
+        std::memcpy(c.pinned_sfh, io.sfh_par, sizeof(double) * np);
+        if ((e = c.d_wz.reserve((size_t)n * nt * nz)) != cudaSuccess || (e = c.d_sfhpar.reserve(np)) != cudaSuccess || (e = c.d_w.reserve((size_t)nt * n)) != cudaSuccess ||
+            (e = c.d_sfh_scratch.reserve((size_t)2 * nt * n)) != cudaSuccess ||
+            (e = c.d_sfh_mtab.reserve((size_t)(nt + 1) * n)) != cudaSuccess ||
+            (e = c.d_lblend.reserve((size_t)3 * n)) != cudaSuccess || (e = c.d_sfr.reserve(n)) != cudaSuccess ||
+            (io.given_w && (e = c.d_wgiven.reserve((size_t)nt * n)) != cudaSuccess) ||
+            (e = cudaMemcpyAsync(c.d_sfhpar.p, c.pinned_sfh, sizeof(double) * np, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (io.given_w && (e = cudaMemcpyAsync(c.d_wgiven.p, io.given_w, sizeof(double) * nt * n, cudaMemcpyHostToDevice, st)) != cudaSuccess)) {
+            err = cuda_msg("SFH inputs", e);
+            return ST_DATA_MISSING;
+        }
+        SfhArgs sa;
+        sa.n = n; sa.nt = nt; sa.nz = nz; sa.sfh = io.sfh_type; sa.itesc = itesc;
+        sa.tf = c.d_logage.p; sa.t10 = c.d_logage.p + nt; sa.lz = c.d_lz.p; sa.lbol = c.d_lbol.p; sa.par = c.d_sfhpar.p;
+        sa.given = io.given_w ? c.d_wgiven.p : nullptr;
+        sa.w = c.d_w.p; sa.scratch = c.d_sfh_scratch.p; sa.wz = c.d_wz.p; sa.lblend = c.d_lblend.p; sa.sfr = c.d_sfr.p;
+        sa.mtab = c.d_sfh_mtab.p;
+        if ((io.sfh_type == 2 || io.sfh_type == 3) && !io.given_w) {
+            // the tabular SFH: ages then SFRs, each with its zero entry past the table
+            const size_t nt1 = (size_t)c.ntab + 1;
+            if (c.sfh_tab_dirty || c.d_sfhtab.n < 2 * nt1) {
+                if ((e = c.d_sfhtab.reserve(2 * nt1)) != cudaSuccess ||
+                    (e = cudaMemcpyAsync(c.d_sfhtab.p, c.sfh_tab_t.data(), sizeof(double) * nt1, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+                    (e = cudaMemcpyAsync(c.d_sfhtab.p + nt1, c.sfh_tab_sfr.data(), sizeof(double) * nt1, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
+                    err = cuda_msg("tabular SFH copy", e);
+                    return ST_DATA_MISSING;
+                }
+                c.sfh_tab_dirty = false;
+            }
+            sa.ntab = c.ntab;
+            sa.tab = c.d_sfhtab.p;
+        }
+        if ((e = run_sfh_forward(sa, st)) != cudaSuccess) { err = cuda_msg("SFH weights kernel", e); return ST_DATA_MISSING; }
     }
     // nebular lines: one profile table per batch, from the first model's sigma (prepare_line_gaussians(ctx,
     // psets(1)), src/physics/opensps_csp_batch.f90:1733); a model whose own sigma would give other widths is
@@ -596,16 +678,19 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     double line_sigma = 0.0;
     if (neb) {
         const double s1 = par(0, PF_SIGMA_SMOOTH);
-        const bool f1 = lines_floor_limited(c, s1);
-        line_sigma = f1 ? 0.0 : s1;
         // below 0.999 of the smallest line's threshold every line is at the floor (no per-line test needed)
-        double thr = 1e300;
-        for (int l = 0; l < c.nline; ++l) {
-            const double pos = c.line_lambda[l];
-            int j = find_interval0(c.lam.data(), c.nspec, pos) + 1;
-            j = std::max(1, std::min(j, c.nspec - 1));
-            thr = std::min(thr, 2.0 * (c.lam[j] - c.lam[j - 1]) / (pos * (1.0e13 / C_LIGHT)));
+        if (c.line_thr < 0.0) {
+            c.line_thr = 1e300;
+            for (int l = 0; l < c.nline; ++l) {
+                const double pos = c.line_lambda[l];
+                int j = find_interval0(c.lam.data(), c.nspec, pos) + 1;
+                j = std::max(1, std::min(j, c.nspec - 1));
+                c.line_thr = std::min(c.line_thr, 2.0 * (c.lam[j] - c.lam[j - 1]) / (pos * (1.0e13 / C_LIGHT)));
+            }
         }
+        const double thr = c.line_thr;
+        const bool f1 = s1 < 0.999 * thr || lines_floor_limited(c, s1);
+        line_sigma = f1 ? 0.0 : s1;
         for (int m = 1; m < n; ++m) {
             const double sm = par(m, PF_SIGMA_SMOOTH);
             if (sm == s1) continue;
@@ -659,6 +744,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         }
         dem = c.pinned_dem;
         if (io.keep_parts) c.h_dchain.assign((size_t)n, make_float4(0.f, 0.f, 0.f, 0.f));
+#pragma omp parallel for schedule(static) if (n >= OMP_CELL_MODELS)
         for (int m = 0; m < n; ++m) {
             DustEmModel &q = dem[m];
             q = DustEmModel{};
@@ -818,11 +904,6 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         for (int k = 0; k < 6; ++k) c.pix_key[k] = key[k];
     }
     const int tab_curve = c.dust_type != 0 ? 1 : 0;   // (models' own curves from the tables, else the power law)
-    // the smoothed pixels: lambda within [min_wave_smooth, max_wave_smooth]
-    int sm_lo = ns, sm_hi = -1;
-    for (int j = 0; j < ns; ++j)
-        if (c.lam[j] >= minl && c.lam[j] <= maxl) { sm_lo = std::min(sm_lo, j); sm_hi = std::max(sm_hi, j); }
-
     c.geom.bop = bop;
     c.geom.nacc = nacc;
     c.geom.sm_lo = any_smooth ? sm_lo : ns;
@@ -839,8 +920,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
 
     // ---- scratch
     const int kpad = ops ? 64 : bop->kpad;
-    cudaError_t e;
     const size_t nwz = (size_t)n * nt * nz;
+    sfh_in_flight.st = nullptr;   // (every check has passed)
     if ((!io.dev_inputs && (e = c.d_wz.reserve(nwz)) != cudaSuccess) ||
         (e = c.d_params.reserve((size_t)PAR_DEVICE * n)) != cudaSuccess ||
         (e = c.d_whi.reserve((size_t)n * kpad)) != cudaSuccess || (e = c.d_wlo.reserve((size_t)n * kpad)) != cudaSuccess ||
@@ -850,46 +931,12 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         err = cuda_msg("device memory", e);
         return ST_DATA_MISSING;
     }
-    cudaStream_t st = c.stream;
     const double *d_wz = io.wz;
     const double *d_par = nullptr;
     std::vector<double> hp;
     if (io.dev_inputs) {
         d_par = io.dev_params;   // already PAR_DEVICE x n on the device
     } else if (io.sfh_par) {
-        // the weights over ages (the SFH's, or the caller's) and their blend at logzsol, formed on the device
-        if ((e = c.d_sfhpar.reserve((size_t)SFH_NCOL * n)) != cudaSuccess || (e = c.d_w.reserve((size_t)nt * n)) != cudaSuccess ||
-            (e = c.d_sfh_scratch.reserve((size_t)2 * nt * n)) != cudaSuccess ||
-            (e = c.d_sfh_mtab.reserve((size_t)(nt + 1) * n)) != cudaSuccess ||
-            (e = c.d_lblend.reserve((size_t)3 * n)) != cudaSuccess || (e = c.d_sfr.reserve(n)) != cudaSuccess ||
-            (io.given_w && (e = c.d_wgiven.reserve((size_t)nt * n)) != cudaSuccess) ||
-            (e = cudaMemcpyAsync(c.d_sfhpar.p, io.sfh_par, sizeof(double) * SFH_NCOL * n, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-            (io.given_w && (e = cudaMemcpyAsync(c.d_wgiven.p, io.given_w, sizeof(double) * nt * n, cudaMemcpyHostToDevice, st)) != cudaSuccess)) {
-            err = cuda_msg("SFH inputs", e);
-            return ST_DATA_MISSING;
-        }
-        SfhArgs sa;
-        sa.n = n; sa.nt = nt; sa.nz = nz; sa.sfh = io.sfh_type; sa.itesc = itesc;
-        sa.tf = c.d_logage.p; sa.t10 = c.d_logage.p + nt; sa.lz = c.d_lz.p; sa.lbol = c.d_lbol.p; sa.par = c.d_sfhpar.p;
-        sa.given = io.given_w ? c.d_wgiven.p : nullptr;
-        sa.w = c.d_w.p; sa.scratch = c.d_sfh_scratch.p; sa.wz = c.d_wz.p; sa.lblend = c.d_lblend.p; sa.sfr = c.d_sfr.p;
-        sa.mtab = c.d_sfh_mtab.p;
-        if ((io.sfh_type == 2 || io.sfh_type == 3) && !io.given_w) {
-            // the tabular SFH: ages then SFRs, each with its zero entry past the table
-            const size_t nt1 = (size_t)c.ntab + 1;
-            if (c.sfh_tab_dirty || c.d_sfhtab.n < 2 * nt1) {
-                if ((e = c.d_sfhtab.reserve(2 * nt1)) != cudaSuccess ||
-                    (e = cudaMemcpyAsync(c.d_sfhtab.p, c.sfh_tab_t.data(), sizeof(double) * nt1, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
-                    (e = cudaMemcpyAsync(c.d_sfhtab.p + nt1, c.sfh_tab_sfr.data(), sizeof(double) * nt1, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
-                    err = cuda_msg("tabular SFH copy", e);
-                    return ST_DATA_MISSING;
-                }
-                c.sfh_tab_dirty = false;
-            }
-            sa.ntab = c.ntab;
-            sa.tab = c.d_sfhtab.p;
-        }
-        if ((e = run_sfh_forward(sa, st)) != cudaSuccess) { err = cuda_msg("SFH weights kernel", e); return ST_DATA_MISSING; }
         d_wz = c.d_wz.p;
     } else {
         if (!chunked && (e = cudaMemcpyAsync(c.d_wz.p, io.wz, sizeof(double) * nwz, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
@@ -912,7 +959,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             c.pinned_par_n = np;
         }
         double *hpp = c.pinned_par;
-#pragma omp parallel for schedule(static) if (n >= 8192)
+#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
         for (int m = 0; m < n; ++m)
             for (int k = 0; k < PAR_DEVICE; ++k) hpp[(size_t)PAR_DEVICE * m + k] = par(m, k);
         // (with the weights in chunks the table goes up on the side stream between the first chunk and the others:
@@ -1053,8 +1100,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             if (w.mpar) w.mpar = c.d_mpar.p + (size_t)MODEL_PAR_FLOATS * off;
             // the operand (which does not read the model parameters unless it forms escaping-light columns) on its
             // own stream beside the model parameters, forked from the batch's stream and joined before the
-            // contraction
-            const bool fork_w = !direct && !w.mpar;
+            // contraction; small batches' kernels (26 us together at 1000 models) are not worth the fork's four calls
+            const bool fork_w = !direct && !w.mpar && nk > FORK_MODELS;
             if (fork_w && ((e = cudaEventRecord(c.ev_w0, st)) != cudaSuccess || (e = cudaStreamWaitEvent(c.side4, c.ev_w0, 0)) != cudaSuccess ||
                            (e = run_weights_convert_sums(w, c.side4)) != cudaSuccess || (e = cudaEventRecord(c.ev_w1, c.side4)) != cudaSuccess)) {
                 err = cuda_msg("weights kernel", e);
@@ -1154,15 +1201,9 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             d_y = c.d_young.p;
             d_o = c.d_old.p;
         }
-        if (chunked && want_mags && c.pinned_mags_n < (size_t)n * nb) {
-            if (c.pinned_mags) cudaFreeHost(c.pinned_mags);
-            c.pinned_mags = nullptr;
-            c.pinned_mags_n = 0;
-            if ((e = cudaMallocHost(&c.pinned_mags, sizeof(double) * n * nb)) != cudaSuccess) {
-                err = cuda_msg("page-locked magnitudes", e);
-                return ST_DATA_MISSING;
-            }
-            c.pinned_mags_n = (size_t)n * nb;
+        if (chunked && want_mags && (e = reserve_pinned(c.pinned_mags, c.pinned_mags_n, (size_t)n * nb)) != cudaSuccess) {
+            err = cuda_msg("page-locked magnitudes", e);
+            return ST_DATA_MISSING;
         }
         if (!chunked) {
             if (int rc = run_range(0, n, true)) return rc;
@@ -1305,8 +1346,15 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             return ST_DATA_MISSING;
         }
     }
+    // (to a page-locked caller's array directly, else through the page-locked staging buffer: a copy to pageable memory
+    // holds the host until it is done, with every copy after it)
+    const bool stage_mags = want_mags && !io.dev_inputs && !chunked && !page_locked(io.mags);
+    if (stage_mags && (e = reserve_pinned(c.pinned_mags, c.pinned_mags_n, (size_t)n * nb)) != cudaSuccess) {
+        err = cuda_msg("page-locked magnitudes", e);
+        return ST_DATA_MISSING;
+    }
     if (want_mags && !io.dev_inputs && !chunked) {
-        if ((e = cudaMemcpyAsync(io.mags, c.d_mags.p, sizeof(double) * n * nb, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
+        if ((e = cudaMemcpyAsync(stage_mags ? c.pinned_mags : io.mags, c.d_mags.p, sizeof(double) * n * nb, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
             err = cuda_msg("magnitudes copy", e);
             return ST_DATA_MISSING;
         }
@@ -1316,15 +1364,9 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     if (want_sums && !io.dev_inputs) {
         // through a page-locked buffer kept by the context
         const size_t ns6 = (size_t)6 * n;
-        if (c.pinned_sums_n < ns6) {
-            if (c.pinned_sums) cudaFreeHost(c.pinned_sums);
-            c.pinned_sums = nullptr;
-            c.pinned_sums_n = 0;
-            if ((e = cudaMallocHost(&c.pinned_sums, sizeof(double) * ns6)) != cudaSuccess) {
-                err = cuda_msg("page-locked sums", e);
-                return ST_DATA_MISSING;
-            }
-            c.pinned_sums_n = ns6;
+        if ((e = reserve_pinned(c.pinned_sums, c.pinned_sums_n, ns6)) != cudaSuccess) {
+            err = cuda_msg("page-locked sums", e);
+            return ST_DATA_MISSING;
         }
         sums = c.pinned_sums;
         if ((e = cudaMemcpyAsync(c.pinned_sums, c.d_sums.p, sizeof(double) * ns6, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
@@ -1335,12 +1377,17 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     // weights formed on the device: L_bol blended in log between the slabs (model_sums MSUMS_BLEND,
     // src/physics/opensps_csp_batch.f90:2129-2176), not the sum over the two slabs' linear L_bol (with the operators
     // L_bol is their linear L_bol row); the SFH's SFR
-    std::vector<double> lblend, sfr_h;
+    // (page-locked: the SFR, then L_bol total, young and old)
+    const double *lblend = nullptr, *sfr_h = nullptr;
     if (io.sfh_par && !io.dev_inputs) {
-        sfr_h.resize(n);
-        if (!ops) lblend.resize((size_t)3 * n);
-        if ((!ops && (e = cudaMemcpyAsync(lblend.data(), c.d_lblend.p, sizeof(double) * lblend.size(), cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
-            (e = cudaMemcpyAsync(sfr_h.data(), c.d_sfr.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
+        if ((e = reserve_pinned(c.pinned_sfhout, c.pinned_sfhout_n, (size_t)4 * n)) != cudaSuccess) {
+            err = cuda_msg("page-locked SFH outputs", e);
+            return ST_DATA_MISSING;
+        }
+        sfr_h = c.pinned_sfhout;
+        if (!ops) lblend = c.pinned_sfhout + n;
+        if ((!ops && (e = cudaMemcpyAsync(c.pinned_sfhout + n, c.d_lblend.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
+            (e = cudaMemcpyAsync(c.pinned_sfhout, c.d_sfr.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
             err = cuda_msg("SFH outputs copy", e);
             return ST_DATA_MISSING;
         }
@@ -1366,8 +1413,9 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
 #pragma omp parallel for schedule(static)
         for (int m = 0; m < n; ++m) std::memcpy(io.mags + (size_t)nb * m, src + (size_t)nb * m, sizeof(double) * nb);
     }
+    if (stage_mags) std::memcpy(io.mags, c.pinned_mags, sizeof(double) * n * nb);
     if (want_sums && !io.dev_inputs) {
-#pragma omp parallel for schedule(static) if (n >= 8192)
+#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
         for (int m = 0; m < n; ++m) {
             const double *s = sums + (size_t)6 * m;
             if (io.mass) io.mass[m] = s[0];
@@ -1386,15 +1434,16 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             if (io.old) io.old[i] = (double)old_h[i];
         }
     }
-    if (!lblend.empty()) {
+    if (lblend) {
+#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
         for (int m = 0; m < n; ++m) {
-            const double *l = lblend.data() + (size_t)3 * m;
+            const double *l = lblend + (size_t)3 * m;
             if (io.lbol) io.lbol[m] = l[0] > SAFE_FLOOR ? std::log10(l[0]) : 0.0;
             if (io.lbol_young) io.lbol_young[m] = std::log10(std::max(l[1], SAFE_FLOOR));
             if (io.lbol_old) io.lbol_old[m] = std::log10(std::max(l[2], SAFE_FLOOR));
         }
     }
-    if (io.sfr) for (int m = 0; m < n; ++m) io.sfr[m] = sfr_h.empty() ? std::nan("") : sfr_h[m];
+    if (io.sfr) for (int m = 0; m < n; ++m) io.sfr[m] = sfr_h ? sfr_h[m] : std::nan("");
     if (io.mdust) for (int m = 0; m < n; ++m) io.mdust[m] = SAFE_FLOOR;
     return 0;
 }

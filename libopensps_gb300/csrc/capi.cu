@@ -191,6 +191,7 @@ int batch_core(Context &cref, int n, int n_params, const char *const *names, con
         sfhp.resize((size_t)SFH_NCOL * n);
         const int ids[SFH_NCOL] = {PF_TAGE, PF_TAU, PF_CONST, PF_FBURST, PF_TBURST, PF_SF_START, PF_SF_TRUNC,
                                    PF_SF_SLOPE, PF_LOGZSOL};
+#pragma omp parallel for schedule(static) if (n >= 8192)
         for (int m = 0; m < n; ++m)
             for (int k = 0; k < SFH_NCOL; ++k) sfhp[(size_t)SFH_NCOL * m + k] = rows[(size_t)PF_COUNT * m + ids[k]];
     }

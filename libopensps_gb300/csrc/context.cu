@@ -194,6 +194,12 @@ Context::~Context() {
     if (pinned_sums) cudaFreeHost(pinned_sums);
     pinned_sums = nullptr;
     pinned_sums_n = 0;
+    if (pinned_sfh) cudaFreeHost(pinned_sfh);
+    pinned_sfh = nullptr;
+    pinned_sfh_n = 0;
+    if (pinned_sfhout) cudaFreeHost(pinned_sfhout);
+    pinned_sfhout = nullptr;
+    pinned_sfhout_n = 0;
     if (pinned_mags) cudaFreeHost(pinned_mags);
     pinned_mags = nullptr;
     pinned_mags_n = 0;
@@ -814,6 +820,9 @@ int context_setup_grid(Context &c, std::string &err) {
         err = std::string("loading the no-allocation entry point's modules: ") + cudaGetErrorString(e);
         return ST_DATA_MISSING;
     }
+    c.sm_range[0] = 0.0;
+    c.sm_range[1] = -1.0;
+    c.line_thr = -1.0;
     c.is_setup = true;
     return 0;
 }

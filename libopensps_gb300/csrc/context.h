@@ -235,6 +235,10 @@ struct Context {
     std::vector<double> zt, dl;  // cosmology table (500)
     std::vector<float> igm_a;    // jtop x 6 Madau wavelength factors
     int jtop = 0;
+    // of the grid: the pixels within the last batch's smoothing range, and the smallest sigma_smooth at which a nebular
+    // line is wider than the grid's floor (negative: not formed yet)
+    double sm_range[2] = {0.0, -1.0}, line_thr = -1.0;
+    int sm_first = 0, sm_last = -1;
 
     // device copies
     int device = 0, num_sms = 0;
@@ -324,9 +328,11 @@ struct Context {
     void *pinned_spec = nullptr; size_t pinned_bytes = 0;
     double *pinned_par = nullptr; size_t pinned_par_n = 0;   // page-locked staging of the per-model parameter table
     DustEmModel *pinned_dem = nullptr; size_t pinned_dem_n = 0;   // page-locked staging of the dust emission / AGN cells
+    double *pinned_sfh = nullptr; size_t pinned_sfh_n = 0;   // page-locked staging of the SFH parameters
+    double *pinned_sfhout = nullptr; size_t pinned_sfhout_n = 0;   // page-locked SFRs and blended L_bol
     double *pinned_sums = nullptr; size_t pinned_sums_n = 0; // page-locked copy of the mass and L_bol sums
     std::vector<int> do_band_h;                               // the band mask last uploaded to d_do_band
-    double *pinned_mags = nullptr; size_t pinned_mags_n = 0; // page-locked staging of the chunked batch's magnitudes
+    double *pinned_mags = nullptr; size_t pinned_mags_n = 0; // page-locked staging of the magnitudes
     std::vector<double> param_rows;                          // the batch's parameter rows (PF_COUNT x n)
     static constexpr int NCHUNK_EV = 64;
     cudaEvent_t chunk_ev[NCHUNK_EV] = {};                    // the chunked batch's weight copies
