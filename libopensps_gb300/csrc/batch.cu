@@ -434,10 +434,6 @@ void prof_mark(Context &c, int k) {
     c.prof_pending[s] = k > 0;
 }
 
-// Batches whose per-model host loops are spread over the host threads: a fork and join takes some tens of us, what 8192
-// models of the light loops take (with 1024 a batch of that size lost 120 us in four loops), and 2048 of the emission
-// cells' (40 ns a model).
-constexpr int OMP_MODELS = 8192, OMP_CELL_MODELS = 2048;
 // Batches whose weight operand runs on a stream of its own beside the model parameters.
 constexpr int FORK_MODELS = 4096;
 
@@ -744,7 +740,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         }
         dem = c.pinned_dem;
         if (io.keep_parts) c.h_dchain.assign((size_t)n, make_float4(0.f, 0.f, 0.f, 0.f));
-#pragma omp parallel for schedule(static) if (n >= OMP_CELL_MODELS)
+// (40 ns a model; a fork and join takes some tens of us, what 8192 models of the lighter loops take)
+#pragma omp parallel for schedule(static) if (n >= 2048)
         for (int m = 0; m < n; ++m) {
             DustEmModel &q = dem[m];
             q = DustEmModel{};
@@ -959,7 +956,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             c.pinned_par_n = np;
         }
         double *hpp = c.pinned_par;
-#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
+#pragma omp parallel for schedule(static) if (n >= 8192)
         for (int m = 0; m < n; ++m)
             for (int k = 0; k < PAR_DEVICE; ++k) hpp[(size_t)PAR_DEVICE * m + k] = par(m, k);
         // (with the weights in chunks the table goes up on the side stream between the first chunk and the others:
@@ -1415,7 +1412,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     }
     if (stage_mags) std::memcpy(io.mags, c.pinned_mags, sizeof(double) * n * nb);
     if (want_sums && !io.dev_inputs) {
-#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
+#pragma omp parallel for schedule(static) if (n >= 8192)
         for (int m = 0; m < n; ++m) {
             const double *s = sums + (size_t)6 * m;
             if (io.mass) io.mass[m] = s[0];
@@ -1435,7 +1432,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         }
     }
     if (lblend) {
-#pragma omp parallel for schedule(static) if (n >= OMP_MODELS)
+#pragma omp parallel for schedule(static) if (n >= 8192)
         for (int m = 0; m < n; ++m) {
             const double *l = lblend + (size_t)3 * m;
             if (io.lbol) io.lbol[m] = l[0] > SAFE_FLOOR ? std::log10(l[0]) : 0.0;

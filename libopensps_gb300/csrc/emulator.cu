@@ -23,8 +23,7 @@
 //
 // A batch of few tiles leaves most SMs without one (four CTAs took 220 us for 500 models): there a CTA takes one member
 // of a tile at a time (SPLIT), its outputs go to the tile's place in the scratch, and emu_reduce_kernel forms the
-// ensemble's results from them, in the order of members the fused kernel sums them in: 224 -> 47 us at 500 models,
-// 441 -> 227 at 20000.
+// ensemble's results from them: 224 -> 47 us at 500 models, 441 -> 227 at 20000.
 //
 // Every mbarrier wait is bounded (status word, no hang); drains wait for the copies and MMAs in flight.
 #include <cuda_runtime.h>
@@ -87,6 +86,71 @@ __device__ __forceinline__ float emu_distance(float z, const float *zt, const fl
     return 5.f * log10f(dm * 0.1f) - 2.5f * log10f(1.f + z);
 }
 
+// The members' outputs of a row by a warp: step k's outputs 4 lane .. 4 lane + 3 (PCA coefficients, then bands) at out +
+// k step.
+__device__ __forceinline__ void emu_load_row(const float *out, size_t step, float (*z)[4]) {
+#pragma unroll
+    for (int k = 0; k < EMU_MEMBERS; ++k) {
+        const float4 t = __ldcg(reinterpret_cast<const float4 *>(out + k * step));   // (past L1: it holds the biases)
+        z[k][0] = t.x; z[k][1] = t.y; z[k][2] = t.z; z[k][3] = t.w;
+    }
+}
+// Model m's results from them: the mean of each, the spread (the population standard deviation over the members, the
+// largest over the bands less than `faint` mag fainter than the brightest) and the flag. mu, sg: the outputs' means and
+// scales; dd: the distance term.
+__device__ __forceinline__ void emu_row(const EmuInferArgs &a, int m, const float (*z)[4], const float *mu, const float *sg,
+                                        float dd, bool outside, bool bad, int lane) {
+    const float invm = 1.f / (float)EMU_MEMBERS;
+    float v[4], sd[4];
+    float mmin = INFINITY;
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int band = 4 * lane + i - EMU_NPC;
+        float sum = 0.f;
+#pragma unroll
+        for (int k = 0; k < EMU_MEMBERS; ++k) sum += z[k][i];
+        v[i] = mu[i] + sg[i] * sum * invm;
+        sd[i] = 0.f;
+        if (band >= 0) {
+            v[i] += dd;
+            const float mean = sum * invm;
+            float var = 0.f;
+#pragma unroll
+            for (int k = 0; k < EMU_MEMBERS; ++k) var += (z[k][i] - mean) * (z[k][i] - mean);
+            sd[i] = sg[i] * sqrtf(var * invm);
+            if (band < a.nb) {
+                if (!isfinite(v[i]) || !isfinite(sd[i])) finite = false;
+                mmin = fminf(mmin, v[i]);
+                a.mags[(size_t)m * a.nb + band] = v[i];
+            }
+        }
+    }
+    if (a.coef && 4 * lane < EMU_NPC)
+        *reinterpret_cast<float4 *>(a.coef + (size_t)m * EMU_NPC + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) mmin = fminf(mmin, __shfl_xor_sync(0xffffffffu, mmin, off));
+    float spread = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int band = 4 * lane + i - EMU_NPC;
+        if (band >= 0 && band < a.nb && v[i] < mmin + a.faint) spread = fmaxf(spread, sd[i]);
+    }
+    // (not negative: ordered as its bits)
+    spread = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(spread)));
+    finite = __all_sync(0xffffffffu, finite);
+    if (lane == 0) {
+        const int f = outside ? 1 : (bad || !finite) ? 3 : (spread > a.spread_max) ? 2 : 0;
+        if (a.spread) a.spread[m] = spread;
+        a.flag[m] = f;
+        if (f) a.flagged[atomicAdd(a.nflag, 1)] = m;
+    }
+}
+__device__ __forceinline__ void emu_scales(const float *par, int lane, float *mu, float *sg) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { mu[i] = __ldg(par + EMU_P_OMU + 4 * lane + i); sg[i] = __ldg(par + EMU_P_OSIG + 4 * lane + i); }
+}
+
 // The work of a CTA: iteration it's tile, and the members it runs there (all of them, or with SPLIT one: unit
 // blockIdx + it gridDim is member unit % EMU_MEMBERS of tile unit / EMU_MEMBERS). The member at step mem is rotated by
 // the CTA index, so that the CTAs stream different members' weights at a time instead of all reading the same tiles
@@ -139,7 +203,8 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
     using Work = EmuWork<SPLIT>;
     const int iters = Work::iters(ntiles);
     int *status = a.status;
-    // per CTA, two slots x 128 rows x 16 words of tile inputs (the input row's 12 f16 words, zred, the flags); this
+    // per CTA, two slots x 128 rows x 16 words of tile inputs (the input row's 12 f16 words, zred, the flags, the
+    // distance term); this
     // row's outputs of each member: scratch[cta][step][row][128], with SPLIT scratch[unit][row][128]
     uint4 *in_row = reinterpret_cast<uint4 *>(a.scratch + (size_t)blockIdx.x * EMU_SCRATCH_IN) + (size_t)r * 4;
     float *scr_row = a.scratch + (size_t)gridDim.x * EMU_SCRATCH_IN +
@@ -149,8 +214,11 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
     bool ok = true;
     // the input words and flags of tile `tile` into slot `slot` (cs = 0 warps, one row each)
     auto prepare_input = [&](int tile, int slot) {
-        if (cs != 0) return;
         const int m = tile * 128 + r;
+        uint4 *dst = in_row + (size_t)slot * 128 * 4;
+        if (!SPLIT && cs == 1)   // (the distance term by the next slice's warps, beside the features)
+            reinterpret_cast<float *>(dst)[14] = m < a.n ? emu_distance(__ldg(a.x + (size_t)m * EMU_NIN + 5), par + EMU_P_ZT, par + EMU_P_DL) : 0.f;
+        if (cs != 0) return;
         float xs[EMU_NFEAT];
         float zred = 0.f;
         uint32_t flags = 0;                      // bit 0: outside the box, bit 1: not finite
@@ -176,31 +244,37 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
             w[i] = pack_f16(xs[2 * i], xs[2 * i + 1]);
             w[6 + i] = pack_f16(f16_lo(xs[2 * i]), f16_lo(xs[2 * i + 1]));
         }
-        uint4 *dst = in_row + (size_t)slot * 128 * 4;
         dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
         dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
         dst[2] = make_uint4(w[8], w[9], w[10], w[11]);
-        dst[3] = make_uint4(__float_as_uint(zred), flags, 0u, 0u);
+        *reinterpret_cast<uint2 *>(dst + 3) = make_uint2(__float_as_uint(zred), flags);
     };
-    // the input row into K block 0 of S (f16: the features' hi parts at K 0..11, lo parts at 16..27), from slot
-    // `slot`; every epilogue warp arrives
-    auto put_input = [&](int slot) {
+    // the input row into K block 0 of S (f16: the features' hi parts at K 0..11, lo parts at 16..27) from its words, read
+    // from the slot before S is free (read after it they held the next member's first MMA back by 4000 cycles); every
+    // epilogue warp arrives
+    auto load_input = [&](int slot, uint4 *iw) {
+        const uint4 *src = in_row + (size_t)slot * 128 * 4;
+#pragma unroll
+        for (int i = 0; i < 3; ++i) iw[i] = src[i];
+    };
+    auto put_input = [&](const uint4 *iw) {
         if (cs == 0) {
-            const uint4 *src = in_row + (size_t)slot * 128 * 4;
-            const uint4 w0 = src[0], w1 = src[1], w2 = src[2];
-            st_shared_v4(s_base + sw128_off(r, 0), w0.x, w0.y, w0.z, w0.w);
-            st_shared_v4(s_base + sw128_off(r, 1), w1.x, w1.y, 0u, 0u);
-            st_shared_v4(s_base + sw128_off(r, 2), w1.z, w1.w, w2.x, w2.y);
-            st_shared_v4(s_base + sw128_off(r, 3), w2.z, w2.w, 0u, 0u);
+            st_shared_v4(s_base + sw128_off(r, 0), iw[0].x, iw[0].y, iw[0].z, iw[0].w);
+            st_shared_v4(s_base + sw128_off(r, 1), iw[1].x, iw[1].y, 0u, 0u);
+            st_shared_v4(s_base + sw128_off(r, 2), iw[1].z, iw[1].w, iw[2].x, iw[2].y);
+            st_shared_v4(s_base + sw128_off(r, 3), iw[2].z, iw[2].w, 0u, 0u);
             fence_proxy_async_smem();
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(inrdy);
     };
     prepare_input(Work::tile(0), 0);
-    put_input(0);
+    {
+        uint4 iw[3];
+        load_input(0, iw);
+        put_input(iw);
+    }
     for (int it = 0; it < iters && ok; ++it) {
-        const int m = Work::tile(it) * 128 + r;
         if (SPLIT && it > 0) scr_row += (size_t)gridDim.x * 128 * EMU_NOUT;
         if (SPLIT && it == 0) scr_row += (size_t)blockIdx.x * 128 * EMU_NOUT;
         const bool stored = !SPLIT || Work::tile(it) < ntiles;
@@ -209,10 +283,10 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
             for (int L = 0; L < 5 && ok; ++L) {
                 const int nch = L == 4 ? 1 : 2;
                 for (int c = 0; c < nch; ++c) {
-                    if (!warp_wait(afull, g & 1u, status, ERR_TIMEOUT_EPILOGUE)) { ok = false; break; }
-                    ++g;
-                    tc_fence_after();
                     if (L < 4) {
+                        if (!warp_wait(afull, g & 1u, status, ERR_TIMEOUT_EPILOGUE)) { ok = false; break; }
+                        ++g;
+                        tc_fence_after();
                         // drain this slice (64 columns) and release the accumulator
                         uint32_t v[64];
                         const uint32_t ta = tmem_base + lane_base + EI_ACC_COL + cs * 64;
@@ -255,9 +329,17 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
                         }
                         __syncwarp();
                         if (lane == 0) mbar_arrive(&hrdy[c]);
-                        // the next tile's inputs, where the epilogue has time to spare
-                        if (mem == 0 && L == 1 && c == 0 && it + 1 < iters) prepare_input(Work::tile(it + 1), (it + 1) & 1);
+                        if (mem == 0 && L == 1 && c == 0) {
+                            // the next tile's inputs, where the epilogue has time to spare
+                            if (it + 1 < iters) prepare_input(Work::tile(it + 1), (it + 1) & 1);
+                        }
                     } else {
+                        // the next member's input row, or the next tile's after the last member (at the end any slot's)
+                        uint4 iw[3];
+                        load_input((mem + 1 < Work::STEPS || it + 1 == iters ? it : it + 1) & 1, iw);
+                        if (!warp_wait(afull, g & 1u, status, ERR_TIMEOUT_EPILOGUE)) { ok = false; break; }
+                        ++g;
+                        tc_fence_after();
                         // the output chunk (128 columns): this slice's 32
                         uint32_t v[32];
                         tmem_ld32_nowait(tmem_base + lane_base + EI_ACC_COL + cs * 32, v);
@@ -265,10 +347,8 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
                         tc_fence_before();
                         __syncwarp();
                         if (lane == 0) mbar_arrive(aempty);
-                        // S is free (the output layer's MMAs are done): the next member's input row, or the next
-                        // tile's after the last member
-                        if (mem + 1 < Work::STEPS) put_input(it & 1);
-                        else if (it + 1 < iters) put_input((it + 1) & 1);
+                        // S is free (the output layer's MMAs are done)
+                        if (mem + 1 < Work::STEPS || it + 1 < iters) put_input(iw);
                         const float4 *b4 = reinterpret_cast<const float4 *>(bm + 4 * EMU_H + cs * 32);
                         float4 *dst = reinterpret_cast<float4 *>(scr_row + mem * SCR_MEM + cs * 32);
 #pragma unroll
@@ -282,74 +362,28 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
             }
         }
         if (SPLIT) continue;
-        // ---- the ensemble's outputs of the quarter's rows: the four slices' scratch writes are in. The barrier is
-        // passed by all four warps whatever happened, and they stop together if any of them, or the status word,
-        // says so (a wait that gave up)
+        // ---- the ensemble's results of the quarter's rows: the four slices' scratch writes are in. The barrier is passed
+        // by all four warps whatever happened, and they stop together if any of them, or the status word, says so (a
+        // wait that gave up). A warp takes eight rows, a row over its lanes, two rows' loads together: a row per thread
+        // of one warp took 75 us of a tile's 220 with the MMAs idle, this about 12 (two warps of their own beside the next
+        // tile held its members back by more).
         if (named_bar_or(1 + q, 128, !ok || *(volatile int *)status != 0)) break;
-        if (m >= a.n) continue;
-        const float invm = 1.f / (float)EMU_MEMBERS;
-        if (cs < 2) {
-            if (a.coef) {
-                float *dst = a.coef + (size_t)m * EMU_NPC + cs * 32;
-#pragma unroll 2
-                for (int j = 0; j < 32; j += 4) {
-                    const int col = cs * 32 + j;
-                    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+        const int wrow = q * 32 + cs * 8, m0 = Work::tile(it) * 128 + wrow;
+        const float *out = scr_row - (size_t)r * EMU_NOUT + (size_t)wrow * EMU_NOUT + 4 * lane;
+        // (lane i: row i's flags, bit 0 outside the box, bit 1 not finite, and its distance term)
+        const uint4 t = __ldcg(in_row - (size_t)r * 4 + ((size_t)(it & 1) * 128 + wrow + (lane & 7)) * 4 + 3);
+        float mu[4], sg[4];
+        emu_scales(par, lane, mu, sg);
+#pragma unroll 1
+        for (int i = 0; i < 8; i += 2) {
+            float z[2][EMU_MEMBERS][4];
+            emu_load_row(out + (size_t)i * EMU_NOUT, SCR_MEM, z[0]);
+            emu_load_row(out + (size_t)(i + 1) * EMU_NOUT, SCR_MEM, z[1]);
 #pragma unroll
-                    for (int k = 0; k < EMU_MEMBERS; ++k) {
-                        const float4 t = *reinterpret_cast<const float4 *>(scr_row + k * SCR_MEM + col);
-                        sum.x += t.x; sum.y += t.y; sum.z += t.z; sum.w += t.w;
-                    }
-                    float4 o;
-                    o.x = par[EMU_P_OMU + col] + par[EMU_P_OSIG + col] * sum.x * invm;
-                    o.y = par[EMU_P_OMU + col + 1] + par[EMU_P_OSIG + col + 1] * sum.y * invm;
-                    o.z = par[EMU_P_OMU + col + 2] + par[EMU_P_OSIG + col + 2] * sum.z * invm;
-                    o.w = par[EMU_P_OMU + col + 3] + par[EMU_P_OSIG + col + 3] * sum.w * invm;
-                    *reinterpret_cast<float4 *>(dst + j) = o;
-                }
-            }
-        } else if (cs == 2) {
-            // the row's zred and flags from the tile's input slot (written by this quarter's cs = 0 warp)
-            const uint4 info = in_row[(size_t)(it & 1) * 128 * 4 + 3];
-            const bool outside = (info.y & 1u) != 0, bad = (info.y & 2u) != 0;
-            const float dd = emu_distance(__uint_as_float(info.x), par + EMU_P_ZT, par + EMU_P_DL);
-            const float *scr = scr_row + EMU_NPC;
-            // pass 1: the ensemble mean of each band (its magnitude) and the brightest band
-            float mmin = INFINITY;
-            bool finite = true;
-            float *mdst = a.mags + (size_t)m * a.nb;
-            for (int j = 0; j < a.nb; ++j) {
-                float sum = 0.f;
-#pragma unroll
-                for (int k = 0; k < EMU_MEMBERS; ++k) sum += scr[k * SCR_MEM + j];
-                const int o = EMU_NPC + j;
-                const float mag = par[EMU_P_OMU + o] + par[EMU_P_OSIG + o] * sum * invm + dd;
-                if (!isfinite(mag)) finite = false;
-                mmin = fminf(mmin, mag);
-                mdst[j] = mag;
-            }
-            // pass 2: the spread of the bands that count
-            float spread = 0.f;
-            for (int j = 0; j < a.nb; ++j) {
-                float z[EMU_MEMBERS], mean = 0.f;
-#pragma unroll
-                for (int k = 0; k < EMU_MEMBERS; ++k) { z[k] = scr[k * SCR_MEM + j]; mean += z[k]; }
-                mean *= invm;
-                float var = 0.f;
-#pragma unroll
-                for (int k = 0; k < EMU_MEMBERS; ++k) var += (z[k] - mean) * (z[k] - mean);
-                const int o = EMU_NPC + j;
-                const float sd = par[EMU_P_OSIG + o] * sqrtf(var * invm);
-                const float mag = par[EMU_P_OMU + o] + par[EMU_P_OSIG + o] * mean + dd;
-                if (!isfinite(sd)) finite = false;
-                if (mag < mmin + a.faint) spread = fmaxf(spread, sd);
-            }
-            const int f = outside ? 1 : (bad || !finite) ? 3 : (spread > a.spread_max) ? 2 : 0;
-            if (a.spread) a.spread[m] = spread;
-            a.flag[m] = f;
-            if (f) {
-                const int k = atomicAdd(a.nflag, 1);
-                a.flagged[k] = m;
+            for (int k = 0; k < 2; ++k) {
+                const float d = __uint_as_float(__shfl_sync(0xffffffffu, t.z, i + k));
+                const uint32_t f = __shfl_sync(0xffffffffu, t.y, i + k);
+                if (m0 + i + k < a.n) emu_row(a, m0 + i + k, z[k], mu, sg, d, (f & 1u) != 0, (f & 2u) != 0, lane);
             }
         }
     }
@@ -489,73 +523,22 @@ emu_infer_kernel(const __grid_constant__ CUtensorMap tm_w0, const __grid_constan
     }
 }
 
-// The ensemble's results of a SPLIT batch, one warp per model: four outputs per lane, the members in the fused kernel's
-// order (member (k + tile) % EMU_MEMBERS at step k, the order of a CTA's first tile).
+// The ensemble's results of a SPLIT batch, one warp per model.
 __global__ void __launch_bounds__(256) emu_reduce_kernel(EmuInferArgs a, const float *out) {
     const int m = (blockIdx.x * 256 + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     if (m >= a.n) return;
-    const float *par = a.par;
     const int tile = m >> 7, r = m & 127;
-    const float invm = 1.f / (float)EMU_MEMBERS;
-    float z[EMU_MEMBERS][4];
-#pragma unroll
-    for (int k = 0; k < EMU_MEMBERS; ++k) {
-        const int unit = tile * EMU_MEMBERS + (k + tile) % EMU_MEMBERS;
-        const float4 t = *reinterpret_cast<const float4 *>(out + ((size_t)unit * 128 + r) * EMU_NOUT + 4 * lane);
-        z[k][0] = t.x; z[k][1] = t.y; z[k][2] = t.z; z[k][3] = t.w;
-    }
     float x[EMU_NIN], xs[EMU_NFEAT];
 #pragma unroll
     for (int i = 0; i < EMU_NIN; ++i) x[i] = __ldg(a.x + (size_t)m * EMU_NIN + i);
-    const bool outside = !emu_features(x, par, xs);
+    const bool outside = !emu_features(x, a.par, xs);
     bool bad = false;
 #pragma unroll
     for (int i = 0; i < EMU_NFEAT; ++i) bad = bad || !isfinite(xs[i]);
-    // (the fused kernel's distance of a model that is not finite is zred's too)
-    const float dd = emu_distance(x[5], par + EMU_P_ZT, par + EMU_P_DL);
-    float v[4], sd[4];
-    float mmin = INFINITY;
-    bool finite = true;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int col = 4 * lane + i, band = col - EMU_NPC;
-        float sum = 0.f;
-#pragma unroll
-        for (int k = 0; k < EMU_MEMBERS; ++k) sum += z[k][i];
-        v[i] = par[EMU_P_OMU + col] + par[EMU_P_OSIG + col] * sum * invm;
-        sd[i] = 0.f;
-        if (band < 0) continue;
-        v[i] += dd;
-        const float mean = sum * invm;
-        float var = 0.f;
-#pragma unroll
-        for (int k = 0; k < EMU_MEMBERS; ++k) var += (z[k][i] - mean) * (z[k][i] - mean);
-        sd[i] = par[EMU_P_OSIG + col] * sqrtf(var * invm);
-        if (band < a.nb) {
-            if (!isfinite(v[i]) || !isfinite(sd[i])) finite = false;
-            mmin = fminf(mmin, v[i]);
-            a.mags[(size_t)m * a.nb + band] = v[i];
-        }
-    }
-    if (a.coef && 4 * lane < EMU_NPC)
-        *reinterpret_cast<float4 *>(a.coef + (size_t)m * EMU_NPC + 4 * lane) = make_float4(v[0], v[1], v[2], v[3]);
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) mmin = fminf(mmin, __shfl_xor_sync(0xffffffffu, mmin, off));
-    float spread = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int band = 4 * lane + i - EMU_NPC;
-        if (band >= 0 && band < a.nb && v[i] < mmin + a.faint) spread = fmaxf(spread, sd[i]);
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) spread = fmaxf(spread, __shfl_xor_sync(0xffffffffu, spread, off));
-    finite = __all_sync(0xffffffffu, finite);
-    if (lane == 0) {
-        const int f = outside ? 1 : (bad || !finite) ? 3 : (spread > a.spread_max) ? 2 : 0;
-        if (a.spread) a.spread[m] = spread;
-        a.flag[m] = f;
-        if (f) a.flagged[atomicAdd(a.nflag, 1)] = m;
-    }
+    float z[EMU_MEMBERS][4], mu[4], sg[4];
+    emu_load_row(out + ((size_t)tile * EMU_MEMBERS * 128 + r) * EMU_NOUT + 4 * lane, (size_t)128 * EMU_NOUT, z);
+    emu_scales(a.par, lane, mu, sg);
+    emu_row(a, m, z, mu, sg, emu_distance(x[5], a.par + EMU_P_ZT, a.par + EMU_P_DL), outside, bad, lane);
 }
 
 // One member per CTA while that shortens the longest CTA: members (tiles x 5) in rounds of num_sms against five members
