@@ -114,6 +114,7 @@ struct Emulator {
     int *d_flag = nullptr, *d_nflag = nullptr, *d_flagged = nullptr;
     float *d_scratch = nullptr;                  // the inference kernel's tile inputs and member outputs
     size_t scratch_cap = 0;                      // its floats
+    float *h_stage = nullptr;                    // page-locked staging of predict's inputs and outputs
     int cap = 0;
     void release();
 };

@@ -63,6 +63,8 @@ void Emulator::release() {
     bias = d_par = d_pca_mean = d_pca_basis = master = adam_m = adam_v = nullptr;
     d_x = d_mags = d_coef = d_spread = d_scratch = nullptr;
     scratch_cap = 0;
+    if (h_stage) cudaFreeHost(h_stage);
+    h_stage = nullptr;
     d_flag = d_nflag = d_flagged = nullptr;
     cap = 0;
     ready = trainable = false;
@@ -751,8 +753,11 @@ static int emu_step(Context &c, Emulator &e, EmuTrainBufs &b, const float *y, co
 }
 
 // ---------------------------------------------------------------------------------------------- inference scratch
+// (at least 16384 models' worth, 8 MB: small batches of growing size do not allocate again; with page-locked staging of
+// the inputs and outputs, x then mags, coef, spread and flags)
 static int emu_scratch(Emulator &e, int n, std::string &err) {
     if (n <= e.cap) return 0;
+    n = std::max(n, 16384);
     for (void *p : {(void *)e.d_x, (void *)e.d_mags, (void *)e.d_coef, (void *)e.d_spread, (void *)e.d_flag,
                     (void *)e.d_flagged})
         if (p) cudaFree(p);
@@ -767,6 +772,9 @@ static int emu_scratch(Emulator &e, int n, std::string &err) {
     ok(dalloc(&e.d_flag, (size_t)n));
     ok(dalloc(&e.d_flagged, (size_t)n));
     if (!e.d_nflag) ok(dalloc(&e.d_nflag, 4));
+    if (e.h_stage) cudaFreeHost(e.h_stage);
+    e.h_stage = nullptr;
+    ok(cudaMallocHost(&e.h_stage, sizeof(float) * (size_t)n * (EMU_NIN + EMU_MAX_BANDS + EMU_NPC + 2)));
     if (r != cudaSuccess) { err = cmsg("emulator scratch", r); e.cap = 0; return ST_DATA_MISSING; }
     e.cap = n;
     return 0;
@@ -778,8 +786,10 @@ int emu_infer_device(Context &c, int n, const float *d_x, float *d_mags, float *
     Emulator &e = c.emu;
     if (!e.ready) { err = "no emulator on the context (opensps_gb300_emulator_load / _train)"; return ST_NO_OPERATOR; }
     if (e.nb != c.nbands) { err = "the emulator was trained for another band set"; return ST_UNSUPPORTED; }
-    const size_t need = emu_scratch_floats(n, c.num_sms);
-    if (e.scratch_cap < need) {
+    if (e.scratch_cap < emu_scratch_floats(n, c.num_sms)) {
+        // (the most any batch takes: one member of a tile per CTA up to two tiles per SM, else the CTAs' own)
+        size_t need = 0;
+        for (int t = 1; t <= 2 * c.num_sms + 1; ++t) need = std::max(need, emu_scratch_floats(128 * t, c.num_sms));
         cudaFree(e.d_scratch);
         e.d_scratch = nullptr;
         e.scratch_cap = 0;
@@ -1378,32 +1388,29 @@ int emu_predict(Context &c, int n, const double *inputs, int fallback, double *m
     if (!inputs) { err = "emulator: inputs are NULL"; return ST_BAD_ARG; }
     if (int rc = emu_scratch(e, n, err)) return rc;
     const int nb = e.nb;
-    std::vector<float> xh((size_t)n * EMU_NIN);
-    for (int m = 0; m < n; ++m)
-        for (int i = 0; i < EMU_NIN; ++i) xh[(size_t)m * EMU_NIN + i] = (float)inputs[(size_t)i + (size_t)EMU_NIN * m];
-    cudaMemcpyAsync(e.d_x, xh.data(), sizeof(float) * xh.size(), cudaMemcpyHostToDevice, c.stream);
+    float *xh = e.h_stage, *mg = xh + (size_t)n * EMU_NIN, *cf = mg + (size_t)n * nb, *sp = cf + (size_t)n * EMU_NPC;
+    int *fl = reinterpret_cast<int *>(sp + n);
+    for (size_t i = 0; i < (size_t)n * EMU_NIN; ++i) xh[i] = (float)inputs[i];
+    cudaMemcpyAsync(e.d_x, xh, sizeof(float) * n * EMU_NIN, cudaMemcpyHostToDevice, c.stream);
     if (int rc = emu_infer_device(c, n, e.d_x, e.d_mags, pca ? e.d_coef : nullptr, e.d_spread, e.d_flag, e.d_nflag,
                                   e.d_flagged, err))
         return rc;
-    std::vector<float> mg((size_t)n * nb), cf(pca ? (size_t)n * EMU_NPC : 0), sp(spread ? n : 0);
-    std::vector<int> fl(n);
     int nf = 0;
-    cudaMemcpyAsync(mg.data(), e.d_mags, sizeof(float) * mg.size(), cudaMemcpyDeviceToHost, c.stream);
-    cudaMemcpyAsync(fl.data(), e.d_flag, sizeof(int) * n, cudaMemcpyDeviceToHost, c.stream);
-    cudaMemcpyAsync(&nf, e.d_nflag, sizeof(int), cudaMemcpyDeviceToHost, c.stream);
-    if (pca) cudaMemcpyAsync(cf.data(), e.d_coef, sizeof(float) * cf.size(), cudaMemcpyDeviceToHost, c.stream);
-    if (spread) cudaMemcpyAsync(sp.data(), e.d_spread, sizeof(float) * n, cudaMemcpyDeviceToHost, c.stream);
+    cudaMemcpyAsync(mg, e.d_mags, sizeof(float) * n * nb, cudaMemcpyDeviceToHost, c.stream);
+    cudaMemcpyAsync(fl, e.d_flag, sizeof(int) * n, cudaMemcpyDeviceToHost, c.stream);
+    if (pca) cudaMemcpyAsync(cf, e.d_coef, sizeof(float) * n * EMU_NPC, cudaMemcpyDeviceToHost, c.stream);
+    if (spread) cudaMemcpyAsync(sp, e.d_spread, sizeof(float) * n, cudaMemcpyDeviceToHost, c.stream);
     if (int rc = check_status(c, err)) return rc;
     if (mags)
-        for (int m = 0; m < n; ++m)
-            for (int b = 0; b < nb; ++b) mags[(size_t)b + (size_t)nb * m] = mg[(size_t)m * nb + b];
+        for (size_t i = 0; i < (size_t)n * nb; ++i) mags[i] = mg[i];
     if (pca)
-        for (int m = 0; m < n; ++m)
-            for (int k = 0; k < EMU_NPC; ++k) pca[(size_t)k + (size_t)EMU_NPC * m] = cf[(size_t)m * EMU_NPC + k];
+        for (size_t i = 0; i < (size_t)n * EMU_NPC; ++i) pca[i] = cf[i];
     if (spread)
         for (int m = 0; m < n; ++m) spread[m] = sp[m];
-    if (source)
-        for (int m = 0; m < n; ++m) source[m] = fl[m];
+    for (int m = 0; m < n; ++m) {
+        if (source) source[m] = fl[m];
+        nf += fl[m] != 0;
+    }
     if (n_fallback) *n_fallback = nf;
     if (!fallback || nf == 0) return 0;
     // ---- the flagged models through the plain CSP (in model order)
