@@ -181,7 +181,7 @@ Context::~Context() {
     d_logage.release(); d_lz.release(); d_lbol.release(); d_sfhpar.release(); d_wgiven.release(); d_w.release();
     d_sfh_scratch.release(); d_lblend.release(); d_sfr.release(); d_wbar.release(); d_dual.release(); d_sfhtab.release(); d_user_imf.release();
     ops.release(); dustem.release(); agn.release(); neb.release(); d_alpha.release(); d_vhi.release(); d_vlo.release(); d_yo.release(); d_vpart.release();
-    d_spart.release(); d_vflag.release(); d_vbar.release(); d_apart.release(); d_ix_hi.release(); d_ix_lo.release(); d_ipart.release(); d_bpart.release(); d_sfh_mtab.release(); d_ix_const.release(); d_ix_dln.release(); d_dem.release(); d_w64.release(); d_y64.release(); d_bc64.release(); d_igm_a64.release();
+    d_spart.release(); d_vflag.release(); d_vbar.release(); d_apart.release(); d_ix_hi.release(); d_ix_lo.release(); d_ipart.release(); d_bpart.release(); d_sfh_mtab.release(); d_ix_const.release(); d_ix_dln.release(); d_fold.release(); d_dem.release(); d_w64.release(); d_y64.release(); d_bc64.release(); d_igm_a64.release();
     fp64_release(*this);
     emu.release();
     if (pinned_spec) cudaFreeHost(pinned_spec);
@@ -194,6 +194,9 @@ Context::~Context() {
     if (pinned_sums) cudaFreeHost(pinned_sums);
     pinned_sums = nullptr;
     pinned_sums_n = 0;
+    if (pinned_fold) cudaFreeHost(pinned_fold);
+    pinned_fold = nullptr;
+    pinned_fold_n = 0;
     if (pinned_sfh) cudaFreeHost(pinned_sfh);
     pinned_sfh = nullptr;
     pinned_sfh_n = 0;
@@ -773,8 +776,8 @@ int context_setup_grid(Context &c, std::string &err) {
     for (int j = 0; j < c.jtop; ++j) igm_pixel_terms(c.lam[j], igm_a64.data() + (size_t)j * 6);
     std::vector<double> lnlam(ns);
     for (int j = 0; j < ns; ++j) lnlam[j] = std::log(c.lam[j]);
-    std::vector<double> lzv(c.nz);
-    for (int z = 0; z < c.nz; ++z) lzv[z] = std::log10(c.zlegend[z] / c.zsol);
+    c.lzv.resize(c.nz);
+    for (int z = 0; z < c.nz; ++z) c.lzv[z] = std::log10(c.zlegend[z] / c.zsol);
     cosmology_table(c.h0, c.om0, c.ol0, c.zt, c.dl);
     std::vector<double> ages(c.log_age);   // log10 of the grid's ages, then the ages (yr)
     for (int t = 0; t < c.nt; ++t) ages.push_back(std::pow(10.0, c.log_age[t]));
@@ -786,7 +789,7 @@ int context_setup_grid(Context &c, std::string &err) {
         (e = upload(c.d_mass, c.mass.data(), c.mass.size())) != cudaSuccess ||
         (e = upload(c.d_llin, c.llin.data(), c.llin.size())) != cudaSuccess ||
         (e = upload(c.d_logage, ages.data(), ages.size())) != cudaSuccess ||
-        (e = upload(c.d_lz, lzv.data(), lzv.size())) != cudaSuccess ||
+        (e = upload(c.d_lz, c.lzv.data(), c.lzv.size())) != cudaSuccess ||
         (e = upload(c.d_lbol, c.lbol.data(), c.lbol.size())) != cudaSuccess ||
         (e = upload(c.d_zt, c.zt.data(), c.zt.size())) != cudaSuccess ||
         (e = upload(c.d_dl, c.dl.data(), c.dl.size())) != cudaSuccess ||

@@ -231,6 +231,7 @@ struct Context {
     int nspec = 0, nt = 0, nz = 0, nline = 0, nbands = 0;
     double zsol = 0.0142, dlnl = 0.0;
     std::vector<double> lam, log_age, zlegend, ssp, mass, lbol, line_lambda, line_lum, bands, band_center;
+    std::vector<double> lzv;     // log10(Z / Zsun)
     std::vector<double> llin;    // 10^lbol
     std::vector<double> zt, dl;  // cosmology table (500)
     std::vector<float> igm_a;    // jtop x 6 Madau wavelength factors
@@ -307,6 +308,8 @@ struct Context {
     DevBuf<double> d_spart;
     DevBuf<__nv_bfloat16> d_ix_hi, d_ix_lo;   // the interpolated fold's operand: node values x SFH weights
     DevBuf<float> d_ipart;       // and its GEMM's split-K partial sums
+    DevBuf<int4> d_fold;         // the fold's M tiles, then its rows' (model, slab) pairs (models sorted by metallicity)
+    int4 *pinned_fold = nullptr; size_t pinned_fold_n = 0;
     DevBuf<double2> d_ix_const;  // and each model's 1 / T and c2
     DevBuf<double> d_ix_dln;     // and d ln T / d alpha (the reverse pass)
     DevBuf<DustEmModel> d_dem;   // the batch's dust emission cells (one per model)
@@ -407,8 +410,9 @@ int run_fp64_tail(Context &c, const BatchIO &io, BasisOperand *bop, const double
 void fp64_release(Context &c);
 // the reverse of the interpolated fold (ssp_op.cu): r as for run_ops_reverse, the template cotangents in r.vbar
 int run_ops_interp_reverse(Context &c, const OpsRevArgs &r, std::string &err);
-int run_ops_parts(Context &c, int n, const double *d_wz, const double *d_alpha, const double *h_alpha, int itesc,
-                  float *d_young, float *d_old, std::string &err);
+// (h_sfh: the SFH columns of weights blended at logzsol, host, or null)
+int run_ops_parts(Context &c, int n, const double *d_wz, const double *d_alpha, const double *h_alpha, const double *h_sfh,
+                  int itesc, float *d_young, float *d_old, std::string &err);
 void imf_pack(int imf_type, const double *pv, double *ap);
 // The IMF's limits and user segments for the operator kernels (the user IMF read and uploaded when imf_type is 5): 0,
 // or ST_IMF_FILE / ST_DATA_MISSING with err.

@@ -196,6 +196,10 @@ struct GemmArgs {
     long long a_grp = 0, b_grp = 0;              // rows between the groups' A / B operands
     long long d_grp = 0, d_split = 0;            // elements between the groups' / splits' D
     int f16 = 0;                                 // one-product kind: operands f16 (else bf16)
+    // slabs (three products only; mtab null: none): per M tile (first row, end row, slab z, 0), the tiles, the ages, the
+    // columns of an age's two slabs in A and of all its slabs in B
+    const int4 *mtab = nullptr;
+    int n_mtiles = 0, ages = 0, slab2 = 0, age_cols = 0;
 };
 struct GemmPlan {
     CUtensorMap tm_a_hi, tm_a_lo, tm_b_hi, tm_b_lo;
@@ -350,6 +354,9 @@ struct OpsFoldArgs {
 cudaError_t run_ops_fold(const OpsFoldArgs &a, cudaStream_t st);
 // The interpolated fold's operand (one row per model of a chunk) and its GEMM's reduction.
 struct OpsInterpArgs {
+    // slabs (rowz null: none): per row of the chunk its model and the lower of the two metallicities that hold its weights;
+    // the operand then has the columns (age, slab of the two, node) of those alone
+    const int2 *rowz = nullptr;
     int m0, nt, nz, R, ktot, itesc;          // models m0 .. m0 + gridDim.x - 1; ktot = nt nz R columns
     int imf_type = 2;                        // 2 Kroupa (slopes per model; 0 Salpeter as Kroupa), 1 Chabrier
     unsigned rg_magic;                       // 2^32 / (R / 8), rounded up
@@ -365,6 +372,7 @@ struct OpsInterpArgs {
 struct OpsInterpReduceArgs {
     int n, m0, rows, ntpad, ntempl, ks_young, ks_old;
     const float *part_young, *part_old;      // ks x rows x ntpad split-K partial sums
+    const int2 *rowz = nullptr;              // the rows' models (OpsInterpArgs::rowz), or null: m0 + row
     __nv_bfloat16 *v_hi, *v_lo;              // 2n x ntpad
 };
 // The operator's reverse pass: from the template cotangents, the cotangents of the SFH weights over ages and

@@ -13,6 +13,11 @@
 // [s * nkb / ksplit, (s + 1) * nkb / ksplit) and writes its partial sums from s * d_split. The emulator's five
 // ensemble members are the groups; the weight gradients (K = the minibatch) are split over K.
 //
+// Slabs (mtab): the operator's fold of models whose weights lie in two metallicity slabs z, z + 1 of every age. An M tile
+// holds rows of one z; a K block is 64 columns of an age's two slabs (slab2 columns, contiguous in A's rows at age slab2
+// and in B's at age age_cols + z slab2 / 2), so that the other slabs' columns, all zero in A, are neither read nor
+// multiplied.
+//
 // Tile 128 x 256 x 64, persistent CTAs over tiles; warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner,
 // warps 2..5 = epilogue (one accumulator row per thread); TMEM double-buffered. Two smem stages of 96 KB (split) or
 // four of 48 KB (plain). Every mbarrier wait is bounded (status word, no hang).
@@ -38,11 +43,18 @@ struct GemmCfg {
 };
 
 struct GemmTile {
-    int g, s, m0, n0;
+    int g, s, m0, n0, rows, z;   // rows: of D from m0 that this tile stores (an end); z: its slab (GemmArgs::mtab)
 };
+template <bool SLABS>
 __device__ __forceinline__ GemmTile gemm_tile(const GemmArgs &g, int tile, int mt_n, int nt_n) {
     GemmTile t;
     t.m0 = (tile % mt_n) * G_BM;
+    t.rows = g.M;
+    t.z = 0;
+    if constexpr (SLABS) {
+        const int4 e = __ldg(g.mtab + tile % mt_n);
+        t.m0 = e.x; t.rows = e.y; t.z = e.z;
+    }
     int r = tile / mt_n;
     t.n0 = (r % nt_n) * G_BN;
     r /= nt_n;
@@ -51,7 +63,7 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmArgs &g, int tile, int m
     return t;
 }
 
-template <int NPROD>
+template <int NPROD, bool SLABS>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
                  const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
@@ -65,9 +77,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
     uint64_t *mma_done = bars + 2 * NS + 4;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NS + 5);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt_n = (g.M + G_BM - 1) / G_BM, nt_n = (g.N + G_BN - 1) / G_BN;
+    const int mt_n = SLABS ? g.n_mtiles : (g.M + G_BM - 1) / G_BM, nt_n = (g.N + G_BN - 1) / G_BN;
     const int n_tiles = mt_n * nt_n * g.ksplit * g.groups;
-    const int nkb = (g.K + G_BK - 1) / G_BK;
+    // (SLABS: K blocks of an age's two slabs, kpa of them, the last with ktail columns)
+    const int kpa = SLABS ? (g.slab2 + G_BK - 1) / G_BK : 1, nkb = SLABS ? g.ages * kpa : (g.K + G_BK - 1) / G_BK;
+    const int tail_steps = SLABS ? (g.slab2 - (kpa - 1) * G_BK + 15) / 16 : G_BK / 16;
     int *status = g.status;
 
     if (threadIdx.x == 0) {
@@ -89,7 +103,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
             for (int i = 0; i < NS; ++i) last_fill[i] = -1;
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const GemmTile t = gemm_tile(g, tile, mt_n, nt_n);
+                const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
                 const int arow = (int)(t.g * g.a_grp) + t.m0;
                 const int brow = (int)(t.g * g.b_grp) + g.b_row0 + t.n0;
                 const int kb0 = t.s * nkb / g.ksplit, kb1 = (t.s + 1) * nkb / g.ksplit;
@@ -98,10 +112,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                     uint8_t *st = smem + s * C::STAGE_BYTES;
                     mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
                     if (NPROD == 3) {
-                        tma_load_2d(st, &tm_a_hi, kb * G_BK, arow, &full[s]);
-                        tma_load_2d(st + G_A_BYTES, &tm_a_lo, kb * G_BK, arow, &full[s]);
-                        tma_load_2d(st + 2 * G_A_BYTES, &tm_b_hi, kb * G_BK, brow, &full[s]);
-                        tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES, &tm_b_lo, kb * G_BK, brow, &full[s]);
+                        int xa = kb * G_BK, xb = xa;
+                        if constexpr (SLABS) {
+                            const int age = kb / kpa, off = (kb - age * kpa) * G_BK;
+                            xa = age * g.slab2 + off;
+                            xb = age * g.age_cols + t.z * (g.slab2 / 2) + off;
+                        }
+                        tma_load_2d(st, &tm_a_hi, xa, arow, &full[s]);
+                        tma_load_2d(st + G_A_BYTES, &tm_a_lo, xa, arow, &full[s]);
+                        tma_load_2d(st + 2 * G_A_BYTES, &tm_b_hi, xb, brow, &full[s]);
+                        tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES, &tm_b_lo, xb, brow, &full[s]);
                     } else {
                         tma_load_2d(st, &tm_a_hi, kb * G_BK, arow, &full[s]);
                         tma_load_2d(st + G_A_BYTES, &tm_b_hi, kb * G_BK, brow, &full[s]);
@@ -119,7 +139,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
             int acc = 0; uint32_t aph = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const GemmTile t = gemm_tile(g, tile, mt_n, nt_n);
+                const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
                 const int kb0 = t.s * nkb / g.ksplit, kb1 = (t.s + 1) * nkb / g.ksplit;
                 if (!mbar_wait(&tempty[acc], aph ^ 1u, status, ERR_TIMEOUT_MMA)) { ok = false; break; }
                 tc_fence_after();
@@ -131,6 +151,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                     const uint32_t sa = smem_u32(smem + s * C::STAGE_BYTES);
 #pragma unroll
                     for (int k = 0; k < G_BK / 16; ++k) {
+                        if (SLABS && k >= tail_steps && kb % kpa == kpa - 1) break;
                         const uint32_t off = k * 32;
                         const uint32_t first = (kb > kb0 || k > 0) ? 1u : 0u;
                         if (NPROD == 3) {
@@ -157,7 +178,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
         const int q = warp & 3;
         int acc = 0; uint32_t aph = 0;
         for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const GemmTile t = gemm_tile(g, tile, mt_n, nt_n);
+            const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
             mbar_wait(&tfull[acc], aph, status, ERR_TIMEOUT_EPILOGUE);
             named_bar_sync(1, 128);
             if (*(volatile int *)status != 0) break;
@@ -169,7 +190,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                 if (t.n0 + c >= g.N) break;
                 float v[32];
                 tmem_ld32(trow + c, v);
-                if (row < g.M) {
+                if (row < t.rows) {
                     float *dst = dbase + (size_t)row * g.ldd + t.n0 + c;
                     if (t.n0 + c + 32 <= g.N && ((g.ldd | g.d_grp | g.d_split) & 3) == 0) {
 #pragma unroll
@@ -215,22 +236,24 @@ int gemm_choose_ksplit(int tiles_mn, int nkb, int num_sms) {
     return best;
 }
 
-template <int NPROD>
+template <int NPROD, bool SLABS = false>
 static cudaError_t launch_gemm(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.groups <= 0 || g.ksplit <= 0) return cudaSuccess;
-    const int nkb = (g.K + G_BK - 1) / G_BK;
+    const int nkb = SLABS ? g.ages * ((g.slab2 + G_BK - 1) / G_BK) : (g.K + G_BK - 1) / G_BK;
     if (g.ksplit > nkb) return cudaErrorInvalidValue;          // every split needs a K block
     if ((reinterpret_cast<uintptr_t>(g.D) & 15) != 0) return cudaErrorInvalidValue;
     using C = GemmCfg<NPROD>;
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<NPROD>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<NPROD, SLABS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) return e;
-    const long long tiles = (long long)((g.M + G_BM - 1) / G_BM) * ((g.N + G_BN - 1) / G_BN) * g.ksplit * g.groups;
+    const long long tiles = (long long)(SLABS ? g.n_mtiles : (g.M + G_BM - 1) / G_BM) * ((g.N + G_BN - 1) / G_BN) * g.ksplit * g.groups;
     const int grid = tiles < pl.num_sms ? (int)tiles : pl.num_sms;
-    gemm_bf16_kernel<NPROD><<<grid, G_THREADS, C::SMEM, st>>>(pl.tm_a_hi, pl.tm_a_lo, pl.tm_b_hi, pl.tm_b_lo, g);
+    gemm_bf16_kernel<NPROD, SLABS><<<grid, G_THREADS, C::SMEM, st>>>(pl.tm_a_hi, pl.tm_a_lo, pl.tm_b_hi, pl.tm_b_lo, g);
     return cudaGetLastError();
 }
 
-cudaError_t run_gemm_bf16x3(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) { return launch_gemm<3>(pl, g, st); }
+cudaError_t run_gemm_bf16x3(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) {
+    return g.mtab ? launch_gemm<3, true>(pl, g, st) : launch_gemm<3>(pl, g, st);
+}
 cudaError_t run_gemm_bf16(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) { return launch_gemm<1>(pl, g, st); }
 
 }  // namespace sps

@@ -715,18 +715,24 @@ __device__ __forceinline__ double ops_node_value(int imf_type, int q, double x, 
     return (q == 0 ? 1.0 : c2) * it * exp(-al[q] * x);
 }
 
+//
+// SLABS: the operand's columns of the model's two slabs only (age, slab, node). The column groups' terms of the sums go
+// through shared memory, where each thread adds those it has in the full operand's order and flushes to FP64 at the same
+// places, so that the sums keep their bits (the groups left out are zero).
+template <bool SLABS>
 __global__ void __launch_bounds__(OPS_IX_THREADS) ops_interp_x_kernel(OpsInterpArgs a) {
     __shared__ __align__(16) float ctk[OPS_IMAXR];
     __shared__ float sws[OPS_IMAXG];
     __shared__ double red[OPS_IX_THREADS / 32][4];
-    const int row = blockIdx.x, m = a.m0 + row, tid = threadIdx.x;
+    const int2 rz = SLABS ? a.rowz[blockIdx.x] : make_int2(a.m0 + (int)blockIdx.x, 0);
+    const int row = blockIdx.x, m = rz.x, zlo = rz.y, tid = threadIdx.x;
     const int ng = a.nt * a.nz;
     const double *al = a.alpha + 3 * (size_t)m;
     const double *wzm = a.wz + (size_t)ng * m;
-    for (int g = tid; g < ng; g += OPS_IX_THREADS) {
+    for (int g = tid; g < (SLABS ? 2 * a.nt : ng); g += OPS_IX_THREADS) {
         const int t = g % a.nt, z = g / a.nt;                 // the weights' order: age fastest
-        const double sw = wzm[g];
-        sws[t * a.nz + z] = sw > SAFE_FLOOR ? (float)sw : 0.f;   // the columns' order: (t nz + z)
+        const double sw = wzm[SLABS ? g + zlo * a.nt : g];
+        sws[SLABS ? 2 * t + z : t * a.nz + z] = sw > SAFE_FLOOR ? (float)sw : 0.f;   // the columns' order: (t nz + z)
     }
     const double2 kc = a.kconst[m];                  // 1 / T, c2
     const double it = kc.x, c2 = kc.y;
@@ -743,9 +749,11 @@ __global__ void __launch_bounds__(OPS_IX_THREADS) ops_interp_x_kernel(OpsInterpA
         ctk[r] = v;
     }
     __syncthreads();
+    extern __shared__ float2 terms[];                // SLABS: the groups' mass and L_bol terms
     const int rg = a.R >> 3, ngrp = ng * rg, gyoung = a.itesc * a.nz;
-    uint4 *xh = reinterpret_cast<uint4 *>(a.x_hi + (size_t)row * a.ktot);
-    uint4 *xl = reinterpret_cast<uint4 *>(a.x_lo + (size_t)row * a.ktot);
+    const size_t ld = SLABS ? (size_t)2 * a.nt * a.R : (size_t)a.ktot;
+    uint4 *xh = reinterpret_cast<uint4 *>(a.x_hi + (size_t)row * ld);
+    uint4 *xl = reinterpret_cast<uint4 *>(a.x_lo + (size_t)row * ld);
     const float4 *mr4 = reinterpret_cast<const float4 *>(a.mrow), *lr4 = reinterpret_cast<const float4 *>(a.lrow);
     const float4 *ct4 = reinterpret_cast<const float4 *>(ctk);
     // mass young, mass old, L_bol young, L_bol old: FP32 over up to 16 thread steps, then FP64 (GB300's FP64 pipe
@@ -753,10 +761,8 @@ __global__ void __launch_bounds__(OPS_IX_THREADS) ops_interp_x_kernel(OpsInterpA
     double acc[4] = {0.0, 0.0, 0.0, 0.0};
     float fac[4] = {0.f, 0.f, 0.f, 0.f};
     int nstep = 0;
-    for (int q = tid; q < ngrp; q += OPS_IX_THREADS) {
-        const int gp = (int)__umulhi((unsigned)q, a.rg_magic);
-        const int rq = q - gp * rg;
-        const float sw = sws[gp];
+    // column group rq of a grid point with the weight sw: its operand columns at qx, its terms of the sums
+    auto group = [&](int q, int rq, int qx, float sw) -> float2 {
         const float4 c0 = ct4[2 * rq], c1 = ct4[2 * rq + 1];
         const float4 ma = __ldg(mr4 + 2 * (size_t)q), mb = __ldg(mr4 + 2 * (size_t)q + 1);
         const float4 la = __ldg(lr4 + 2 * (size_t)q), lb = __ldg(lr4 + 2 * (size_t)q + 1);
@@ -775,15 +781,46 @@ __global__ void __launch_bounds__(OPS_IX_THREADS) ops_interp_x_kernel(OpsInterpA
             ms = fmaf(v[i], mrv[i], fmaf(v[i + 1], mrv[i + 1], ms));
             ls = fmaf(v[i], lrv[i], fmaf(v[i + 1], lrv[i + 1], ls));
         }
-        xh[q] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
-        xl[q] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
-        const int part = gp < gyoung ? 0 : 1;
-        fac[part] += ms;
-        fac[2 + part] += ls;
-        if (++nstep == 16) {
+        xh[qx] = make_uint4(hw[0], hw[1], hw[2], hw[3]);
+        xl[qx] = make_uint4(lw[0], lw[1], lw[2], lw[3]);
+        return make_float2(ms, ls);
+    };
+    auto add = [&](int part, float2 v) {
+        fac[part] += v.x;
+        fac[2 + part] += v.y;
+    };
+    auto flush = [&]() {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) { acc[i] += (double)fac[i]; fac[i] = 0.f; }
-            nstep = 0;
+        for (int i = 0; i < 4; ++i) { acc[i] += (double)fac[i]; fac[i] = 0.f; }
+    };
+    if constexpr (SLABS) {
+        const unsigned magic2 = a.rg_magic;          // (of a grid point's rg groups)
+        for (int qx = tid; qx < 2 * a.nt * rg; qx += OPS_IX_THREADS) {
+            const int g2 = (int)__umulhi((unsigned)qx, magic2), rq = qx - g2 * rg, t = g2 >> 1, z = g2 & 1;
+            terms[qx] = group((t * a.nz + zlo + z) * rg + rq, rq, qx, sws[g2]);
+        }
+        __syncthreads();
+        // an age's groups lie at q = (t nz + zlo) rg .. + 2 rg - 1: this thread's (q = tid mod 256) is at most one of
+        // them while 2 rg <= 256 (R <= OPS_IMAXR)
+        static_assert(2 * OPS_IMAXR / 8 <= OPS_IX_THREADS, "a thread has one group per age");
+        // (the ages by the 16 thread steps their groups lie in, every lane flushing together: FP64 instructions take 64
+        // cycles however few lanes run them)
+        constexpr int SPAN = 16 * OPS_IX_THREADS;    // groups of a flush
+        const int tq = a.nz * rg;                    // groups from one age to the next
+        for (int s0 = 0; s0 < ngrp; s0 += SPAN) {
+            // ages whose groups q0 .. q0 + 2 rg - 1 reach into s0 .. s0 + SPAN - 1
+            const int t0 = max(0, (s0 - 2 * rg - zlo * rg) / tq), t1 = min(a.nt - 1, (s0 + SPAN) / tq);
+            for (int t = t0; t <= t1; ++t) {
+                const int q0 = t * tq + zlo * rg, d = (tid - q0) & (OPS_IX_THREADS - 1), q = q0 + d;
+                if (d < 2 * rg && q >= s0 && q < s0 + SPAN) add(t < a.itesc ? 0 : 1, terms[2 * t * rg + d]);
+            }
+            flush();
+        }
+    } else {
+        for (int q = tid; q < ngrp; q += OPS_IX_THREADS) {
+            const int gp = (int)__umulhi((unsigned)q, a.rg_magic);
+            add(gp < gyoung ? 0 : 1, group(q, q - gp * rg, q, sws[gp]));
+            if (++nstep == 16) { flush(); nstep = 0; }
         }
     }
 #pragma unroll
@@ -826,7 +863,7 @@ __global__ void ops_interp_reduce_kernel(OpsInterpReduceArgs a) {
                 v.x += p.x; v.y += p.y; v.z += p.z; v.w += p.w;
             }
         const float vv[4] = {v.x, v.y, v.z, v.w};
-        const size_t o = ((size_t)(part ? a.n : 0) + a.m0 + row) * a.ntpad + e;
+        const size_t o = ((size_t)(part ? a.n : 0) + (a.rowz ? a.rowz[row].x : a.m0 + row)) * a.ntpad + e;
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const float x = e + k < a.ntempl ? vv[k] : 0.f;
@@ -2146,19 +2183,74 @@ static bool ops_interp_ok(const Context &c, const double *h_alpha, int n) {
 
 // The interpolated fold of n models into the template GEMM's operand (d_vhi / d_vlo) and the sums: per chunk of
 // models the operand X, the young and old split-K GEMMs against the operator basis, their reduction.
-static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d_alpha, int itesc, std::string &err) {
+// With h_sfh (weights blended at logzsol between two metallicities) the models are sorted by their slabs and only those
+// slabs' columns are formed, read and multiplied: a sixth of the work at 12 metallicities (1024 models: the two
+// GEMMs 765 -> 265 us, the operand 151 -> 73).
+static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d_alpha, const double *h_sfh, int itesc,
+                          std::string &err) {
     SspOps &o = c.ops;
     cudaStream_t st = c.stream;
     cudaError_t e;
     const int nt = c.nt, nz = c.nz, R = o.interp_R;
     const size_t ktot = (size_t)nt * nz * R;
     if (nt * nz > OPS_IMAXG || (size_t)nt * nz * (R / 8) >= (1u << 20)) { err = "operator grid too large for the interpolated fold"; return ST_UNSUPPORTED; }
-    const int chunk = std::min(n, 4096);
+    const int chunk = std::min(n, 4096), nchunk = (n + chunk - 1) / chunk;
     const int ky = itesc * nz * R, ko = (nt - itesc) * nz * R;
-    const int tiles_mn = ((chunk + gemm_bm() - 1) / gemm_bm()) * ((o.ntempl + gemm_bn() - 1) / gemm_bn());
-    const int ks_y = ky > 0 ? gemm_choose_ksplit(tiles_mn, (ky + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
-    const int ks_o = ko > 0 ? gemm_choose_ksplit(tiles_mn, (ko + gemm_bk() - 1) / gemm_bk(), c.num_sms) : 0;
-    if ((e = c.d_ix_hi.reserve((size_t)chunk * ktot)) != cudaSuccess || (e = c.d_ix_lo.reserve((size_t)chunk * ktot)) != cudaSuccess ||
+    const bool slabs = h_sfh != nullptr && nz >= 2;
+    const int slab2 = 2 * R, kpa = (slab2 + gemm_bk() - 1) / gemm_bk();
+    // slabs: the models by the lower of their two metallicities (the interval sfh_forward_kernel takes), and per chunk of
+    // that order the M tiles of one metallicity
+    std::vector<int> tile0(nchunk + 1, 0);
+    if (slabs) {
+        const size_t cap = (size_t)n + n / gemm_bm() + (size_t)nchunk * nz;   // tiles (int4) and rows (two to an int4)
+        if (c.pinned_fold_n < cap) {
+            if (c.pinned_fold) cudaFreeHost(c.pinned_fold);
+            c.pinned_fold = nullptr;
+            c.pinned_fold_n = 0;
+            if ((e = cudaMallocHost(&c.pinned_fold, sizeof(int4) * cap)) != cudaSuccess) {
+                err = cmsg("page-locked fold tiles", e);
+                return ST_DATA_MISSING;
+            }
+            c.pinned_fold_n = cap;
+        }
+        std::vector<int> zl(n), at(nz + 1, 0);
+        for (int m = 0; m < n; ++m) {
+            const int k = find_interval0(c.lzv.data(), nz, h_sfh[(size_t)SFH_NCOL * m + SFH_LOGZSOL]) + 1;
+            zl[m] = std::max(1, std::min(k, nz - 1)) - 1;
+            ++at[zl[m] + 1];
+        }
+        for (int z = 0; z < nz; ++z) at[z + 1] += at[z];
+        int2 *rz = reinterpret_cast<int2 *>(c.pinned_fold);
+        for (int m = 0; m < n; ++m) rz[at[zl[m]]++] = make_int2(m, zl[m]);
+        int4 *mt = c.pinned_fold + (n + 1) / 2;
+        int nt_all = 0;
+        for (int k = 0; k < nchunk; ++k) {
+            tile0[k] = nt_all;
+            const int r0 = k * chunk, r1 = std::min(n, r0 + chunk);
+            for (int r = r0; r < r1;) {
+                int end = r;
+                while (end < r1 && rz[end].y == rz[r].y) ++end;
+                for (; r < end; r += gemm_bm()) mt[nt_all++] = make_int4(r - r0, end - r0, rz[end - 1].y, 0);
+                r = end;
+            }
+        }
+        tile0[nchunk] = nt_all;
+        const size_t used = (size_t)(n + 1) / 2 + nt_all;
+        if ((e = c.d_fold.reserve(cap)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(c.d_fold.p, c.pinned_fold, sizeof(int4) * used, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
+            err = cmsg("fold tiles", e);
+            return ST_DATA_MISSING;
+        }
+    }
+    // K blocks and K splits of the young and old ranges
+    const int nkb_y = slabs ? itesc * kpa : (ky + gemm_bk() - 1) / gemm_bk();
+    const int nkb_o = slabs ? (nt - itesc) * kpa : (ko + gemm_bk() - 1) / gemm_bk();
+    const int mtiles = slabs ? tile0[1] : (chunk + gemm_bm() - 1) / gemm_bm();
+    const int tiles_mn = mtiles * ((o.ntempl + gemm_bn() - 1) / gemm_bn());
+    const int ks_y = ky > 0 ? gemm_choose_ksplit(tiles_mn, nkb_y, c.num_sms) : 0;
+    const int ks_o = ko > 0 ? gemm_choose_ksplit(tiles_mn, nkb_o, c.num_sms) : 0;
+    const size_t xld = slabs ? (size_t)nt * slab2 : ktot;                    // the operand's columns
+    if ((e = c.d_ix_hi.reserve((size_t)chunk * xld)) != cudaSuccess || (e = c.d_ix_lo.reserve((size_t)chunk * xld)) != cudaSuccess ||
         (e = c.d_ix_const.reserve((size_t)n)) != cudaSuccess ||
         (e = c.d_ipart.reserve((size_t)std::max(ks_y + ks_o, 1) * chunk * o.ntpad)) != cudaSuccess) {
         err = cmsg("device memory", e);
@@ -2178,7 +2270,17 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
         xa.lim_lo = 0.08f; xa.lim_hi = 120.f; xa.imf_type = c.imf_type;
         xa.wz = d_wz; xa.alpha = d_alpha; xa.kconst = c.d_ix_const.p; xa.mrow = o.i_mrow.p; xa.lrow = o.i_lrow.p;
         xa.x_hi = c.d_ix_hi.p; xa.x_lo = c.d_ix_lo.p; xa.sums = c.d_sums.p;
-        ops_interp_x_kernel<<<rows, OPS_IX_THREADS, 0, st>>>(xa);
+        if (slabs) {
+            xa.rowz = reinterpret_cast<const int2 *>(c.d_fold.p) + m0;
+            const int smem = 2 * nt * (R / 8) * (int)sizeof(float2);
+            if ((e = cudaFuncSetAttribute(ops_interp_x_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) {
+                err = cmsg("interpolated fold operand kernel", e);
+                return ST_DATA_MISSING;
+            }
+            ops_interp_x_kernel<true><<<rows, OPS_IX_THREADS, smem, st>>>(xa);
+        } else {
+            ops_interp_x_kernel<false><<<rows, OPS_IX_THREADS, 0, st>>>(xa);
+        }
         c.ops_launches += 2 + (ky > 0 ? 1 : 0) + (ko > 0 ? 1 : 0);   // operand, GEMMs, reduction
         if ((e = cudaGetLastError()) != cudaSuccess) { err = cmsg("interpolated fold operand kernel", e); return ST_DATA_MISSING; }
         const size_t per = (size_t)rows * o.ntpad;
@@ -2186,10 +2288,12 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
             const int K = part ? ko : ky, ks = part ? ks_o : ks_y;
             if (K <= 0) continue;
             const size_t c0 = part ? (size_t)ky : 0;
+            const int ages = part ? nt - itesc : itesc;
+            const size_t a0 = !part ? 0 : slabs ? (size_t)itesc * slab2 : c0, ka = slabs ? (size_t)ages * slab2 : (size_t)K;
             GemmPlan pl;
             pl.num_sms = c.num_sms;
-            if ((e = encode_tmap_2d_16s(&pl.tm_a_hi, c.d_ix_hi.p + c0, K, rows, ktot, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
-                (e = encode_tmap_2d_16s(&pl.tm_a_lo, c.d_ix_lo.p + c0, K, rows, ktot, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
+            if ((e = encode_tmap_2d_16s(&pl.tm_a_hi, c.d_ix_hi.p + a0, ka, rows, xld, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
+                (e = encode_tmap_2d_16s(&pl.tm_a_lo, c.d_ix_lo.p + a0, ka, rows, xld, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
                 (e = encode_tmap_2d_16s(&pl.tm_b_hi, o.ib_hi.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_bn(), false)) != cudaSuccess ||
                 (e = encode_tmap_2d_16s(&pl.tm_b_lo, o.ib_lo.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_bn(), false)) != cudaSuccess) {
                 err = cmsg("interpolated fold tensor map", e);
@@ -2199,6 +2303,11 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
             g.M = rows; g.N = o.ntempl; g.K = K; g.ldd = o.ntpad; g.b_row0 = 0; g.status = c.d_status.p;
             g.D = c.d_ipart.p + (part ? (size_t)ks_y * per : 0);
             g.ksplit = ks; g.d_split = (long long)per;
+            if (slabs) {
+                g.mtab = c.d_fold.p + (n + 1) / 2 + tile0[m0 / chunk];
+                g.n_mtiles = tile0[m0 / chunk + 1] - tile0[m0 / chunk];
+                g.ages = ages; g.slab2 = slab2; g.age_cols = nz * R;
+            }
             if ((e = run_gemm_bf16x3(pl, g, st)) != cudaSuccess) { err = cmsg("interpolated fold GEMM", e); return ST_DATA_MISSING; }
         }
         OpsInterpReduceArgs ra;
@@ -2206,6 +2315,7 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
         ra.ks_young = ks_y; ra.ks_old = ks_o;
         ra.part_young = c.d_ipart.p; ra.part_old = c.d_ipart.p + (size_t)ks_y * per;
         ra.v_hi = c.d_vhi.p; ra.v_lo = c.d_vlo.p;
+        ra.rowz = slabs ? reinterpret_cast<const int2 *>(c.d_fold.p) + m0 : nullptr;
         const size_t n4 = 2 * per / 4;
         ops_interp_reduce_kernel<<<(unsigned)std::min<size_t>((n4 + 255) / 256, 4096), 256, 0, st>>>(ra);
         if ((e = cudaGetLastError()) != cudaSuccess) { err = cmsg("interpolated fold reduce kernel", e); return ST_DATA_MISSING; }
@@ -2217,8 +2327,8 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
 // Kroupa slopes on the device / host) through the operator: the fold (interpolated when every model's slopes allow,
 // else exact), then the template GEMM into d_young / d_old (n x nspec each, contiguous: d_old = d_young + n nspec);
 // the mass and L_bol sums into the context's sums (n x 6).
-int run_ops_parts(Context &c, int n, const double *d_wz, const double *d_alpha, const double *h_alpha, int itesc,
-                  float *d_young, float *d_old, std::string &err) {
+int run_ops_parts(Context &c, int n, const double *d_wz, const double *d_alpha, const double *h_alpha, const double *h_sfh,
+                  int itesc, float *d_young, float *d_old, std::string &err) {
     SspOps &o = c.ops;
     cudaStream_t st = c.stream;
     cudaError_t e;
@@ -2238,7 +2348,7 @@ int run_ops_parts(Context &c, int n, const double *d_wz, const double *d_alpha, 
     c.ops_last_interp = interp;
     c.ops_launches = 1;                  // (the template GEMM)
     if (interp) {
-        if (int rc = run_ops_interp(c, n, d_wz, d_alpha, itesc, err)) return rc;
+        if (int rc = run_ops_interp(c, n, d_wz, d_alpha, h_sfh, itesc, err)) return rc;
     } else {
     c.ops_launches += 2;                 // the fold and its slab reduction
     OpsFoldArgs fa;
@@ -2381,7 +2491,7 @@ int ops_evaluate(Context &c, int imf_type, const double *imf_params, double *mas
     }
     cudaMemsetAsync(c.d_status.p, 0, sizeof(int), st);
     // every age young (itesc = nt): the spectra are the young sums
-    int rc = run_ops_parts(c, nt, c.d_wz.p, c.d_alpha.p, alpha.data(), nt, c.d_yo.p, c.d_yo.p + (size_t)nt * ns, err);
+    int rc = run_ops_parts(c, nt, c.d_wz.p, c.d_alpha.p, alpha.data(), nullptr, nt, c.d_yo.p, c.d_yo.p + (size_t)nt * ns, err);
     if (rc) return rc;
     std::vector<float> y((size_t)nt * ns);
     std::vector<double> sums((size_t)6 * nt);
