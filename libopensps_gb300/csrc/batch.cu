@@ -1023,7 +1023,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     WeightsArgs wa;
     wa.n_models = n; wa.nt = nt; wa.nz = nz; wa.kpad = kpad; wa.kmap = bop ? bop->kmap.p : nullptr;
     wa.wz = d_wz; wa.mass = c.d_mass.p; wa.llin = c.d_llin.p; wa.w_hi = c.d_whi.p; wa.w_lo = c.d_wlo.p;
-    wa.sums = c.d_sums.p;
+    // (device inputs: the sums go nowhere, no entry point returns them and dust emission and the AGN need host inputs)
+    wa.sums = io.dev_inputs ? nullptr : c.d_sums.p;
     wa.parts = (io.mass_young || io.mass_old || io.lbol_young || io.lbol_old) ? 1 : 0;
     wa.itesc = itesc;
     wa.grid = 0;
@@ -1093,7 +1094,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         auto run_range = [&](int off, int nk, bool marks) -> int {
             WeightsArgs w = wa;
             w.n_models = nk; w.wz = d_wz + (size_t)nt * nz * off; w.w_hi = c.d_whi.p + (size_t)kpad * off;
-            w.w_lo = c.d_wlo.p + (size_t)kpad * off; w.sums = c.d_sums.p + (size_t)6 * off;
+            w.w_lo = c.d_wlo.p + (size_t)kpad * off; if (w.sums) w.sums += (size_t)6 * off;
             if (w.mpar) w.mpar = c.d_mpar.p + (size_t)MODEL_PAR_FLOATS * off;
             // the operand (which does not read the model parameters unless it forms escaping-light columns) on its
             // own stream beside the model parameters, forked from the batch's stream and joined before the

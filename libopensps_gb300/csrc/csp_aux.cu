@@ -16,26 +16,29 @@ namespace sps {
 constexpr int WC_CTA_MODELS = 8192;
 
 // ---------------------------------------------------------------------------------------------- weights
-// The operand and, from the same FP64 weights, the FP64 sums of model_sums_zw (one warp per model, the sums in the
-// operand's column order; young ages by the column map's KMAP_YOUNG bit): the sums ride the FP64 pipe while the
-// conversion waits on memory, instead of a second pass over the weights bound by that pipe. Escaping-light columns
-// (KMAP_ION) carry the weight times the model's escaping fraction clamp(frac_obrun, 0, 1) (nebular_kernels step 2,
-// OpenSPS src/physics/opensps_csp_batch.f90:2726-2750, with fesc of batch_nebular_indices :1696) and join no sum.
+// The operand and, from the same FP64 weights, the FP64 sums of model_sums_zw (in the operand's column order; young
+// ages by the column map's KMAP_YOUNG bit): the sums ride the FP64 pipe while the conversion waits on memory, instead
+// of a second pass over the weights bound by that pipe. Escaping-light columns (KMAP_ION) carry the weight times the
+// model's escaping fraction clamp(frac_obrun, 0, 1) (nebular_kernels step 2, OpenSPS
+// src/physics/opensps_csp_batch.f90:2726-2750, with fesc of batch_nebular_indices :1696) and join no sum.
 //
 // WPM warps share a model: one on large batches (the warps of the batch fill the GPU), the CTA's eight on small ones,
 // where a lane that walked 42 columns alone took 50 us of dependent loads whatever the batch (with eight warps 6.3 us
 // at one model and 15 at 1000).
 constexpr int WC_THREADS = 256, WC_WARPS = WC_THREADS / 32;
 
-template <bool PARTS, int WPM>
+// NSUM sums: 0 for batches whose sums no call can read (device inputs), the operand alone. The sums' fused
+// multiply-adds hold a large batch on the FP64 pipe: 433 us at 65536 models with them, 235 us without (10.3 KB
+// of weights and 5 KB of operand a model: 4.4 TB/s); 80 and 47 us at 9001.
+template <int NSUM, int WPM>
 __global__ void __launch_bounds__(WC_THREADS) weights_convert_sums_kernel(WeightsArgs a) {
-    constexpr int NSUM = PARTS ? 6 : 2;   // mass, L_bol; then mass young, old, L_bol young, old
+    constexpr bool PARTS = NSUM == 6;     // mass, L_bol; then mass young, old, L_bol young, old
     const int m = (blockIdx.x * WC_WARPS + (threadIdx.x >> 5)) / WPM;
     const int lane = threadIdx.x & 31, part = (threadIdx.x >> 5) % WPM;
     if (m >= a.n_models) return;          // (WPM = WC_WARPS: the whole CTA)
     const double *w = a.wz + (size_t)m * a.nt * a.nz;
     __nv_bfloat16 *hi = a.w_hi + (size_t)m * a.kpad, *lo = a.w_lo + (size_t)m * a.kpad;
-    double s[NSUM];
+    double s[NSUM > 0 ? NSUM : 2];
 #pragma unroll
     for (int i = 0; i < NSUM; ++i) s[i] = 0.0;
     const float fesc = a.mpar ? fminf(fmaxf(__ldg(a.mpar + (size_t)m * MODEL_PAR_FLOATS + MP_FO), 0.f), 1.f) : 0.f;
@@ -49,7 +52,7 @@ __global__ void __launch_bounds__(WC_THREADS) weights_convert_sums_kernel(Weight
             wf = weight_to_f32(wv);
             if (code & KMAP_ION) {
                 wf *= fesc;
-            } else if (__double_as_longlong(wv) > 0x0010000000000000LL) {   // wv > DBL_MIN (and not negative)
+            } else if (NSUM > 0 && __double_as_longlong(wv) > 0x0010000000000000LL) {   // wv > DBL_MIN (and not negative)
                 const double mk = __ldg(a.mass + idx), lk = __ldg(a.llin + idx);
                 s[0] = fma(wv, mk, s[0]);
                 s[1] = fma(wv, lk, s[1]);
@@ -67,36 +70,39 @@ __global__ void __launch_bounds__(WC_THREADS) weights_convert_sums_kernel(Weight
     for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
         for (int i = 0; i < NSUM; ++i) s[i] += __shfl_xor_sync(0xffffffffu, s[i], off);
-    if constexpr (WPM > 1) {
+    if constexpr (NSUM == 0) {
+        return;
+    } else if constexpr (WPM > 1) {
         __shared__ double part_sums[WC_WARPS][NSUM];
         if (lane == 0)
 #pragma unroll
             for (int i = 0; i < NSUM; ++i) part_sums[part][i] = s[i];
         __syncthreads();
-        if (threadIdx.x < NSUM && a.sums) {
+        if (threadIdx.x < NSUM) {
             double v = 0.0;
 #pragma unroll
             for (int p = 0; p < WPM; ++p) v += part_sums[p][threadIdx.x];
             a.sums[(size_t)m * 6 + threadIdx.x] = v;
         }
-    } else if (lane == 0 && a.sums) {
+    } else if (lane == 0) {
         double *o = a.sums + (size_t)m * 6;
 #pragma unroll
         for (int i = 0; i < NSUM; ++i) o[i] = s[i];
     }
 }
 
-template <bool PARTS>
+template <int NSUM>
 static void launch_weights_convert_sums(const WeightsArgs &a, cudaStream_t st) {
     // a CTA per model up to the batch whose single warps would fill the SMs about once (152 x 8 CTAs of eight warps)
-    if (a.n_models <= WC_CTA_MODELS) weights_convert_sums_kernel<PARTS, WC_WARPS><<<a.n_models, WC_THREADS, 0, st>>>(a);
-    else weights_convert_sums_kernel<PARTS, 1><<<(a.n_models + WC_WARPS - 1) / WC_WARPS, WC_THREADS, 0, st>>>(a);
+    if (a.n_models <= WC_CTA_MODELS) weights_convert_sums_kernel<NSUM, WC_WARPS><<<a.n_models, WC_THREADS, 0, st>>>(a);
+    else weights_convert_sums_kernel<NSUM, 1><<<(a.n_models + WC_WARPS - 1) / WC_WARPS, WC_THREADS, 0, st>>>(a);
 }
 
 cudaError_t run_weights_convert_sums(const WeightsArgs &a, cudaStream_t st) {
     if (a.n_models <= 0) return cudaSuccess;
-    if (a.parts) launch_weights_convert_sums<true>(a, st);
-    else launch_weights_convert_sums<false>(a, st);
+    if (!a.sums) launch_weights_convert_sums<0>(a, st);
+    else if (a.parts) launch_weights_convert_sums<6>(a, st);
+    else launch_weights_convert_sums<2>(a, st);
     return cudaGetLastError();
 }
 

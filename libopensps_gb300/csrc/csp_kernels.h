@@ -138,7 +138,7 @@ struct WeightsArgs {
     const double *mass;     // nt x nz
     const double *llin;     // nt x nz: 10^log L_bol
     __nv_bfloat16 *w_hi, *w_lo;   // n_models x kpad
-    double *sums;           // n_models x 6: mass, lsum, mass_young, mass_old, lsum_young, lsum_old
+    double *sums;           // n_models x 6: mass, lsum, mass_young, mass_old, lsum_young, lsum_old; null: not formed
     int parts;              // also the young and old sums
     int itesc;              // ages t < itesc (0-based) are young
     int grid;               // blocks of the FP64 sums kernel (0: one warp per model)

@@ -35,3 +35,22 @@ def test_batch_sizes(setup, n, birth_cloud):
     assert rel_err_spec(got["spec"][pick], ref["spec"]) <= 1e-4
     assert np.nanmax(np.abs(got["mags"][pick] - ref["mags"])) <= 1e-3
     assert np.max(np.abs(got["mass"][pick] / ref["mass"] - 1.0)) <= 1e-12
+
+
+@pytest.mark.parametrize("n", [1, 33, 8192, 8193])
+@pytest.mark.parametrize("fesc", [0.0, 0.4])
+def test_device_inputs(setup, n, fesc):
+    """Device inputs form the weight operand without the sums: the magnitudes of the same batch from host inputs, to
+    FP32 rounding (1e-4 mag)."""
+    import torch
+    from libopensps_gb300 import workloads
+    ctx, _ = setup
+    wz, params = config3_inputs(n, seed=n)
+    if fesc:
+        params = dict(params, frac_obrun=np.full(n, fesc))
+    want = ctx.csp_batch(params, ssp_weights_z=wz, spec=False)
+    d_wz = torch.from_numpy(wz).cuda()
+    d_par = torch.from_numpy(workloads.device_param_table(params, n)).cuda()
+    d_mags = torch.empty((n, ctx.nbands), dtype=torch.float64, device="cuda")
+    ctx.batch_device(n, d_par.data_ptr(), d_wz.data_ptr(), d_mags.data_ptr(), sync=True)
+    np.testing.assert_allclose(d_mags.cpu().numpy(), want["mags"], rtol=0, atol=1e-4)
