@@ -16,11 +16,18 @@
 // 9 warps of 16 rows at 92), warp 16 issues the band matrix's TMA and the MMAs.
 // Two stages with mbarriers: a builder warp signals its rows of stage s on full_a[s] and goes on to the next stage as
 // soon as the MMAs that read that buffer have completed (empty[s], a tcgen05 commit), so that the warps do not wait
-// for one another between stages.
+// for one another between stages. The band matrix comes up to three blocks ahead in slots of its own.
+// The pixel blocks split over the CTAs of a cluster (band_gemm_ksplit); each leaves its partial fluxes in its shared
+// memory, and the CTAs read one another's to form the magnitudes, a share of the rows each, in split order: no scratch
+// in memory and no second kernel.
+// Bound by the builders' instructions (a warp's 8 rows of a block take 300: 46 of the 62 us at 9001 models are left
+// without any load). 20001 models: 111 us, 144 unsplit, when 5 SMs had two of the 157 tiles; 1000 models: 18 us
+// against 22 and a second kernel; 65536: 277, as before.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cuda_bf16.h>
 #include <cfloat>
+#include <cmath>
 #include <cstdint>
 #include "sm103_ptx.cuh"
 #include "csp_kernels.h"
@@ -34,10 +41,19 @@ constexpr int BG_BUILD_THREADS = BG_BUILD_WARPS * 32;
 constexpr int BG_MMA_WARP = BG_BUILD_WARPS;             // TMA of the band matrix and the MMAs
 constexpr int BG_THREADS = BG_BUILD_THREADS + 32;
 constexpr int BG_A_BYTES = BG_M * BG_K * 2;   // 16 KB
+constexpr int BG_AHEAD = 1;                             // row pairs whose loads are in flight while one is converted
+constexpr int BG_MAX_SPLIT = 16, BG_MIN_BLOCKS = 4, BG_SETUP = 3, BG_FEW_TILES = 32;   // (band_gemm_ksplit)
 
 struct BandGemmSmem {
     static int b_bytes(int npad) { return npad * BG_K * 2; }
-    static int total(int npad) { return 2 * (2 * BG_A_BYTES + 2 * b_bytes(npad)) + 256 + 1024; }
+    static int total(int npad, int slots) { return 4 * BG_A_BYTES + slots * 2 * b_bytes(npad) + 256 + 1024; }
+    // Band-matrix slots: three, unless a second CTA fits the SM with two only, or not even one CTA with three.
+    static int slots(int npad) {
+        constexpr int SM_BYTES = 232448, OTHER = 1024 + 6144;   // (per CTA: the system's, and the static arrays)
+        if (2 * (total(npad, 3) + OTHER) <= SM_BYTES) return 3;
+        if (2 * (total(npad, 2) + OTHER) <= SM_BYTES) return 2;
+        return total(npad, 3) + OTHER <= SM_BYTES ? 3 : 2;
+    }
 };
 
 // 2^x by the SFU
@@ -62,13 +78,15 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int npad = a.npad;
     const int b_bytes = npad * BG_K * 2;
-    const int stage_bytes = 2 * BG_A_BYTES + 2 * b_bytes;
-    uint64_t *bars = reinterpret_cast<uint64_t *>(smem + 2 * stage_bytes);
-    uint64_t *full_a = bars;         // [2] the builder warps' rows of a stage (8 arrivals)
-    uint64_t *full_b = bars + 2;     // [2] the band matrix's TMA of a stage
-    uint64_t *empty = bars + 4;      // [2] the MMAs that read a stage have completed
-    uint64_t *bar_done = bars + 6;   // every MMA has completed
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 7);
+    constexpr int stage_bytes = 2 * BG_A_BYTES;      // two stages of the A operand (hi, lo), then the B slots (hi, lo)
+    uint8_t *bslots = smem + 2 * stage_bytes;
+    const int nb = a.slots;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(bslots + nb * 2 * b_bytes);
+    uint64_t *full_a = bars;         // [2] the builder warps' rows of a stage (16 arrivals)
+    uint64_t *empty = bars + 2;      // [2] the MMAs that read a stage have completed
+    uint64_t *full_b = bars + 4;     // [3] the band matrix's TMA of a slot
+    uint64_t *bar_done = bars + 7;   // every MMA has completed
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 8);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * BG_M;
     // this CTA's pixel blocks: split blockIdx.y of gridDim.y
@@ -78,13 +96,16 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
     int *status = a.status;
     const uint32_t tcols = npad <= 32 ? 32 : (npad <= 64 ? 64 : (npad <= 128 ? 128 : 256));
     __shared__ float4 zsm[BG_M];     // the observed-frame shift of the CTA's models (w = 2: no model in this row)
-    __shared__ int2 rsh[BG_M];       // per row: the rest-frame offset d (observed pixel j reads j - d, j - d + 1) and
-                                     // the last first-pixel j of a lane whose five rest pixels j - d .. j - d + 4 and
-                                     // four observed ones lie inside the grid (the interior case: d <= j <= that;
-                                     // a row without a model has none)
+    // per row, for the interior case: observed pixel j reads rest pixels j - d and j - d + 1; a lane's five, of its
+    // four observed pixels, lie in the two aligned float4 that begin at rest pixel p = j - d - mis (mis: the row's
+    // place in a float4, the same for every lane, whose first pixels differ by multiples of four). x = d + mis,
+    // y = the largest p whose eight rest pixels and four observed ones lie inside the grid (interior: p <= y, as
+    // unsigned), z = 4 x the row's offset from the CTA's first model's + mis, w = t; a row without a model has none
+    __shared__ int4 rsh[BG_M];
 
     if (tid == 0) {
-        for (int s = 0; s < 2; ++s) { mbar_init(&full_a[s], BG_BUILD_WARPS); mbar_init(&full_b[s], 1); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 2; ++s) { mbar_init(&full_a[s], BG_BUILD_WARPS); mbar_init(&empty[s], 1); }
+        for (int s = 0; s < 3; ++s) mbar_init(&full_b[s], 1);
         mbar_init(bar_done, 1);
         fence_mbar_init();
         tma_prefetch_desc(&tm_c_hi);
@@ -97,7 +118,11 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
         // the interior interpolation's first rest pixel: n0 + 1 below the observed one unless the shift is whole
         const int kind = zs.w == 1.f ? 1 : (zs.w == 0.f ? 0 : 2);
         const int d = kind == 1 ? __float_as_int(zs.x) + (zs.y > 0.f ? 1 : 0) : 0;
-        rsh[i] = make_int2(d, kind == 2 ? -1 : min(a.nspec - 5 + d, a.nspec - 4));
+        const float *row = a.spec + (size_t)(m0 + i) * a.ld_spec;
+        const int mis = (int)((((long long)(reinterpret_cast<uintptr_t>(row) >> 2)) + a.j0 - d) & 3);
+        const int last = min(a.nspec - 8, a.nspec - 4 - (d + mis));
+        rsh[i] = kind == 2 || last < 0 ? make_int4(1 << 30, 0, 0, 0)
+                                       : make_int4(d + mis, last, 4 * i * a.ld_spec + mis, __float_as_int(kind == 1 ? zs.y : 0.f));
     }
     tc_fence_before();
     __syncthreads();
@@ -108,22 +133,26 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
         // ---------------------------------------------------------------- band matrix TMA and MMAs (one thread)
         if (lane == 0) {
             const uint32_t idesc = idesc_bf16_f32(BG_M, npad);
-            int last_fill[2] = {-1, -1};      // parity of the last TMA issued into each stage, -1: none
+            // block li's band matrix in slot li mod nb, nb blocks ahead of its MMAs (issued when the block's A operand
+            // was asked for, its latency was a third of the time of each block)
+            auto fetch = [&](int li, int slot) {
+                uint8_t *bs = bslots + slot * 2 * b_bytes;
+                mbar_arrive_expect_tx(&full_b[slot], 2 * b_bytes);
+                tma_load_2d(bs, &tm_c_hi, (kb0 + li) * BG_K, 0, &full_b[slot]);
+                tma_load_2d(bs + b_bytes, &tm_c_lo, (kb0 + li) * BG_K, 0, &full_b[slot]);
+            };
+            int fetched = 0;                              // blocks whose copies were issued
+            for (; fetched < min(nb, nst); ++fetched) fetch(fetched, fetched);
             bool ok = true;
-            for (int li = 0; li < nst && ok; ++li) {
-                const int s = li & 1, kb = kb0 + li;
-                uint8_t *st = smem + s * stage_bytes;
-                // the stage's B buffer is free once the MMAs of stage li - 2 have completed
-                if (li >= 2 && !mbar_wait(&empty[s], ((li - 2) >> 1) & 1, status, ERR_TIMEOUT_BAND)) { ok = false; break; }
-                mbar_arrive_expect_tx(&full_b[s], 2 * b_bytes);
-                tma_load_2d(st + 2 * BG_A_BYTES, &tm_c_hi, kb * BG_K, 0, &full_b[s]);
-                tma_load_2d(st + 2 * BG_A_BYTES + b_bytes, &tm_c_lo, kb * BG_K, 0, &full_b[s]);
-                last_fill[s] = (li >> 1) & 1;
+            int slot = 0, bpar = 0, done = 0;             // done: blocks whose copies have landed
+            for (int li = 0; li < nst; ++li) {
+                const int s = li & 1;
                 if (!mbar_wait(&full_a[s], (li >> 1) & 1, status, ERR_TIMEOUT_BAND) ||
-                    !mbar_wait(&full_b[s], (li >> 1) & 1, status, ERR_TIMEOUT_BAND)) { ok = false; break; }
+                    !mbar_wait(&full_b[slot], bpar, status, ERR_TIMEOUT_BAND)) { ok = false; break; }
+                ++done;
                 tc_fence_after();
-                const uint32_t sa = smem_u32(st);
-                const uint32_t ahi = sa, alo = sa + BG_A_BYTES, bhi = sa + 2 * BG_A_BYTES, blo = bhi + b_bytes;
+                const uint32_t ahi = smem_u32(smem + s * stage_bytes), alo = ahi + BG_A_BYTES;
+                const uint32_t bhi = smem_u32(bslots + slot * 2 * b_bytes), blo = bhi + b_bytes;
 #pragma unroll
                 for (int k = 0; k < BG_K / 16; ++k) {
                     const uint32_t o = k * 32;
@@ -132,50 +161,72 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
                     mma_bf16(tmem, sw128_desc(alo + o), sw128_desc(bhi + o), idesc, 1u);
                 }
                 mma_commit(&empty[s]);
+                // the slot of block li - 1 is free once its MMAs have completed: the block nb after it
+                if (li >= 1 && fetched < nst) {
+                    if (!mbar_wait(&empty[s ^ 1], ((li - 1) >> 1) & 1, status, ERR_TIMEOUT_BAND)) { ok = false; break; }
+                    fetch(fetched, slot == 0 ? nb - 1 : slot - 1);
+                    ++fetched;
+                }
+                if (++slot == nb) { slot = 0; bpar ^= 1; }
             }
-            // every MMA issued completes on bar_done (the epilogue's wait, and the TMEM's release below); the copies
-            // still in flight land before the CTA may exit
+            // every MMA issued completes on bar_done (the epilogue's wait, and the TMEM's release below), after the
+            // copies still in flight have landed
+            for (; done < fetched; ++done) {              // (none unless a wait gave up)
+                mbar_wait(&full_b[done % nb], (uint32_t)(done / nb) & 1u, status, ERR_TIMEOUT_BAND, false);
+            }
             mma_commit(bar_done);
-            for (int s = 0; s < 2; ++s)
-                if (last_fill[s] >= 0) mbar_wait(&full_b[s], (uint32_t)last_fill[s], status, ERR_TIMEOUT_BAND, false);
             if (!ok) mbar_wait(bar_done, 0, status, ERR_TIMEOUT_BAND, false);
         }
     } else {
         // ---------------------------------------------------------------- A operand builders (warps 0..15)
-        const float dl2 = (float)(a.dlnl * 1.4426950408889634);   // grid step in log2 units
-        const float inv_em1 = (float)(1.0 / expm1(a.dlnl));
+        const float dl2 = a.dl2, inv_em1 = a.inv_em1;
         // each warp builds 8 model rows, two at a time: lane l takes row parity l / 16 and pixels 4 (l % 16) ..
         // 4 (l % 16) + 3 of the stage
         const int q = lane & 15, hr = lane >> 4;
+        const int row0 = warp * 8 + hr;
+        // an interior row pair's loads are two aligned float4 a lane (five scalar loads touched each line five times:
+        // L1 at 75 % of its peak, now 27), and BG_AHEAD pairs are in flight while one is converted, across the stages
+        // (none ahead: 85 us at 9001 models; one: 62; two or three: 64 to 66)
+        float4 va[4], vb[4];
+        const float *rows = a.spec + (size_t)m0 * a.ld_spec;
+        auto interior = [&](int li, int i) {                 // (of a lane's pixels of block li in its row of pair i)
+            const int2 rs = *reinterpret_cast<const int2 *>(&rsh[row0 + 2 * i]);
+            return (unsigned)(a.j0 + (kb0 + li) * BG_K + 4 * q - rs.x) <= (unsigned)rs.y;
+        };
+        // (the zeros: without them the old values stay live through the condition, and spill)
+        auto load = [&](int li, int i) {
+            va[i] = vb[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (li < nst && interior(li, i)) {
+                const int4 rs = rsh[row0 + 2 * i];
+                const float4 *sp = reinterpret_cast<const float4 *>(rows + ((rs.z >> 2) + a.j0 + (kb0 + li) * BG_K + 4 * q - rs.x));
+                va[i] = __ldg(sp);
+                vb[i] = __ldg(sp + 1);
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < BG_AHEAD; ++i) load(0, i);
         for (int li = 0; li < nst; ++li) {
             const int s = li & 1, kb = kb0 + li;
             uint8_t *st = smem + s * stage_bytes;
+            const int j = a.j0 + kb * BG_K + 4 * q;          // first observed pixel of this lane
             // the stage's A buffer is free once the MMAs of stage li - 2 have completed
             if (li >= 2 && !mbar_wait(&empty[s], ((li - 2) >> 1) & 1, status, ERR_TIMEOUT_BAND)) break;
-            const int j = a.j0 + kb * BG_K + 4 * q;          // first observed pixel of this lane
-            // the loads of all 4 row pairs first (rows whose 5 rest pixels lie inside the grid: the interior case),
-            // then the arithmetic
-            float sv[4][5];
-            bool inner[4];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                const int r = warp * 8 + 2 * i + hr;
-                const int2 rs = rsh[r];
-                inner[i] = j >= rs.x && j <= rs.y;
-                const float *sp = a.spec + (size_t)(m0 + r) * a.ld_spec + (j - rs.x);
-#pragma unroll
-                for (int u = 0; u < 5; ++u) sv[i][u] = inner[i] ? __ldg(sp + u) : 0.f;
-            }
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int r = warp * 8 + 2 * i + hr;
+                load(li + (i + BG_AHEAD) / 4, (i + BG_AHEAD) % 4);
+                const int r = row0 + 2 * i;
                 float f[4];
-                if (inner[i]) {
+                if (interior(li, i)) {
                     // v = s(c) + t (s(c + 1) - s(c)), t = 0 for whole shifts and the rest frame (v = s(c) exactly
                     // for finite spectra); NaN -> 0 and negatives -> 0 in one fmaxf
-                    const float t = zsm[r].y;
+                    const int2 rs = *reinterpret_cast<const int2 *>(&rsh[r].z);
+                    const float t = __int_as_float(rs.y);
+                    const bool m1 = rs.x & 1, m2 = rs.x & 2;
+                    const float w0 = m2 ? va[i].z : va[i].x, w1 = m2 ? va[i].w : va[i].y, w2 = m2 ? vb[i].x : va[i].z,
+                                w3 = m2 ? vb[i].y : va[i].w, w4 = m2 ? vb[i].z : vb[i].x, w5 = m2 ? vb[i].w : vb[i].y;
+                    const float sv[5] = {m1 ? w1 : w0, m1 ? w2 : w1, m1 ? w3 : w2, m1 ? w4 : w3, m1 ? w5 : w4};
 #pragma unroll
-                    for (int u = 0; u < 4; ++u) f[u] = fmaxf(fmaf(t, sv[i][u + 1] - sv[i][u], sv[i][u]), 0.f);
+                    for (int u = 0; u < 4; ++u) f[u] = fmaxf(fmaf(t, sv[u + 1] - sv[u], sv[u]), 0.f);
                 } else {
                     // the general case: no model, pixels past the grid's end, or intervals outside the grid (they
                     // extrapolate from the first / last one, the reference's clamped find_interval: position
@@ -219,45 +270,46 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
         mbar_wait(bar_done, 0, status, ERR_TIMEOUT_BAND, false);
         tc_fence_after();
 
-        // epilogue (warps 0..7): warps w and w + 4 read lane quarter w % 4 (one model per thread), columns
-        // 32 (w / 4) + 64 i
+        // the CTA's fluxes from TMEM into shared memory, over the stages (no copy is in flight into them: bar_done came
+        // after the last): warps w and w + 4 read lane quarter w % 4 (one model per thread), columns 32 (w / 4) + 64 i
         if (warp < 8 && *(volatile int *)status == 0) {
-            const int q = warp & 3;
-            const int r = q * 32 + lane, m = m0 + r;
-            const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+            const int r = (warp & 3) * 32 + lane;
+            const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+            float *dst = reinterpret_cast<float *>(smem) + r * (npad + 1);   // (odd pitch: a column without conflicts)
             for (int c0 = (warp >> 2) * 32; c0 < npad; c0 += 64) {
                 float v[32];
                 tmem_ld32(trow + c0, v);
-                if (split) {
-                    // the split's partial fluxes (band_finish_kernel sums them and forms the magnitudes)
-                    if (m < a.n_models) {
-                        float *dst = a.fpart + ((size_t)blockIdx.y * a.n_models + m) * npad + c0;
 #pragma unroll
-                        for (int i = 0; i < 32; i += 4)   // (npad is a multiple of 16)
-                            if (c0 + i < npad)
-                                *reinterpret_cast<float4 *>(dst + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-                    }
-                    continue;
-                }
-                if (m < a.n_models) {
-#pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const int b = c0 + i;
-                        if (b < a.nbands) {
-                            const double f = (double)v[i];
-                            if (a.fband) a.fband[(size_t)m * a.nbands + b] = f;
-                            if (a.mags) {
-                                double mg = __longlong_as_double(0x7ff8000000000000LL);
-                                if (a.do_band == nullptr || a.do_band[b] != 0)
-                                    mg = band_mag(v[i], a.zp, a.dist[m]);
-                                a.mags[(size_t)m * a.nbands + b] = mg;
-                            }
-                        }
-                    }
-                }
+                for (int i = 0; i < 32; ++i)
+                    if (c0 + i < npad) dst[c0 + i] = v[i];
             }
         }
     }
+    // the magnitudes: the cluster's CTAs share the tile's rows, each summing its rows' partial fluxes in split order
+    __syncwarp();
+    if (split) cluster_sync();
+    else __syncthreads();
+    if (*(volatile int *)status == 0) {
+        const int ks = (int)gridDim.y, r0 = BG_M * (int)blockIdx.y / ks, r1 = BG_M * ((int)blockIdx.y + 1) / ks;
+        const int tot = (min(r1, a.n_models - m0) - r0) * a.nbands;
+        for (int i = tid; i < tot; i += BG_THREADS) {
+            const int r = r0 + i / a.nbands, b = i % a.nbands, m = m0 + r;
+            const float *src = reinterpret_cast<const float *>(smem) + r * (npad + 1) + b;
+            float v = 0.f;
+            if (split)
+                for (int k = 0; k < ks; ++k) v += ld_cluster_f32(cluster_addr(src, (uint32_t)k));
+            else
+                v = *src;
+            if (a.fband) a.fband[(size_t)m * a.nbands + b] = (double)v;
+            if (a.mags) {
+                double mg = __longlong_as_double(0x7ff8000000000000LL);
+                if (a.do_band == nullptr || a.do_band[b] != 0) mg = band_mag(v, a.zp, a.dist[m]);
+                a.mags[(size_t)m * a.nbands + b] = mg;
+            }
+        }
+    }
+    __syncwarp();
+    if (split) cluster_sync();   // (no CTA leaves while another reads its fluxes)
     tc_fence_before();
     __syncthreads();
     if (warp == 0) {
@@ -268,27 +320,21 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
 
 int band_gemm_npad(int nbands) { return (nbands + 15) / 16 * 16 < 32 ? 32 : (nbands + 15) / 16 * 16; }
 
-// The split partial fluxes summed in split order, then the fluxes and magnitudes as the GEMM's epilogue forms them.
-__global__ void band_finish_kernel(BandGemmArgs a) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)a.n_models * a.nbands) return;
-    const int m = (int)(i / a.nbands), b = (int)(i % a.nbands);
-    float v = 0.f;
-    for (int s = 0; s < a.ksplit; ++s) v += a.fpart[((size_t)s * a.n_models + m) * a.npad + b];
-    if (a.fband) a.fband[i] = (double)v;
-    if (a.mags) {
-        double mg = __longlong_as_double(0x7ff8000000000000LL);
-        if (a.do_band == nullptr || a.do_band[b] != 0) mg = band_mag(v, a.zp, a.dist[m]);
-        a.mags[i] = mg;
-    }
-}
-
-// Splits of the pixel blocks when the batch's 128-model tiles give fewer than two CTAs per SM (two fit on an SM):
-// up to two CTAs per SM, each split keeping at least 4 pixel blocks.
+// Splits of the pixel blocks over a cluster's CTAs. Few tiles (at most 4096 models): up to two CTAs per SM. More: the
+// split with the least work on the busiest SM, its CTAs times a CTA's pixel blocks and the BG_SETUP blocks' time that
+// every CTA takes besides (its setup, the pipeline's fill, its magnitudes; with 12 blocks for it 20001 models take 127
+// us, unsplit 144, against 111 with 3).
 int band_gemm_ksplit(int n_models, int nkb, int num_sms) {
     const int tiles = (n_models + BG_M - 1) / BG_M;
-    if (tiles >= 2 * num_sms || nkb < 8) return 1;
-    return std::max(1, std::min((2 * num_sms + tiles - 1) / tiles, nkb / 4));
+    const int most = std::max(1, std::min(nkb / BG_MIN_BLOCKS, BG_MAX_SPLIT));
+    if (tiles <= BG_FEW_TILES) return std::min((2 * num_sms + tiles - 1) / tiles, most);
+    int best = 1;
+    long long best_cost = 0;
+    for (int ks = 1; ks <= std::min(most, 8); ++ks) {
+        const long long cost = (((long long)tiles * ks + num_sms - 1) / num_sms) * ((nkb + ks - 1) / ks + BG_SETUP);
+        if (ks == 1 || cost < best_cost) { best = ks; best_cost = cost; }
+    }
+    return best;
 }
 
 // Loads the band GEMM's module on the current device (CUDA loads modules lazily, on first use), so that a later
@@ -296,7 +342,6 @@ int band_gemm_ksplit(int n_models, int nkb, int num_sms) {
 cudaError_t band_gemm_load() {
     cudaFuncAttributes fa;
     cudaError_t e = cudaFuncGetAttributes(&fa, band_gemm_kernel);
-    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, band_finish_kernel);
     return e;
 }
 
@@ -304,17 +349,28 @@ cudaError_t run_band_gemm(const BandGemmArgs &a_in, const CUtensorMap &tm_hi, co
                           cudaStream_t st) {
     if (a_in.n_models <= 0 || a_in.nkb <= 0) return cudaSuccess;
     BandGemmArgs a = a_in;
-    a.ksplit = a.fpart ? band_gemm_ksplit(a.n_models, a.nkb, a.num_sms) : 1;
-    if (a.ksplit > 1 && (size_t)a.ksplit * a.n_models * a.npad > a.fpart_cap) a.ksplit = 1;
-    const int smem = BandGemmSmem::total(a.npad);
+    a.slots = BandGemmSmem::slots(a.npad);
+    a.dl2 = (float)(a.dlnl * 1.4426950408889634);
+    a.inv_em1 = (float)(1.0 / std::expm1(a.dlnl));   // (on the host: each CTA's warps took 7 us for it on the FP64 pipe)
+    const int ks = band_gemm_ksplit(a.n_models, a.nkb, a.num_sms);
+    const int smem = BandGemmSmem::total(a.npad, a.slots);
     cudaError_t e = cudaFuncSetAttribute(band_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    const dim3 grid((a.n_models + BG_M - 1) / BG_M, a.ksplit);
-    band_gemm_kernel<<<grid, BG_THREADS, smem, st>>>(tm_hi, tm_lo, a);
-    if ((e = cudaGetLastError()) != cudaSuccess || a.ksplit == 1) return e;
-    const size_t tot = (size_t)a.n_models * a.nbands;
-    band_finish_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, st>>>(a);
-    return cudaGetLastError();
+    if (ks > 8 && (e = cudaFuncSetAttribute(band_gemm_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) != cudaSuccess)
+        return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((a.n_models + BG_M - 1) / BG_M, ks);
+    cfg.blockDim = dim3(BG_THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = (unsigned)ks;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = ks > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, band_gemm_kernel, tm_hi, tm_lo, a);
 }
 
 }  // namespace sps

@@ -1042,12 +1042,6 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         ba.mags = (io.dev_inputs ? io.mags : c.d_mags.p) + (size_t)nb * off;
         ba.status = c.d_status.p;
         ba.num_sms = c.num_sms;
-        const int ks = band_gemm_ksplit(nk, c.band_nkb, c.num_sms);
-        if (ks > 1) {
-            const size_t cap = (size_t)ks * nk * c.band_npad;
-            if (c.d_bpart.reserve(cap) == cudaSuccess) { ba.fpart = c.d_bpart.p; ba.fpart_cap = cap; }
-            else cudaGetLastError();
-        }
         return run_band_gemm(ba, c.tm_cb_hi, c.tm_cb_lo, st);
     };
     // the per-model epilogue from the young and old sums (the operator's path, and any batch with dust emission)
@@ -1255,7 +1249,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         }
         if (want_mags && !fp64) {
             if ((e = bands(0, n)) != cudaSuccess) { err = cuda_msg("band kernel", e); return ST_DATA_MISSING; }
-            launches += band_gemm_ksplit(n, c.band_nkb, c.num_sms) > 1 ? 2 : 1;
+            ++launches;
         }
         prof_mark(c, 4);
         // the FP64 mass and L_bol sums (the operator's fold forms its own)

@@ -313,7 +313,6 @@ struct Context {
     DevBuf<double2> d_ix_const;  // and each model's 1 / T and c2
     DevBuf<double> d_ix_dln;     // and d ln T / d alpha (the reverse pass)
     DevBuf<DustEmModel> d_dem;   // the batch's dust emission cells (one per model)
-    DevBuf<float> d_bpart;       // the band GEMM's partial fluxes when it splits the pixels (few models)
     DevBuf<float> d_vbar;        // reverse pass with operators: 2n x ntpad template cotangents (young, old)
     DevBuf<__nv_bfloat16> d_vbh, d_vbl;   // and as bf16 hi / lo (the interpolated reverse fold's A operand)
     DevBuf<float> d_xbar;        // the interpolated reverse fold: a chunk's cotangents of the operand X

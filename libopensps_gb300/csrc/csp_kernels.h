@@ -160,15 +160,12 @@ struct BandGemmArgs {
     double *fband;          // n_models x nbands (may be null)
     double *mags;           // n_models x nbands (may be null)
     int *status;
-    // with few models, the pixels split over CTAs: partial band fluxes (ksplit x n_models x npad floats, at most
-    // fpart_cap) summed by a second kernel that forms the magnitudes (fpart null: no split)
-    float *fpart = nullptr;
-    size_t fpart_cap = 0;
-    int num_sms = 148;
-    int ksplit = 1;         // set by run_band_gemm
+    int num_sms = 152;
+    float dl2 = 0.f, inv_em1 = 0.f;   // set by run_band_gemm: the grid step in log2 units, 1 / (e^dlnl - 1)
+    int slots = 2;                    // set by run_band_gemm: shared-memory slots of the band matrix
 };
 int band_gemm_npad(int nbands);
-// The pixel splits run_band_gemm takes for n_models (1: none).
+// The CTAs of a cluster that run_band_gemm splits the pixels over for n_models (1: none).
 int band_gemm_ksplit(int n_models, int nkb, int num_sms);
 cudaError_t run_band_gemm(const BandGemmArgs &a, const CUtensorMap &tm_hi, const CUtensorMap &tm_lo,
                           cudaStream_t st);

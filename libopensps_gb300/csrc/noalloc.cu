@@ -141,6 +141,7 @@ int run_mags_noalloc(Context &c, int n, const float *d_spec, const double *d_zre
             ba.dlnl = c.dlnl; ba.dist = dist;
             ba.zp = 48.60 + 2.5 * std::log10(3.828e33 / (4.0 * M_PI * std::pow(10.0 * (648000.0 / M_PI) * 1.495978707e13, 2)));
             ba.do_band = do_band; ba.fband = nullptr; ba.mags = d_mags; ba.status = status;
+            ba.num_sms = c.num_sms;
             e = run_band_gemm(ba, c.tm_cb_hi, c.tm_cb_lo, st);
         }
         if (e == cudaSuccess && sync) {
