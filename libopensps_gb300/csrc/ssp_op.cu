@@ -1390,17 +1390,28 @@ __device__ __forceinline__ float2 dl07_shape2(const float *tab, int ns, int nq, 
 // memory: the attenuated sum through the IGM with the AGN added (the AGN does not depend on the energy balance), and
 // with dust emission the escaping template through the IGM and the frequency-trapezoid sums of the absorbed and
 // escaping light (before the IGM), reduced over the block; the emission scaled by their ratio then joins the
-// spectrum. Pass 2 smooths from shared memory. Each thread issues the young and old loads of EPI_U pixel pairs before
-// it uses them.
-constexpr int EPI_U = 4;
+// spectrum. Pass 2 smooths from shared memory. Each thread issues the young and old loads of EpiCfg::U pixel pairs
+// before it uses them.
+//
+// DEM: batches with dust emission or AGN (226 us at 4001 models: the eight template rows of a model's cell, 192 KB of L2
+// reads a model, and 80 registers; four CTAs per SM, other unrollings and 512 threads took 243 to 290). Without them the
+// kernel takes 32 registers, its warps fill the SM and hide the loads: 24 us at 1024 models (3.0 TB/s of 49 MB of sums
+// and 25 MB of spectra), 42 when they shared the other's registers and 24 warps per SM.
+// THREADS: 512 where the models leave SMs idle (9 us at 100 models, 15 with 256 threads before), else 256.
+template <bool DEM, int THREADS>
+struct EpiCfg {
+    static constexpr int U = DEM ? 4 : 1, CTAS = DEM ? 3 : 2048 / THREADS;
+};
+constexpr int EPI_WIDE_MODELS = 304;       // (run_parts_epilogue: two models of 512 threads per SM)
 
 // TAB: the models' curves differ and are tabulated (dust_type other than 0): each from the pixel's T0..T3 and the
 // model's scalars (a separate instantiation keeps the others' registers as they were)
-template <bool TAB>
-__global__ void __launch_bounds__(256, 3) parts_epilogue_kernel(PartsEpilogueArgs a) {
+template <bool TAB, bool DEM, int THREADS>
+__global__ void __launch_bounds__(THREADS, EpiCfg<DEM, THREADS>::CTAS) parts_epilogue_kernel(PartsEpilogueArgs a) {
+    constexpr int EPI_U = EpiCfg<DEM, THREADS>::U;
     extern __shared__ float tsm[];         // nspec: the spectrum; with dust emission a second nspec: its emission
     float *esm = tsm + a.nspec;
-    __shared__ float red[2][8];
+    __shared__ float red[2][THREADS / 32];
     const int ns = a.nspec, m = blockIdx.x;
     const float *mp = a.mpar + (size_t)MODEL_PAR_FLOATS * m;
     const float *yv = a.young + (size_t)m * ns, *ov = a.old + (size_t)m * ns;
@@ -1410,9 +1421,9 @@ __global__ void __launch_bounds__(256, 3) parts_epilogue_kernel(PartsEpilogueArg
     const int jmax = __float_as_int(mp[MP_IGM_JMAX]);
     const int igm_top = mp[MP_IGM_ON] != 0.f ? a.jtop : 0;     // pixels below carry the IGM
     DustEmModel dm{};
-    if (a.dem) dm = a.dem[m];
-    const bool emis = a.dem != nullptr && dm.on != 0;
-    const bool agn = a.dem != nullptr && dm.agn != 0;
+    if (DEM && a.dem) dm = a.dem[m];
+    const bool emis = DEM && a.dem != nullptr && dm.on != 0;
+    const bool agn = DEM && a.dem != nullptr && dm.agn != 0;
     // the AGN's luminosity: fagn times the model's L_bol (add_agn_batch :4342-4433, the value the batch outputs;
     // 1 when it is not above SAFE_FLOOR, as log10 L_bol is then 0)
     float lagn = 0.f;
@@ -1469,7 +1480,7 @@ __global__ void __launch_bounds__(256, 3) parts_epilogue_kernel(PartsEpilogueArg
         if (agn) tot = fmaf(lagn * fmaf(dm.wta, t1 - t0, t0), td, tot);
         return tot;
     };
-    const int bd = (int)blockDim.x;
+    constexpr int bd = THREADS;
     const bool pairs = (ns & 1) == 0;
     if (pairs) {
         const int np2 = ns >> 1;
@@ -1888,16 +1899,22 @@ cudaError_t run_nebular_continuum(const NebContArgs &a, int ngroups, cudaStream_
     return cudaSuccess;
 }
 
+template <bool TAB, bool DEM, int THREADS>
+static cudaError_t launch_parts_epilogue(const PartsEpilogueArgs &a, cudaStream_t st) {
+    const size_t smem = sizeof(float) * (size_t)a.nspec * (DEM ? 2 : 1);
+    const cudaError_t e = cudaFuncSetAttribute(parts_epilogue_kernel<TAB, DEM, THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    parts_epilogue_kernel<TAB, DEM, THREADS><<<a.n, THREADS, smem, st>>>(a);
+    return cudaGetLastError();
+}
+
 cudaError_t run_parts_epilogue(const PartsEpilogueArgs &a, cudaStream_t st) {
     if (a.n <= 0) return cudaSuccess;
-    const size_t smem = sizeof(float) * (size_t)a.nspec * (a.dem ? 2 : 1);
     const bool tab = !a.uniform_index && a.tab_curve;
-    cudaError_t e = tab ? cudaFuncSetAttribute(parts_epilogue_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                        : cudaFuncSetAttribute(parts_epilogue_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    if (tab) parts_epilogue_kernel<true><<<a.n, 256, smem, st>>>(a);
-    else parts_epilogue_kernel<false><<<a.n, 256, smem, st>>>(a);
-    return cudaGetLastError();
+    if (a.dem) return tab ? launch_parts_epilogue<true, true, 256>(a, st) : launch_parts_epilogue<false, true, 256>(a, st);
+    if (a.n <= EPI_WIDE_MODELS)
+        return tab ? launch_parts_epilogue<true, false, 512>(a, st) : launch_parts_epilogue<false, false, 512>(a, st);
+    return tab ? launch_parts_epilogue<true, false, 256>(a, st) : launch_parts_epilogue<false, false, 256>(a, st);
 }
 
 // ---------------------------------------------------------------------------------------------- host side
