@@ -924,8 +924,8 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         transpose_bf16_kernel<<<grid, block, 0, s>>>(o.lib_hi.p, o.lib_thi.p, ns, o.ntpad, o.ntpad, ppad);
         transpose_bf16_kernel<<<grid, block, 0, s>>>(o.lib_lo.p, o.lib_tlo.p, ns, o.ntpad, o.ntpad, ppad);
         if ((e = cudaGetLastError()) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&o.tm_lib_thi, o.lib_thi.p, ppad, o.ntpad, gemm_bk(), gemm_bn())) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&o.tm_lib_tlo, o.lib_tlo.p, ppad, o.ntpad, gemm_bk(), gemm_bn())) != cudaSuccess) {
+            (e = encode_tmap_2d_bf16(&o.tm_lib_thi, o.lib_thi.p, ppad, o.ntpad, gemm_bk(), gemm_box_n())) != cudaSuccess ||
+            (e = encode_tmap_2d_bf16(&o.tm_lib_tlo, o.lib_tlo.p, ppad, o.ntpad, gemm_bk(), gemm_box_n())) != cudaSuccess) {
             err = msg("transposed library", e);
             o.lib_thi.release(); o.lib_tlo.release();
             return ST_DATA_MISSING;
@@ -954,8 +954,8 @@ int run_grad_batch(Context &c, const BatchIO &io_in, const double *mags_bar, con
         transpose_bf16_kernel<<<grid, block, 0, s>>>(bop->hi.p, bop->thi.p, ns, kpad, ld_basis, ppad);
         transpose_bf16_kernel<<<grid, block, 0, s>>>(bop->lo.p, bop->tlo.p, ns, kpad, ld_basis, ppad);
         if ((e = cudaGetLastError()) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&bop->tm_thi, bop->thi.p, ppad, kpad, gemm_bk(), gemm_bn())) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&bop->tm_tlo, bop->tlo.p, ppad, kpad, gemm_bk(), gemm_bn())) != cudaSuccess) {
+            (e = encode_tmap_2d_bf16(&bop->tm_thi, bop->thi.p, ppad, kpad, gemm_bk(), gemm_box_n())) != cudaSuccess ||
+            (e = encode_tmap_2d_bf16(&bop->tm_tlo, bop->tlo.p, ppad, kpad, gemm_bk(), gemm_box_n())) != cudaSuccess) {
             err = msg("transposed basis", e);
             bop->thi.release(); bop->tlo.release();
             return ST_DATA_MISSING;

@@ -205,6 +205,7 @@ struct GemmPlan {
 int gemm_bk();
 int gemm_bm();
 int gemm_bn();
+int gemm_box_n();   // rows of the B tensor maps' boxes for three products (one product: gemm_bn)
 int gemm_choose_ksplit(int tiles_mn, int nkb, int num_sms);
 cudaError_t run_gemm_bf16x3(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st);   // three products (hi / lo)
 cudaError_t run_gemm_bf16(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st);     // one product (hi only)

@@ -18,9 +18,10 @@
 // and in B's at age age_cols + z slab2 / 2), so that the other slabs' columns, all zero in A, are neither read nor
 // multiplied.
 //
-// Tile 128 x 256 x 64, persistent CTAs over tiles; warp 0 = TMA producer, warp 1 = MMA issuer and TMEM owner,
-// warps 2..5 = epilogue (one accumulator row per thread); TMEM double-buffered. Two smem stages of 96 KB (split) or
-// four of 48 KB (plain). Every mbarrier wait is bounded (status word, no hang).
+// Tile 128 x 256 x 64, or 256 x 256 x 64 by a CTA pair (three products, gemm_pairs), persistent CTAs over tiles; warp 0 =
+// TMA producer, warp 1 = MMA issuer and TMEM owner,
+// warps 2..5 = epilogue (one accumulator row per thread); TMEM double-buffered. Two smem stages of 96 KB (split), three
+// of 64 KB (split, a CTA of a pair) or four of 48 KB (plain). Every mbarrier wait is bounded (status word, no hang).
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 #include <algorithm>
@@ -33,22 +34,22 @@ namespace sps {
 constexpr int G_BM = 128, G_BN = 256, G_BK = 64;
 constexpr int G_A_BYTES = G_BM * G_BK * 2, G_B_BYTES = G_BN * G_BK * 2;
 constexpr int G_THREADS = 6 * 32;
-constexpr uint32_t G_IDESC = idesc_bf16_f32(G_BM, G_BN);
 
-template <int NPROD>
+template <int NPROD, int CTAS = 1>
 struct GemmCfg {
-    static constexpr int STAGE_BYTES = NPROD == 3 ? 2 * G_A_BYTES + 2 * G_B_BYTES : G_A_BYTES + G_B_BYTES;
-    static constexpr int STAGES = NPROD == 3 ? 2 : 4;
+    static constexpr int B_BYTES = G_B_BYTES / CTAS;     // a pair's CTA holds half of the tile's B rows
+    static constexpr int STAGE_BYTES = NPROD == 3 ? 2 * G_A_BYTES + 2 * B_BYTES : G_A_BYTES + B_BYTES;
+    static constexpr int STAGES = NPROD == 3 ? (CTAS == 2 ? 3 : 2) : 4;
     static constexpr int SMEM = STAGES * STAGE_BYTES + 256 + 1024;
 };
 
 struct GemmTile {
     int g, s, m0, n0, rows, z;   // rows: of D from m0 that this tile stores (an end); z: its slab (GemmArgs::mtab)
 };
-template <bool SLABS>
-__device__ __forceinline__ GemmTile gemm_tile(const GemmArgs &g, int tile, int mt_n, int nt_n) {
+template <bool SLABS, int CTAS>
+__device__ __forceinline__ GemmTile gemm_tile(const GemmArgs &g, int tile, int mt_n, int nt_n, int rank) {
     GemmTile t;
-    t.m0 = (tile % mt_n) * G_BM;
+    t.m0 = (tile % mt_n * CTAS + rank) * G_BM;
     t.rows = g.M;
     t.z = 0;
     if constexpr (SLABS) {
@@ -63,12 +64,13 @@ __device__ __forceinline__ GemmTile gemm_tile(const GemmArgs &g, int tile, int m
     return t;
 }
 
-template <int NPROD, bool SLABS>
+// CTAS = 2: a CTA pair takes 256 x 256, half of A's and of B's rows in each CTA's shared memory (CTA 0 issues the MMAs).
+template <int NPROD, bool SLABS, int CTAS>
 __global__ void __launch_bounds__(G_THREADS, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_constant__ CUtensorMap tm_a_lo,
                  const __grid_constant__ CUtensorMap tm_b_hi, const __grid_constant__ CUtensorMap tm_b_lo,
                  GemmArgs g) {
-    using C = GemmCfg<NPROD>;
+    using C = GemmCfg<NPROD, CTAS>;
     constexpr int NS = C::STAGES;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -77,7 +79,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
     uint64_t *mma_done = bars + 2 * NS + 4;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 2 * NS + 5);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int mt_n = SLABS ? g.n_mtiles : (g.M + G_BM - 1) / G_BM, nt_n = (g.N + G_BN - 1) / G_BN;
+    const int rank = CTAS == 2 ? (int)cluster_ctarank() : 0, tile0 = blockIdx.x / CTAS, tile_step = gridDim.x / CTAS;
+    const int mt_n = SLABS ? g.n_mtiles : (g.M + CTAS * G_BM - 1) / (CTAS * G_BM), nt_n = (g.N + G_BN - 1) / G_BN;
     const int n_tiles = mt_n * nt_n * g.ksplit * g.groups;
     // (SLABS: K blocks of an age's two slabs, kpa of them, the last with ktail columns)
     const int kpa = SLABS ? (g.slab2 + G_BK - 1) / G_BK : 1, nkb = SLABS ? g.ages * kpa : (g.K + G_BK - 1) / G_BK;
@@ -86,13 +89,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < NS; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], 4); }
+        for (int b = 0; b < 2; ++b) { mbar_init(&tfull[b], 1); mbar_init(&tempty[b], CTAS * 4); }
         mbar_init(mma_done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    if (warp == 1) {
+        if constexpr (CTAS == 2) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+        else { tmem_alloc(tmem_slot, 512); tmem_relinquish(); }
+    }
     tc_fence_before();
     __syncthreads();
+    if constexpr (CTAS == 2) cluster_sync();      // (the barriers of both CTAs are ready)
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
 
@@ -102,15 +109,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
             int last_fill[NS];
             for (int i = 0; i < NS; ++i) last_fill[i] = -1;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
+            for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+                const GemmTile t = gemm_tile<SLABS, CTAS>(g, tile, mt_n, nt_n, rank);
                 const int arow = (int)(t.g * g.a_grp) + t.m0;
-                const int brow = (int)(t.g * g.b_grp) + g.b_row0 + t.n0;
+                const int brow = (int)(t.g * g.b_grp) + g.b_row0 + t.n0 + rank * (G_BN / CTAS);
                 const int kb0 = t.s * nkb / g.ksplit, kb1 = (t.s + 1) * nkb / g.ksplit;
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(&empty[s], ph ^ 1u, status, ERR_TIMEOUT_PRODUCER)) { ok = false; break; }
                     uint8_t *st = smem + s * C::STAGE_BYTES;
-                    mbar_arrive_expect_tx(&full[s], C::STAGE_BYTES);
+                    // (a pair's copies, of both CTAs, complete on CTA 0's barrier, whose phase its producer arms for all)
+                    if (rank == 0) mbar_arrive_expect_tx(&full[s], CTAS * C::STAGE_BYTES);
                     if (NPROD == 3) {
                         int xa = kb * G_BK, xb = xa;
                         if constexpr (SLABS) {
@@ -118,10 +126,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                             xa = age * g.slab2 + off;
                             xb = age * g.age_cols + t.z * (g.slab2 / 2) + off;
                         }
-                        tma_load_2d(st, &tm_a_hi, xa, arow, &full[s]);
-                        tma_load_2d(st + G_A_BYTES, &tm_a_lo, xa, arow, &full[s]);
-                        tma_load_2d(st + 2 * G_A_BYTES, &tm_b_hi, xb, brow, &full[s]);
-                        tma_load_2d(st + 2 * G_A_BYTES + G_B_BYTES, &tm_b_lo, xb, brow, &full[s]);
+                        uint8_t *b_hi = st + 2 * G_A_BYTES, *b_lo = b_hi + C::B_BYTES;
+                        if constexpr (CTAS == 2) {
+                            const uint32_t bar = cluster_addr(&full[s], 0);
+                            tma_load_2d_pair(st, &tm_a_hi, xa, arow, bar);
+                            tma_load_2d_pair(st + G_A_BYTES, &tm_a_lo, xa, arow, bar);
+                            tma_load_2d_pair(b_hi, &tm_b_hi, xb, brow, bar);
+                            tma_load_2d_pair(b_lo, &tm_b_lo, xb, brow, bar);
+                        } else {                  // (B's box is 128 rows, a pair's half)
+                            tma_load_2d(st, &tm_a_hi, xa, arow, &full[s]);
+                            tma_load_2d(st + G_A_BYTES, &tm_a_lo, xa, arow, &full[s]);
+                            tma_load_2d(b_hi, &tm_b_hi, xb, brow, &full[s]);
+                            tma_load_2d(b_hi + G_B_BYTES / 2, &tm_b_hi, xb, brow + G_BN / 2, &full[s]);
+                            tma_load_2d(b_lo, &tm_b_lo, xb, brow, &full[s]);
+                            tma_load_2d(b_lo + G_B_BYTES / 2, &tm_b_lo, xb, brow + G_BN / 2, &full[s]);
+                        }
                     } else {
                         tma_load_2d(st, &tm_a_hi, kb * G_BK, arow, &full[s]);
                         tma_load_2d(st + G_A_BYTES, &tm_b_hi, kb * G_BK, brow, &full[s]);
@@ -131,20 +150,28 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                 }
             }
             for (int i = 0; i < NS; ++i)
-                if (last_fill[i] >= 0) mbar_wait(&full[i], (uint32_t)last_fill[i], status, ERR_TIMEOUT_PRODUCER, false);
+                if (last_fill[i] >= 0 && rank == 0) mbar_wait(&full[i], (uint32_t)last_fill[i], status, ERR_TIMEOUT_PRODUCER, false);
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        if (lane == 0 && rank == 0) {
+            auto mma = [](uint32_t d, uint64_t da, uint64_t db, uint32_t id, uint32_t accum) {
+                if constexpr (CTAS == 2) mma_bf16_pair(d, da, db, id, accum);
+                else mma_bf16(d, da, db, id, accum);
+            };
+            auto commit = [](uint64_t *bar) {
+                if constexpr (CTAS == 2) mma_commit_pair(bar);
+                else mma_commit(bar);
+            };
             int s = 0; uint32_t ph = 0;
             int acc = 0; uint32_t aph = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
+            for (int tile = tile0; tile < n_tiles && ok; tile += tile_step) {
+                const GemmTile t = gemm_tile<SLABS, CTAS>(g, tile, mt_n, nt_n, rank);
                 const int kb0 = t.s * nkb / g.ksplit, kb1 = (t.s + 1) * nkb / g.ksplit;
                 if (!mbar_wait(&tempty[acc], aph ^ 1u, status, ERR_TIMEOUT_MMA)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d = tmem_base + acc * G_BN;
-                const uint32_t idesc = (NPROD == 1 && g.f16) ? idesc_f16_f32(G_BM, G_BN) : G_IDESC;
+                const uint32_t idesc = (NPROD == 1 && g.f16) ? idesc_f16_f32(G_BM, G_BN) : idesc_bf16_f32(CTAS * G_BM, G_BN);
                 for (int kb = kb0; kb < kb1; ++kb) {
                     if (!mbar_wait(&full[s], ph, status, ERR_TIMEOUT_MMA)) { ok = false; break; }
                     tc_fence_after();
@@ -155,30 +182,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
                         const uint32_t off = k * 32;
                         const uint32_t first = (kb > kb0 || k > 0) ? 1u : 0u;
                         if (NPROD == 3) {
-                            const uint32_t a_hi = sa, a_lo = sa + G_A_BYTES, b_hi = sa + 2 * G_A_BYTES, b_lo = b_hi + G_B_BYTES;
-                            mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_hi + off), G_IDESC, first);
-                            mma_bf16(d, sw128_desc(a_hi + off), sw128_desc(b_lo + off), G_IDESC, 1u);
-                            mma_bf16(d, sw128_desc(a_lo + off), sw128_desc(b_hi + off), G_IDESC, 1u);
+                            const uint32_t a_hi = sa, a_lo = sa + G_A_BYTES, b_hi = sa + 2 * G_A_BYTES, b_lo = b_hi + C::B_BYTES;
+                            mma(d, sw128_desc(a_hi + off), sw128_desc(b_hi + off), idesc, first);
+                            mma(d, sw128_desc(a_hi + off), sw128_desc(b_lo + off), idesc, 1u);
+                            mma(d, sw128_desc(a_lo + off), sw128_desc(b_hi + off), idesc, 1u);
                         } else {
-                            mma_bf16(d, sw128_desc(sa + off), sw128_desc(sa + G_A_BYTES + off), idesc, first);
+                            mma(d, sw128_desc(sa + off), sw128_desc(sa + G_A_BYTES + off), idesc, first);
                         }
                     }
-                    mma_commit(&empty[s]);
+                    commit(&empty[s]);
                     if (++s == NS) { s = 0; ph ^= 1u; }
                 }
                 if (!ok) break;
-                mma_commit(&tfull[acc]);
+                commit(&tfull[acc]);
                 if (++acc == 2) { acc = 0; aph ^= 1u; }
             }
-            mma_commit(mma_done);
+            commit(mma_done);
             mbar_wait(mma_done, 0, status, ERR_TIMEOUT_MMA, false);
         }
     } else {
         // epilogue: warp w reads TMEM lanes 32 (w % 4) .. : one row of D per thread
         const int q = warp & 3;
         int acc = 0; uint32_t aph = 0;
-        for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-            const GemmTile t = gemm_tile<SLABS>(g, tile, mt_n, nt_n);
+        for (int tile = tile0; tile < n_tiles; tile += tile_step) {
+            const GemmTile t = gemm_tile<SLABS, CTAS>(g, tile, mt_n, nt_n, rank);
             mbar_wait(&tfull[acc], aph, status, ERR_TIMEOUT_EPILOGUE);
             named_bar_sync(1, 128);
             if (*(volatile int *)status != 0) break;
@@ -205,21 +232,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
             }
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tempty[acc]);
+            if (lane == 0) {
+                if constexpr (CTAS == 2) mbar_arrive_cluster(cluster_addr(&tempty[acc], 0));
+                else mbar_arrive(&tempty[acc]);
+            }
             if (++acc == 2) { acc = 0; aph ^= 1u; }
         }
     }
     tc_fence_before();
     __syncthreads();
+    // (a pair's CTAs leave together: CTA 0's MMAs read CTA 1's shared memory, CTA 1 arrives on CTA 0's barriers)
+    if constexpr (CTAS == 2) cluster_sync();
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, 512);
+        if constexpr (CTAS == 2) tmem_dealloc_pair(tmem_base, 512);
+        else tmem_dealloc(tmem_base, 512);
     }
 }
 
 int gemm_bk() { return G_BK; }
 int gemm_bm() { return G_BM; }
 int gemm_bn() { return G_BN; }
+int gemm_box_n() { return G_BN / 2; }
+
+static long long gemm_tiles(long long rows, int tile) { return (rows + tile - 1) / tile; }
 
 // K splits for a GEMM of tiles_mn output tiles over nkb K blocks: the fewest giving at least two waves over the SMs
 // with the last wave at least 85% full (else the fullest last wave), each split keeping 8 or more K blocks.
@@ -236,23 +272,45 @@ int gemm_choose_ksplit(int tiles_mn, int nkb, int num_sms) {
     return best;
 }
 
-template <int NPROD, bool SLABS = false>
+template <int NPROD, bool SLABS = false, int CTAS = 1>
 static cudaError_t launch_gemm(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) {
     if (g.M <= 0 || g.N <= 0 || g.K <= 0 || g.groups <= 0 || g.ksplit <= 0) return cudaSuccess;
     const int nkb = SLABS ? g.ages * ((g.slab2 + G_BK - 1) / G_BK) : (g.K + G_BK - 1) / G_BK;
     if (g.ksplit > nkb) return cudaErrorInvalidValue;          // every split needs a K block
     if ((reinterpret_cast<uintptr_t>(g.D) & 15) != 0) return cudaErrorInvalidValue;
-    using C = GemmCfg<NPROD>;
-    cudaError_t e = cudaFuncSetAttribute(gemm_bf16_kernel<NPROD, SLABS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    using C = GemmCfg<NPROD, CTAS>;
+    auto kern = gemm_bf16_kernel<NPROD, SLABS, CTAS>;
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) return e;
-    const long long tiles = (long long)(SLABS ? g.n_mtiles : (g.M + G_BM - 1) / G_BM) * ((g.N + G_BN - 1) / G_BN) * g.ksplit * g.groups;
-    const int grid = tiles < pl.num_sms ? (int)tiles : pl.num_sms;
-    gemm_bf16_kernel<NPROD, SLABS><<<grid, G_THREADS, C::SMEM, st>>>(pl.tm_a_hi, pl.tm_a_lo, pl.tm_b_hi, pl.tm_b_lo, g);
-    return cudaGetLastError();
+    const long long tiles = (SLABS ? g.n_mtiles : gemm_tiles(g.M, CTAS * G_BM)) * gemm_tiles(g.N, G_BN) * g.ksplit * g.groups;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(CTAS * std::min<long long>(tiles, pl.num_sms / CTAS)));
+    cfg.blockDim = dim3(G_THREADS);
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = st;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = CTAS;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = CTAS > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, pl.tm_a_hi, pl.tm_a_lo, pl.tm_b_hi, pl.tm_b_lo, g);
+}
+
+// Pairs where their waves cost less: an MMA of 256 x 256 over two SMs takes 147 cycles against 200 for 128 x 256 in one
+// (each SM reads 8 KB of operands from shared memory instead of 12), but the pairs' tiles are coarser. Measured, one CTA
+// -> pairs: the operator's templates at 1024 models (2048 x 5994 x 2752) 152 -> 142 us (8.8 TB/s of operands from L2 to
+// shared memory), at 100 models 56 -> 49; the reverse pass's weights at 2000 models 38.5 -> 34.5 and 60 -> 52.
+static bool gemm_pairs(const GemmPlan &pl, const GemmArgs &g) {
+    const long long rest = gemm_tiles(g.N, G_BN) * g.ksplit * g.groups, pairs = std::max(pl.num_sms / 2, 1);
+    const long long one = (gemm_tiles(g.M, G_BM) * rest + pl.num_sms - 1) / pl.num_sms;
+    const long long two = (gemm_tiles(g.M, 2 * G_BM) * rest + pairs - 1) / pairs;
+    return pl.num_sms >= 2 && two * 147 < one * 200;
 }
 
 cudaError_t run_gemm_bf16x3(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) {
-    return g.mtab ? launch_gemm<3, true>(pl, g, st) : launch_gemm<3>(pl, g, st);
+    if (g.mtab) return launch_gemm<3, true>(pl, g, st);
+    return gemm_pairs(pl, g) ? launch_gemm<3, false, 2>(pl, g, st) : launch_gemm<3>(pl, g, st);
 }
 cudaError_t run_gemm_bf16(const GemmPlan &pl, const GemmArgs &g, cudaStream_t st) { return launch_gemm<1>(pl, g, st); }
 

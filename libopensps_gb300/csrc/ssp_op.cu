@@ -1300,8 +1300,8 @@ int run_ops_interp_reverse(Context &c, const OpsRevArgs &r, std::string &err) {
         if ((e = o.ibt_hi.reserve(ktot * o.ntpad)) != cudaSuccess || (e = o.ibt_lo.reserve(ktot * o.ntpad)) != cudaSuccess ||
             (e = run_transpose_bf16(o.ib_hi.p, o.ibt_hi.p, o.ntempl, ktot, ktot, o.ntpad, st)) != cudaSuccess ||
             (e = run_transpose_bf16(o.ib_lo.p, o.ibt_lo.p, o.ntempl, ktot, ktot, o.ntpad, st)) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&o.tm_ibt_hi, o.ibt_hi.p, o.ntpad, ktot, gemm_bk(), gemm_bn())) != cudaSuccess ||
-            (e = encode_tmap_2d_bf16(&o.tm_ibt_lo, o.ibt_lo.p, o.ntpad, ktot, gemm_bk(), gemm_bn())) != cudaSuccess) {
+            (e = encode_tmap_2d_bf16(&o.tm_ibt_hi, o.ibt_hi.p, o.ntpad, ktot, gemm_bk(), gemm_box_n())) != cudaSuccess ||
+            (e = encode_tmap_2d_bf16(&o.tm_ibt_lo, o.ibt_lo.p, o.ntpad, ktot, gemm_bk(), gemm_box_n())) != cudaSuccess) {
             err = cmsg("transposed operator basis", e);
             o.ibt_hi.release(); o.ibt_lo.release();
             return ST_DATA_MISSING;
@@ -2169,8 +2169,8 @@ int ops_build(Context &c, std::string &err) {
         (e = cudaMemcpy(o.ent_c.p, ent_c.data(), sizeof(float) * ent_c.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(o.lib_hi.p, lh.data(), 2 * lh.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
         (e = cudaMemcpy(o.lib_lo.p, ll.data(), 2 * ll.size(), cudaMemcpyHostToDevice)) != cudaSuccess ||
-        (e = encode_tmap_2d_bf16(&o.tm_lib_hi, o.lib_hi.p, ntpad, ns, gemm_bk(), gemm_bn())) != cudaSuccess ||
-        (e = encode_tmap_2d_bf16(&o.tm_lib_lo, o.lib_lo.p, ntpad, ns, gemm_bk(), gemm_bn())) != cudaSuccess) {
+        (e = encode_tmap_2d_bf16(&o.tm_lib_hi, o.lib_hi.p, ntpad, ns, gemm_bk(), gemm_box_n())) != cudaSuccess ||
+        (e = encode_tmap_2d_bf16(&o.tm_lib_lo, o.lib_lo.p, ntpad, ns, gemm_bk(), gemm_box_n())) != cudaSuccess) {
         err = cmsg("SSP operator upload", e);
         o.release();
         return ST_DATA_MISSING;
@@ -2311,8 +2311,8 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
             pl.num_sms = c.num_sms;
             if ((e = encode_tmap_2d_16s(&pl.tm_a_hi, c.d_ix_hi.p + a0, ka, rows, xld, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
                 (e = encode_tmap_2d_16s(&pl.tm_a_lo, c.d_ix_lo.p + a0, ka, rows, xld, gemm_bk(), gemm_bm(), false)) != cudaSuccess ||
-                (e = encode_tmap_2d_16s(&pl.tm_b_hi, o.ib_hi.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_bn(), false)) != cudaSuccess ||
-                (e = encode_tmap_2d_16s(&pl.tm_b_lo, o.ib_lo.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_bn(), false)) != cudaSuccess) {
+                (e = encode_tmap_2d_16s(&pl.tm_b_hi, o.ib_hi.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_box_n(), false)) != cudaSuccess ||
+                (e = encode_tmap_2d_16s(&pl.tm_b_lo, o.ib_lo.p + c0, K, o.ntempl, ktot, gemm_bk(), gemm_box_n(), false)) != cudaSuccess) {
                 err = cmsg("interpolated fold tensor map", e);
                 return ST_DATA_MISSING;
             }
