@@ -47,13 +47,14 @@ constexpr int BG_MAX_SPLIT = 16, BG_MIN_BLOCKS = 4, BG_SETUP = 3, BG_FEW_TILES =
 struct BandGemmSmem {
     static int b_bytes(int npad) { return npad * BG_K * 2; }
     static int total(int npad, int slots) { return 4 * BG_A_BYTES + slots * 2 * b_bytes(npad) + 256 + 1024; }
+    static constexpr int SM_BYTES = 232448, OTHER = 1024 + 6144;   // (OTHER per CTA: the system's, the static arrays)
     // Band-matrix slots: three, unless a second CTA fits the SM with two only, or not even one CTA with three.
     static int slots(int npad) {
-        constexpr int SM_BYTES = 232448, OTHER = 1024 + 6144;   // (per CTA: the system's, and the static arrays)
         if (2 * (total(npad, 3) + OTHER) <= SM_BYTES) return 3;
         if (2 * (total(npad, 2) + OTHER) <= SM_BYTES) return 2;
         return total(npad, 3) + OTHER <= SM_BYTES ? 3 : 2;
     }
+    static bool two_ctas(int npad) { return 2 * (total(npad, slots(npad)) + OTHER) <= SM_BYTES; }   // (per SM)
 };
 
 // 2^x by the SFU
@@ -324,9 +325,10 @@ int band_gemm_npad(int nbands) { return (nbands + 15) / 16 * 16 < 32 ? 32 : (nba
 // split with the least work on the busiest SM, its CTAs times a CTA's pixel blocks and the BG_SETUP blocks' time that
 // every CTA takes besides (its setup, the pipeline's fill, its magnitudes; with 12 blocks for it 20001 models take 127
 // us, unsplit 144, against 111 with 3).
-int band_gemm_ksplit(int n_models, int nkb, int num_sms) {
+static int band_gemm_ksplit(int n_models, int nkb, int npad, int num_sms) {
     const int tiles = (n_models + BG_M - 1) / BG_M;
-    const int most = std::max(1, std::min(nkb / BG_MIN_BLOCKS, BG_MAX_SPLIT));
+    // (clusters beyond the portable eight only where two of their CTAs share an SM)
+    const int most = std::max(1, std::min(nkb / BG_MIN_BLOCKS, BandGemmSmem::two_ctas(npad) ? BG_MAX_SPLIT : 8));
     if (tiles <= BG_FEW_TILES) return std::min((2 * num_sms + tiles - 1) / tiles, most);
     int best = 1;
     long long best_cost = 0;
@@ -352,7 +354,7 @@ cudaError_t run_band_gemm(const BandGemmArgs &a_in, const CUtensorMap &tm_hi, co
     a.slots = BandGemmSmem::slots(a.npad);
     a.dl2 = (float)(a.dlnl * 1.4426950408889634);
     a.inv_em1 = (float)(1.0 / std::expm1(a.dlnl));   // (on the host: each CTA's warps took 7 us for it on the FP64 pipe)
-    const int ks = band_gemm_ksplit(a.n_models, a.nkb, a.num_sms);
+    const int ks = band_gemm_ksplit(a.n_models, a.nkb, a.npad, a.num_sms);
     const int smem = BandGemmSmem::total(a.npad, a.slots);
     cudaError_t e = cudaFuncSetAttribute(band_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;

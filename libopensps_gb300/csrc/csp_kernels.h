@@ -165,8 +165,6 @@ struct BandGemmArgs {
     int slots = 2;                    // set by run_band_gemm: shared-memory slots of the band matrix
 };
 int band_gemm_npad(int nbands);
-// The CTAs of a cluster that run_band_gemm splits the pixels over for n_models (1: none).
-int band_gemm_ksplit(int n_models, int nkb, int num_sms);
 cudaError_t run_band_gemm(const BandGemmArgs &a, const CUtensorMap &tm_hi, const CUtensorMap &tm_lo,
                           cudaStream_t st);
 // Loads the band GEMM's module on the current device (no launch).
