@@ -20,9 +20,9 @@
 // The pixel blocks split over the CTAs of a cluster (band_gemm_ksplit); each leaves its partial fluxes in its shared
 // memory, and the CTAs read one another's to form the magnitudes, a share of the rows each, in split order: no scratch
 // in memory and no second kernel.
-// Bound by the builders' instructions (a warp's 8 rows of a block take 300: 46 of the 62 us at 9001 models are left
-// without any load). 20001 models: 111 us, 144 unsplit, when 5 SMs had two of the 157 tiles; 1000 models: 18 us
-// against 22 and a second kernel; 65536: 277, as before.
+// Bound by the builders' instructions and their latencies (a warp's 8 rows of a block take 300; without any load three
+// quarters of the time are left). 20001 models: 111 us, 144 unsplit, when 5 SMs had two of the 157 tiles; 9001: 49 us
+// against 57 and a second kernel; 1000: 18 us against 15 and 5; 65536: 277, as before.
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cuda_bf16.h>
@@ -187,7 +187,7 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
         const int row0 = warp * 8 + hr;
         // an interior row pair's loads are two aligned float4 a lane (five scalar loads touched each line five times:
         // L1 at 75 % of its peak, now 27), and BG_AHEAD pairs are in flight while one is converted, across the stages
-        // (none ahead: 85 us at 9001 models; one: 62; two or three: 64 to 66)
+        // (split in two, none ahead: 85 us at 9001 models; one: 62; two or three: 64 to 66)
         float4 va[4], vb[4];
         const float *rows = a.spec + (size_t)m0 * a.ld_spec;
         auto interior = [&](int li, int i) {                 // (of a lane's pixels of block li in its row of pair i)
@@ -322,9 +322,10 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
 int band_gemm_npad(int nbands) { return (nbands + 15) / 16 * 16 < 32 ? 32 : (nbands + 15) / 16 * 16; }
 
 // Splits of the pixel blocks over a cluster's CTAs. Few tiles (at most 4096 models): up to two CTAs per SM. More: the
-// split with the least work on the busiest SM, its CTAs times a CTA's pixel blocks and the BG_SETUP blocks' time that
-// every CTA takes besides (its setup, the pipeline's fill, its magnitudes; with 12 blocks for it 20001 models take 127
-// us, unsplit 144, against 111 with 3).
+// split with the least time on the busiest SM, whose CTAs run two at a time: a pair takes 3.1 us a pixel block, a CTA
+// alone 2.3 (a builder warp's own latencies bound it, and two CTAs hide part of them), and every CTA takes BG_SETUP
+// blocks' time besides (its setup, the pipeline's fill, its magnitudes). Measured, us at splits
+// of 1 .. 6: 113, 64, 60, 49, 68, 67 at 9001 models; 145, 132, 111, 114, 110, 116 at 20001; 120 and 90 at 1 and 2 at 16384.
 static int band_gemm_ksplit(int n_models, int nkb, int npad, int num_sms) {
     const int tiles = (n_models + BG_M - 1) / BG_M;
     // (clusters beyond the portable eight only where two of their CTAs share an SM)
@@ -333,7 +334,8 @@ static int band_gemm_ksplit(int n_models, int nkb, int npad, int num_sms) {
     int best = 1;
     long long best_cost = 0;
     for (int ks = 1; ks <= std::min(most, 8); ++ks) {
-        const long long cost = (((long long)tiles * ks + num_sms - 1) / num_sms) * ((nkb + ks - 1) / ks + BG_SETUP);
+        const long long ctas = ((long long)tiles * ks + num_sms - 1) / num_sms;     // of the busiest SM
+        const long long cost = (ctas / 2 * 31 + ctas % 2 * 23) * ((nkb + ks - 1) / ks + BG_SETUP);
         if (ks == 1 || cost < best_cost) { best = ks; best_cost = cost; }
     }
     return best;
