@@ -116,62 +116,71 @@ __device__ __forceinline__ float scaled_to_f32(double x, int k) {
 }
 
 // ---------------------------------------------------------------------------------------------- per-model scalars
-// One thread per model, FP64 (igm_tau_z_terms_dz src/physics/opensps_cosmology.f90:511-522; smooth_sigma_adjoint's
+// FP64 (igm_tau_z_terms_dz src/physics/opensps_cosmology.f90:511-522; smooth_sigma_adjoint's
 // d C / d sigma = C (x^2 - <x^2>) / (sigma_beta^3 c); backward_observed_frame's d t / dz; distance_term_dz).
-__global__ void __launch_bounds__(256) adjoint_prep_kernel(AdjointPrepArgs a) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
+// A CTA's three warps take the same 32 models, a role each (the IGM's factors, the smoothing taps, the observed frame and
+// the distance), so that the chains run beside one another and few models spread over many SMs' FP64 pipes: 7 us at 2000
+// models, 25 by one thread per model in CTAs of 256 (14 in CTAs of 32).
+__global__ void __launch_bounds__(96) adjoint_prep_kernel(AdjointPrepArgs a) {
+    const int m = blockIdx.x * 32 + (threadIdx.x & 31), role = threadIdx.x >> 5;
     if (m >= a.n_models) return;
     const double *pr = a.par + (size_t)PAR_DEVICE * m;
     const float *mp = a.mpar + (size_t)MODEL_PAR_FLOATS * m;
-    float blk[AP_FLOATS];
-#pragma unroll
-    for (int i = 0; i < AP_FLOATS; ++i) blk[i] = 0.f;
+    float *o = a.apar + (size_t)AP_FLOATS * m;
     const double z = pr[PF_ZRED];
-    if (mp[MP_IGM_ON] != 0.f) {
-        // (1 + z)^p with p = 3.46 for k = 0 and 2, 1.68 for the others
-        const double l1z = log1p(z), inv = 1.0 / (1.0 + z), b0 = exp(3.46 * l1z), b1 = exp(1.68 * l1z);
-        const float f0 = (float)b0, f1 = (float)b1, g0 = (float)(3.46 * b0 * inv), g1 = (float)(1.68 * b1 * inv);
+    if (role == 0) {
+        float f0 = 0.f, f1 = 0.f, g0 = 0.f, g1 = 0.f;
+        if (mp[MP_IGM_ON] != 0.f) {
+            // (1 + z)^p with p = 3.46 for k = 0 and 2, 1.68 for the others
+            const double l1z = log1p(z), inv = 1.0 / (1.0 + z), b0 = exp(3.46 * l1z), b1 = exp(1.68 * l1z);
+            f0 = (float)b0; f1 = (float)b1; g0 = (float)(3.46 * b0 * inv); g1 = (float)(1.68 * b1 * inv);
+        }
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
-            blk[AP_B + k] = (k == 0 || k == 2) ? f0 : f1;
-            blk[AP_DB + k] = (k == 0 || k == 2) ? g0 : g1;
+            o[AP_B + k] = (k == 0 || k == 2) ? f0 : f1;
+            o[AP_DB + k] = (k == 0 || k == 2) ? g0 : g1;
         }
-    }
-    const int R = __float_as_int(mp[MP_SMOOTH_R]);
-    const double sig = pr[PF_SIGMA_SMOOTH];
-    if (R >= 0 && sig > 0.0) {
-        const double sb = sig / ADJ_C_KMS;
-        const double inv = 1.0 / (sb * sb * sb * ADJ_C_KMS);
-        double av[9], mean = 0.0;
+    } else if (role == 1) {
+        float tap[AP_KOBS - AP_DTAP];
 #pragma unroll
-        for (int d = -4; d <= 4; ++d) {
-            const int j = min(max(a.sm_lo + d, 0), a.nspec - 1);
-            const double dd = a.lnlam[a.sm_lo] - a.lnlam[j];
-            av[d + 4] = dd * dd * inv;
-            mean += (double)mp[MP_TAPS + d + 4] * av[d + 4];
+        for (int d = 0; d < AP_KOBS - AP_DTAP; ++d) tap[d] = 0.f;
+        const int R = __float_as_int(mp[MP_SMOOTH_R]);
+        const double sig = pr[PF_SIGMA_SMOOTH];
+        if (R >= 0 && sig > 0.0) {
+            const double sb = sig / ADJ_C_KMS;
+            const double inv = 1.0 / (sb * sb * sb * ADJ_C_KMS);
+            double av[9], mean = 0.0;
+#pragma unroll
+            for (int d = -4; d <= 4; ++d) {
+                const int j = min(max(a.sm_lo + d, 0), a.nspec - 1);
+                const double dd = a.lnlam[a.sm_lo] - a.lnlam[j];
+                av[d + 4] = dd * dd * inv;
+                mean += (double)mp[MP_TAPS + d + 4] * av[d + 4];
+            }
+#pragma unroll
+            for (int d = 0; d < 9; ++d) tap[d] = (float)((double)mp[MP_TAPS + d] * (av[d] - mean));
         }
 #pragma unroll
-        for (int d = 0; d < 9; ++d) blk[AP_DTAP + d] = (float)((double)mp[MP_TAPS + d] * (av[d] - mean));
-    }
-    double kobs = 0.0, ddist = 0.0;
-    const float4 zi = a.zinfo[m];
-    if (zi.w == 1.f) {
-        // t = (lambda_j / (1 + z) - lambda_il) / (lambda_(il+1) - lambda_il): dt/dz = -lambda_j / ((1 + z)^2 dlambda_il),
-        // lambda_j / dlambda_il = e^((j - il) dlnl) / (e^dlnl - 1), j - il = nsh on the grid's interior
-        const int nsh = __float_as_int(zi.x) + ((zi.y > 0.f) ? 1 : 0);
-        const double opz = 1.0 + z;
-        kobs = -exp((double)nsh * a.dlnl) / (opz * opz * a.em1);
-        const int idx = cosmology_interval(a.zt, z);
-        const double slope = (a.dl[idx + 1] - a.dl[idx]) / (a.zt[idx + 1] - a.zt[idx]);
-        const double dm = a.dl[idx] + slope * (z - a.zt[idx]);
-        if (dm == dm && dm > SAFE_FLOOR) ddist = 5.0 / log(10.0) * slope / dm - 2.5 / (log(10.0) * opz);
-    }
-    float *o = a.apar + (size_t)AP_FLOATS * m;
+        for (int d = 0; d < AP_KOBS - AP_DTAP; ++d) o[AP_DTAP + d] = tap[d];
+    } else {
+        double kobs = 0.0, ddist = 0.0;
+        const float4 zi = a.zinfo[m];
+        if (zi.w == 1.f) {
+            // t = (lambda_j / (1 + z) - lambda_il) / (lambda_(il+1) - lambda_il): dt/dz = -lambda_j / ((1 + z)^2 dlambda_il),
+            // lambda_j / dlambda_il = e^((j - il) dlnl) / (e^dlnl - 1), j - il = nsh on the grid's interior
+            const int nsh = __float_as_int(zi.x) + ((zi.y > 0.f) ? 1 : 0);
+            const double opz = 1.0 + z;
+            kobs = -exp((double)nsh * a.dlnl) / (opz * opz * a.em1);
+            const int idx = cosmology_interval(a.zt, z);
+            const double slope = (a.dl[idx + 1] - a.dl[idx]) / (a.zt[idx + 1] - a.zt[idx]);
+            const double dm = a.dl[idx] + slope * (z - a.zt[idx]);
+            if (dm == dm && dm > SAFE_FLOOR) ddist = 5.0 / log(10.0) * slope / dm - 2.5 / (log(10.0) * opz);
+        }
+        reinterpret_cast<double *>(o)[AP_KOBS / 2] = kobs;
+        reinterpret_cast<double *>(o)[AP_DDIST / 2] = ddist;
 #pragma unroll
-    for (int i = 0; i < AP_FLOATS; i += 4)
-        reinterpret_cast<float4 *>(o)[i / 4] = make_float4(blk[i], blk[i + 1], blk[i + 2], blk[i + 3]);
-    reinterpret_cast<double *>(o)[AP_KOBS / 2] = kobs;
-    reinterpret_cast<double *>(o)[AP_DDIST / 2] = ddist;
+        for (int i = AP_DDIST + 2; i < AP_FLOATS; ++i) o[i] = 0.f;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------- the adjoint
@@ -845,7 +854,7 @@ __global__ void __launch_bounds__(256) ion_rev_kernel(IonRevArgs a) {
 
 cudaError_t run_adjoint(const AdjointPrepArgs &pa, const AdjointArgs &a, cudaStream_t st) {
     if (a.n_models <= 0) return cudaSuccess;
-    adjoint_prep_kernel<<<(pa.n_models + 255) / 256, 256, 0, st>>>(pa);
+    adjoint_prep_kernel<<<(pa.n_models + 31) / 32, 96, 0, st>>>(pa);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const int nj = a.j1 - a.j0 + 1;

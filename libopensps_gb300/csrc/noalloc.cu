@@ -53,7 +53,8 @@ struct ObsFrameArgs {
 // Per model: the observed-frame shift on the log-uniform grid and the distance term, as the batch's model-parameter
 // kernel forms them (compute_magnitudes_columns' observed_frame_z and distance_term,
 // src/spectra/opensps_batch_photometry.f90:784-903); thread 0 of block 0 also writes the band mask. Bound by the FP64
-// pipe: 12 us at 20001 models, 20 with the divisions, expm1 calls and the bisection observed_frame leaves out.
+// pipe: 9 us at 20001 models in CTAs of a warp, spread evenly over the SMs' pipes (12 in CTAs of 256; 20 with the
+// divisions, expm1 calls and the bisection observed_frame leaves out).
 __global__ void obs_frame_kernel(ObsFrameArgs a) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m == 0)
@@ -131,7 +132,7 @@ int run_mags_noalloc(Context &c, int n, const float *d_spec, const double *d_zre
         oa.zinfo = zinfo; oa.dist = dist; oa.do_band = do_band;
         e = cudaMemsetAsync(status, 0, sizeof(int), st);
         if (e == cudaSuccess) {
-            obs_frame_kernel<<<(n + 255) / 256, 256, 0, st>>>(oa);
+            obs_frame_kernel<<<(n + 31) / 32, 32, 0, st>>>(oa);
             e = cudaGetLastError();
         }
         if (e == cudaSuccess) {
