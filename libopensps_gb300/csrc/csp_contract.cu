@@ -445,8 +445,9 @@ static cudaError_t launch_contract(const ContractPlan &pl, const ContractArgs &a
 // 64 ..). CTA pairs (one accumulator): an MMA of 256 pixels by bn models over two SMs reads a CTA's share of both
 // operands from shared memory once, 8 KB at bn = 256 against 12 KB by one CTA, whose 12 KB at about 64 bytes a cycle
 // take 1.5 times the multiplications' 128 cycles; below 160 models the A operand's share is the bound either way. Two
-// accumulators (at most 128 models a tile, so that they fit TMEM twice) measured the same or slower in pairs (429 us at 9001 models against 450). The
-// widest tile is not always the cheapest: a batch may fill its last wave badly, or hold fewer models than a tile.
+// accumulators (at most 128 models a tile, so that they fit TMEM twice) run on single CTAs: pairs measured 450 us at 9001
+// models against 429. The widest tile is not always the cheapest: a batch may fill its last wave badly, or hold fewer
+// models than a tile.
 // Measured, one CTA per 256 (128) models and eight epilogue warps -> with the rule and sixteen: 38.7 -> 20 us at one
 // model, 80 -> 51 at 1000, 317 -> 239 at 9001, 1951 -> 1591 at 65536 (2.0 PFLOP/s executed). Every tile gives the same
 // bits: an output's products are summed in the same order.
@@ -477,8 +478,8 @@ int contract_bk() { return BK; }
 int contract_bm() { return BM; }
 
 cudaError_t run_contract(int nacc, const ContractPlan &pl, const ContractArgs &a, cudaStream_t st) {
-    if (a.ctas == 2) return nacc == 1 ? launch_contract<1, 2>(pl, a, st) : launch_contract<2, 2>(pl, a, st);
-    return nacc == 1 ? launch_contract<1, 1>(pl, a, st) : launch_contract<2, 1>(pl, a, st);
+    if (nacc == 2) return a.ctas == 1 ? launch_contract<2, 1>(pl, a, st) : cudaErrorInvalidValue;
+    return a.ctas == 2 ? launch_contract<1, 2>(pl, a, st) : launch_contract<1, 1>(pl, a, st);
 }
 
 }  // namespace sps

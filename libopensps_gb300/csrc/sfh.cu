@@ -1,5 +1,6 @@
-// SFH weights on the device, one thread per model in FP64 (OpenSPS batch_sfh_weights → sfh_weights_core,
-// src/physics/opensps_csp_batch.f90:1865-1917, src/physics/opensps_sfh.f90:1077-1212, compute_ssp_weights :97-257):
+// SFH weights on the device in FP64, the moments by a thread per interval limit, the rest by a warp per model (OpenSPS
+// batch_sfh_weights → sfh_weights_core, src/physics/opensps_csp_batch.f90:1865-1917,
+// src/physics/opensps_sfh.f90:1077-1212, compute_ssp_weights :97-257):
 // the mass formed against the hat kernel of each grid age for SFH types 0 (SSP), 1 (tau) and 4 (delayed tau), with
 // the constant and burst components, normalised to one solar mass formed, and 5 (Simha: the delayed tau up to the
 // truncation, then a linear ramp from its SFR there, the two normalised apart and mixed by the ramp's mass fraction).
