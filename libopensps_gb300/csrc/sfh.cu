@@ -443,7 +443,8 @@ __device__ __forceinline__ void zinterval(const double *lz, int nz, double x, in
 // The main component's moments (sfh 1, 4; the delayed tau of sfh 5, set up as sfh_weights_core sets it) at the limits
 // sfh_forward_kernel's intervals end at, one thread per (model, limit): the grid ages clamped to the model's window
 // [max(tq, 1 yr), max(tage, 1 yr)], then the window's start (the youngest edge's lower limit), nt + 1 per model; limits
-// that no interval of positive width ends at are left out. t10 = 10^(log age) from the host. After them one thread per
+// that no interval of positive width ends at are left out (by years, with a margin: sfh_forward_kernel decides by
+// log10 years, whose rounding may leave an interval that ends at tq, up to the oldest age's, a width). t10 = 10^(log age) from the host. After them one thread per
 // model for the SFR, which one lane of a warp per model would take as long for as 32.
 // Bound by the FP64 pipe: about 110 instructions per limit, 612 with the series term by term, pow and logarithms per
 // limit: 116 us at 4001 models, 454 before (sfh_forward_kernel 116, 526 before).
@@ -469,7 +470,7 @@ __global__ void __launch_bounds__(128) sfh_moments_kernel(SfhArgs a) {
     if (j == a.nt || tj <= tlo) {
         t = fmin(tlo, thi);
         lt = t == 1.0 ? 0.0 : log10(t);
-        need = j == a.nt || (j + 1 < a.nt && __ldg(a.t10 + j + 1) * (1.0 + 1e-9) > tlo);
+        need = j == a.nt || __ldg(a.t10 + min(j + 1, a.nt - 1)) * (1.0 + 1e-9) > tlo;
     } else if (tj >= thi) {
         t = thi;
         need = j == 0 || __ldg(a.t10 + j - 1) < thi * (1.0 + 1e-9);
