@@ -447,9 +447,11 @@ static cudaError_t reserve_pinned(double *&p, size_t &n, size_t count) {
     if (e == cudaSuccess) n = count;
     return e;
 }
-static bool page_locked(const void *p) {
+// Memory that a copy by way of a page-locked buffer suits: the host's, neither page-locked nor managed. (The caller's array
+// may be any that a copy from the device reaches: to the device's own memory the host must not write.)
+static bool is_pageable(const void *p) {
     cudaPointerAttributes a;
-    const bool yes = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeHost;
+    const bool yes = cudaPointerGetAttributes(&a, p) == cudaSuccess && a.type == cudaMemoryTypeUnregistered;
     cudaGetLastError();
     return yes;
 }
@@ -1338,9 +1340,9 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             return ST_DATA_MISSING;
         }
     }
-    // (to a page-locked caller's array directly, else through the page-locked staging buffer: a copy to pageable memory
-    // holds the host until it is done, with every copy after it)
-    const bool stage_mags = want_mags && !io.dev_inputs && !chunked && !page_locked(io.mags);
+    // (to pageable memory through the page-locked staging buffer: a copy to it holds the host until it is done, with every
+    // copy after it)
+    const bool stage_mags = want_mags && !io.dev_inputs && !chunked && is_pageable(io.mags);
     if (stage_mags && (e = reserve_pinned(c.pinned_mags, c.pinned_mags_n, (size_t)n * nb)) != cudaSuccess) {
         err = cuda_msg("page-locked magnitudes", e);
         return ST_DATA_MISSING;
