@@ -2263,17 +2263,23 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
     const int nkb_y = slabs ? itesc * kpa : (ky + gemm_bk() - 1) / gemm_bk();
     const int nkb_o = slabs ? (nt - itesc) * kpa : (ko + gemm_bk() - 1) / gemm_bk();
     const int mtiles = slabs ? tile0[1] : (chunk + gemm_bm() - 1) / gemm_bm();
-    const int tiles_mn = mtiles * ((o.ntempl + gemm_bn() - 1) / gemm_bn());
+    const int ntiles = (o.ntempl + gemm_bn() - 1) / gemm_bn();
     // Two slabs: a split's blocks all hold weights, where a split over every slab is mostly zeros, and the tensor core's
-    // accumulator rounds at each step. At most 24 blocks a split (8 up to 512 models, whose partial sums are few) keep
-    // the spectra as near the exact ones as the fold over every slab does: 4.9e-6 of their norm at 1024 models (5.2e-6
-    // over every slab; 5.6e-6 and 31 us less with the splits that fill the SMs alone, 7.0e-6 at 1500).
+    // accumulator rounds at each step: the more blocks of weights a split has, the lower its sums. No split has more of
+    // them than the fold over every slab would give it (its count of splits over as many ages: 2 blocks up to 128 models,
+    // 5 to 256), nor more than 24 (8 up to 512 models): error against 64 bits, of the spectra's
+    // norm, over two slabs and over every slab: 2.6e-6 and 2.6e-6 at one model, 3.8e-6 and 3.8e-6 at 128, 4.1e-6 and 4.3e-6 at
+    // 256, 4.9e-6 and 5.2e-6 at 1024; with the 24 and 8 alone 4.0e-6 at 128, for 11 us less (1024: 21 us less).
     const int most_blocks = chunk <= 512 ? 8 : 24;
-    auto splits = [&](int nkb) {
-        const int ks = gemm_choose_ksplit(tiles_mn, nkb, c.num_sms);
-        return slabs ? std::max(ks, (nkb + most_blocks - 1) / most_blocks) : ks;
+    auto splits = [&](int nkb, int nkb_all) {
+        const int ks = gemm_choose_ksplit(mtiles * ntiles, nkb, c.num_sms);
+        if (!slabs) return ks;
+        const int whole = gemm_choose_ksplit((chunk + gemm_bm() - 1) / gemm_bm() * ntiles, nkb_all, c.num_sms);
+        const int blocks = std::max(1, std::min(most_blocks, nkb / whole));
+        return std::max(ks, (nkb + blocks - 1) / blocks);
     };
-    const int ks_y = ky > 0 ? splits(nkb_y) : 0, ks_o = ko > 0 ? splits(nkb_o) : 0;
+    const int ks_y = ky > 0 ? splits(nkb_y, (ky + gemm_bk() - 1) / gemm_bk()) : 0;
+    const int ks_o = ko > 0 ? splits(nkb_o, (ko + gemm_bk() - 1) / gemm_bk()) : 0;
     const size_t xld = slabs ? (size_t)nt * slab2 : ktot;                    // the operand's columns
     if ((e = c.d_ix_hi.reserve((size_t)chunk * xld)) != cudaSuccess || (e = c.d_ix_lo.reserve((size_t)chunk * xld)) != cudaSuccess ||
         (e = c.d_ix_const.reserve((size_t)n)) != cudaSuccess ||
