@@ -114,7 +114,8 @@ struct Emulator {
     int *d_flag = nullptr, *d_nflag = nullptr, *d_flagged = nullptr;
     float *d_scratch = nullptr;                  // the inference kernel's tile inputs and member outputs
     size_t scratch_cap = 0;                      // its floats
-    float *h_stage = nullptr;                    // page-locked staging of predict's inputs and outputs
+    float *h_stage = nullptr;                    // page-locked staging of predict's inputs and outputs (emu_stage)
+    int stage_cap = 0;                           // its models
     int cap = 0;
     void release();
 };

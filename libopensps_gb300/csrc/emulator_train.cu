@@ -65,6 +65,7 @@ void Emulator::release() {
     scratch_cap = 0;
     if (h_stage) cudaFreeHost(h_stage);
     h_stage = nullptr;
+    stage_cap = 0;
     d_flag = d_nflag = d_flagged = nullptr;
     cap = 0;
     ready = trainable = false;
@@ -753,8 +754,7 @@ static int emu_step(Context &c, Emulator &e, EmuTrainBufs &b, const float *y, co
 }
 
 // ---------------------------------------------------------------------------------------------- inference scratch
-// (at least 16384 models' worth, 8 MB: small batches of growing size do not allocate again; with page-locked staging of
-// the inputs and outputs, x then mags, coef, spread and flags)
+// (at least 16384 models' worth, 8 MB: small batches of growing size do not allocate again)
 static int emu_scratch(Emulator &e, int n, std::string &err) {
     if (n <= e.cap) return 0;
     n = std::max(n, 16384);
@@ -772,12 +772,32 @@ static int emu_scratch(Emulator &e, int n, std::string &err) {
     ok(dalloc(&e.d_flag, (size_t)n));
     ok(dalloc(&e.d_flagged, (size_t)n));
     if (!e.d_nflag) ok(dalloc(&e.d_nflag, 4));
-    if (e.h_stage) cudaFreeHost(e.h_stage);
-    e.h_stage = nullptr;
-    ok(cudaMallocHost(&e.h_stage, sizeof(float) * (size_t)n * (EMU_NIN + EMU_MAX_BANDS + EMU_NPC + 2)));
     if (r != cudaSuccess) { err = cmsg("emulator scratch", r); e.cap = 0; return ST_DATA_MISSING; }
     e.cap = n;
     return 0;
+}
+
+// Host staging of a slice of n models: the inputs, or the magnitudes, coefficients, spread and flags. Page-locked and kept,
+// at most EMU_SLICE models' (30 MB: larger predictions go through it slice by slice), or pageable memory when no more can
+// be page-locked.
+constexpr int EMU_SLICE = 65536;
+constexpr size_t EMU_STAGE_FLOATS = EMU_MAX_BANDS + EMU_NPC + 2;   // (more than the EMU_NIN inputs)
+static float *emu_stage(Emulator &e, int n, std::vector<float> &pageable) {
+    if (n > e.stage_cap) {
+        if (e.h_stage) cudaFreeHost(e.h_stage);
+        e.h_stage = nullptr;
+        e.stage_cap = 0;
+        const int cap = std::max(n, 16384);
+        if (cudaMallocHost(&e.h_stage, sizeof(float) * EMU_STAGE_FLOATS * cap) == cudaSuccess) {
+            e.stage_cap = cap;
+        } else {
+            cudaGetLastError();
+            e.h_stage = nullptr;
+            pageable.resize(EMU_STAGE_FLOATS * n);
+            return pageable.data();
+        }
+    }
+    return e.h_stage;
 }
 
 // The ensemble on n device inputs (n x 10 floats): outputs into the given device arrays.
@@ -1387,37 +1407,50 @@ int emu_predict(Context &c, int n, const double *inputs, int fallback, double *m
     if (n <= 0) { if (n_fallback) *n_fallback = 0; return 0; }
     if (!inputs) { err = "emulator: inputs are NULL"; return ST_BAD_ARG; }
     if (int rc = emu_scratch(e, n, err)) return rc;
-    const int nb = e.nb;
-    float *xh = e.h_stage, *mg = xh + (size_t)n * EMU_NIN, *cf = mg + (size_t)n * nb, *sp = cf + (size_t)n * EMU_NPC;
-    int *fl = reinterpret_cast<int *>(sp + n);
-    for (size_t i = 0; i < (size_t)n * EMU_NIN; ++i) xh[i] = (float)inputs[i];
-    cudaMemcpyAsync(e.d_x, xh, sizeof(float) * n * EMU_NIN, cudaMemcpyHostToDevice, c.stream);
+    const int nb = e.nb, slice = std::min(n, EMU_SLICE);
+    std::vector<float> pageable;
+    float *const stage = emu_stage(e, slice, pageable);
+    // the inputs, a slice at a time (the next one is written once the copy has read this one)
+    for (int m0 = 0; m0 < n; m0 += slice) {
+        const size_t k = (size_t)std::min(slice, n - m0) * EMU_NIN, at = (size_t)m0 * EMU_NIN;
+        cudaError_t r = m0 > 0 ? cudaStreamSynchronize(c.stream) : cudaSuccess;
+        for (size_t i = 0; i < k; ++i) stage[i] = (float)inputs[at + i];
+        if (r == cudaSuccess) r = cudaMemcpyAsync(e.d_x + at, stage, sizeof(float) * k, cudaMemcpyHostToDevice, c.stream);
+        if (r != cudaSuccess) { err = cmsg("emulator inputs", r); return ST_DATA_MISSING; }
+    }
     if (int rc = emu_infer_device(c, n, e.d_x, e.d_mags, pca ? e.d_coef : nullptr, e.d_spread, e.d_flag, e.d_nflag,
-                                  e.d_flagged, err))
+                                  e.d_flagged, err)) {
+        cudaStreamSynchronize(c.stream);         // (the copy that reads the staging buffer)
         return rc;
+    }
     int nf = 0;
-    cudaMemcpyAsync(mg, e.d_mags, sizeof(float) * n * nb, cudaMemcpyDeviceToHost, c.stream);
-    cudaMemcpyAsync(fl, e.d_flag, sizeof(int) * n, cudaMemcpyDeviceToHost, c.stream);
-    if (pca) cudaMemcpyAsync(cf, e.d_coef, sizeof(float) * n * EMU_NPC, cudaMemcpyDeviceToHost, c.stream);
-    if (spread) cudaMemcpyAsync(sp, e.d_spread, sizeof(float) * n, cudaMemcpyDeviceToHost, c.stream);
-    if (int rc = check_status(c, err)) return rc;
-    if (mags)
-        for (size_t i = 0; i < (size_t)n * nb; ++i) mags[i] = mg[i];
-    if (pca)
-        for (size_t i = 0; i < (size_t)n * EMU_NPC; ++i) pca[i] = cf[i];
-    if (spread)
-        for (int m = 0; m < n; ++m) spread[m] = sp[m];
-    for (int m = 0; m < n; ++m) {
-        if (source) source[m] = fl[m];
-        nf += fl[m] != 0;
+    std::vector<int> idx;                        // the flagged models (kept for the fallback)
+    float *const mg = stage, *const cf = mg + (size_t)slice * nb, *const sp = cf + (size_t)slice * EMU_NPC;
+    int *const fl = reinterpret_cast<int *>(sp + slice);
+    for (int m0 = 0; m0 < n; m0 += slice) {
+        const size_t k = std::min(slice, n - m0);
+        cudaMemcpyAsync(mg, e.d_mags + (size_t)m0 * nb, sizeof(float) * k * nb, cudaMemcpyDeviceToHost, c.stream);
+        cudaMemcpyAsync(fl, e.d_flag + m0, sizeof(int) * k, cudaMemcpyDeviceToHost, c.stream);
+        if (pca) cudaMemcpyAsync(cf, e.d_coef + (size_t)m0 * EMU_NPC, sizeof(float) * k * EMU_NPC, cudaMemcpyDeviceToHost, c.stream);
+        if (spread) cudaMemcpyAsync(sp, e.d_spread + m0, sizeof(float) * k, cudaMemcpyDeviceToHost, c.stream);
+        if (int rc = check_status(c, err)) return rc;
+        if (mags)
+            for (size_t i = 0; i < k * nb; ++i) mags[(size_t)m0 * nb + i] = mg[i];
+        if (pca)
+            for (size_t i = 0; i < k * EMU_NPC; ++i) pca[(size_t)m0 * EMU_NPC + i] = cf[i];
+        if (spread)
+            for (size_t m = 0; m < k; ++m) spread[m0 + m] = sp[m];
+        for (size_t m = 0; m < k; ++m) {
+            if (source) source[m0 + m] = fl[m];
+            if (fl[m]) {
+                ++nf;
+                if (fallback) idx.push_back(m0 + (int)m);
+            }
+        }
     }
     if (n_fallback) *n_fallback = nf;
     if (!fallback || nf == 0) return 0;
     // ---- the flagged models through the plain CSP (in model order)
-    std::vector<int> idx;
-    idx.reserve(nf);
-    for (int m = 0; m < n; ++m)
-        if (fl[m]) idx.push_back(m);
     const int nfb = (int)idx.size();
     std::vector<double> vals((size_t)EMU_NIN * nfb), mf((size_t)nb * nfb);
     for (int j = 0; j < nfb; ++j)
