@@ -447,6 +447,13 @@ static cudaError_t reserve_pinned(double *&p, size_t &n, size_t count) {
     if (e == cudaSuccess) n = count;
     return e;
 }
+// Count doubles to copy through: the context's page-locked buffer, or pageable memory where no more can be page-locked.
+static double *staging(double *&p, size_t &n, size_t count, std::vector<double> &pageable) {
+    if (reserve_pinned(p, n, count) == cudaSuccess) return p;
+    cudaGetLastError();
+    pageable.resize(count);
+    return pageable.data();
+}
 // Memory that a copy by way of a page-locked buffer suits: the host's, neither page-locked nor managed. (The caller's array
 // may be any that a copy from the device reaches: to the device's own memory the host must not write.)
 static bool is_pageable(const void *p) {
@@ -455,6 +462,7 @@ static bool is_pageable(const void *p) {
     cudaGetLastError();
     return yes;
 }
+constexpr size_t MAG_STAGE = (size_t)4 << 20;   // the magnitudes' staging, in doubles (32 MB; larger batches by pieces)
 
 static std::string cuda_msg(const char *what, cudaError_t e) { return std::string(what) + ": " + cudaGetErrorString(e); }
 
@@ -624,24 +632,22 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     cudaStream_t st = c.stream;
     // the weights over ages (the SFH's, or the caller's) and their blend at logzsol, formed on the device: queued here,
     // so that they run beside the checks that follow
+    std::vector<double> sfh_pageable, sfhout_pageable;
     struct SfhInFlight {   // (a batch refused after this point waits: the next one reuses the staging buffer)
         cudaStream_t st = nullptr;
         ~SfhInFlight() { if (st) cudaStreamSynchronize(st); }
     } sfh_in_flight;
     if (io.sfh_par) {
         const size_t np = (size_t)SFH_NCOL * n;
-        if ((e = reserve_pinned(c.pinned_sfh, c.pinned_sfh_n, np)) != cudaSuccess) {
-            err = cuda_msg("page-locked SFH parameters", e);
-            return ST_DATA_MISSING;
-        }
         sfh_in_flight.st = st;
-        std::memcpy(c.pinned_sfh, io.sfh_par, sizeof(double) * np);
+        double *const sfh_host = staging(c.pinned_sfh, c.pinned_sfh_n, np, sfh_pageable);
+        std::memcpy(sfh_host, io.sfh_par, sizeof(double) * np);
         if ((e = c.d_wz.reserve((size_t)n * nt * nz)) != cudaSuccess || (e = c.d_sfhpar.reserve(np)) != cudaSuccess || (e = c.d_w.reserve((size_t)nt * n)) != cudaSuccess ||
             (e = c.d_sfh_scratch.reserve((size_t)2 * nt * n)) != cudaSuccess ||
             (e = c.d_sfh_mtab.reserve((size_t)(nt + 1) * n)) != cudaSuccess ||
             (e = c.d_lblend.reserve((size_t)3 * n)) != cudaSuccess || (e = c.d_sfr.reserve(n)) != cudaSuccess ||
             (io.given_w && (e = c.d_wgiven.reserve((size_t)nt * n)) != cudaSuccess) ||
-            (e = cudaMemcpyAsync(c.d_sfhpar.p, c.pinned_sfh, sizeof(double) * np, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (e = cudaMemcpyAsync(c.d_sfhpar.p, sfh_host, sizeof(double) * np, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
             (io.given_w && (e = cudaMemcpyAsync(c.d_wgiven.p, io.given_w, sizeof(double) * nt * n, cudaMemcpyHostToDevice, st)) != cudaSuccess)) {
             err = cuda_msg("SFH inputs", e);
             return ST_DATA_MISSING;
@@ -1342,13 +1348,15 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     }
     // (to pageable memory through the page-locked staging buffer: a copy to it holds the host until it is done, with every
     // copy after it)
-    const bool stage_mags = want_mags && !io.dev_inputs && !chunked && is_pageable(io.mags);
-    if (stage_mags && (e = reserve_pinned(c.pinned_mags, c.pinned_mags_n, (size_t)n * nb)) != cudaSuccess) {
-        err = cuda_msg("page-locked magnitudes", e);
-        return ST_DATA_MISSING;
+    const size_t n_mags = (size_t)n * nb, mag_piece = std::min(n_mags, MAG_STAGE);
+    bool stage_mags = want_mags && !io.dev_inputs && !chunked && is_pageable(io.mags);
+    if (stage_mags && reserve_pinned(c.pinned_mags, c.pinned_mags_n, mag_piece) != cudaSuccess) {
+        cudaGetLastError();
+        stage_mags = false;
     }
     if (want_mags && !io.dev_inputs && !chunked) {
-        if ((e = cudaMemcpyAsync(stage_mags ? c.pinned_mags : io.mags, c.d_mags.p, sizeof(double) * n * nb, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
+        if ((e = cudaMemcpyAsync(stage_mags ? c.pinned_mags : io.mags, c.d_mags.p, sizeof(double) * (stage_mags ? mag_piece : n_mags),
+                                 cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
             err = cuda_msg("magnitudes copy", e);
             return ST_DATA_MISSING;
         }
@@ -1374,14 +1382,11 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     // (page-locked: the SFR, then L_bol total, young and old)
     const double *lblend = nullptr, *sfr_h = nullptr;
     if (io.sfh_par && !io.dev_inputs) {
-        if ((e = reserve_pinned(c.pinned_sfhout, c.pinned_sfhout_n, (size_t)4 * n)) != cudaSuccess) {
-            err = cuda_msg("page-locked SFH outputs", e);
-            return ST_DATA_MISSING;
-        }
-        sfr_h = c.pinned_sfhout;
-        if (!ops) lblend = c.pinned_sfhout + n;
-        if ((!ops && (e = cudaMemcpyAsync(c.pinned_sfhout + n, c.d_lblend.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
-            (e = cudaMemcpyAsync(c.pinned_sfhout, c.d_sfr.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
+        double *const out = staging(c.pinned_sfhout, c.pinned_sfhout_n, (size_t)4 * n, sfhout_pageable);
+        sfr_h = out;
+        if (!ops) lblend = out + n;
+        if ((!ops && (e = cudaMemcpyAsync(out + n, c.d_lblend.p, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) ||
+            (e = cudaMemcpyAsync(out, c.d_sfr.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st)) != cudaSuccess) {
             err = cuda_msg("SFH outputs copy", e);
             return ST_DATA_MISSING;
         }
@@ -1407,7 +1412,15 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
 #pragma omp parallel for schedule(static)
         for (int m = 0; m < n; ++m) std::memcpy(io.mags + (size_t)nb * m, src + (size_t)nb * m, sizeof(double) * nb);
     }
-    if (stage_mags) std::memcpy(io.mags, c.pinned_mags, sizeof(double) * n * nb);
+    for (size_t i = 0; stage_mags && i < n_mags; i += mag_piece) {
+        const size_t k = std::min(mag_piece, n_mags - i);
+        if (i > 0 && ((e = cudaMemcpyAsync(c.pinned_mags, c.d_mags.p + i, sizeof(double) * k, cudaMemcpyDeviceToHost, st)) != cudaSuccess ||
+                      (e = cudaStreamSynchronize(st)) != cudaSuccess)) {
+            err = cuda_msg("magnitudes copy", e);
+            return ST_DATA_MISSING;
+        }
+        std::memcpy(io.mags + i, c.pinned_mags, sizeof(double) * k);
+    }
     if (want_sums && !io.dev_inputs) {
 #pragma omp parallel for schedule(static) if (n >= 8192)
         for (int m = 0; m < n; ++m) {

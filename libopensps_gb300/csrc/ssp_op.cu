@@ -2218,18 +2218,22 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
     // slabs: the models by the lower of their two metallicities (the interval sfh_forward_kernel takes), and per chunk of
     // that order the M tiles of one metallicity
     std::vector<int> tile0(nchunk + 1, 0);
+    std::vector<int4> pageable;              // (in the place of the page-locked table, when none can be had)
     if (slabs) {
         const size_t cap = (size_t)n + n / gemm_bm() + (size_t)nchunk * nz;   // tiles (int4) and rows (two to an int4)
         if (c.pinned_fold_n < cap) {
             if (c.pinned_fold) cudaFreeHost(c.pinned_fold);
             c.pinned_fold = nullptr;
             c.pinned_fold_n = 0;
-            if ((e = cudaMallocHost(&c.pinned_fold, sizeof(int4) * cap)) != cudaSuccess) {
-                err = cmsg("page-locked fold tiles", e);
-                return ST_DATA_MISSING;
+            if (cudaMallocHost(&c.pinned_fold, sizeof(int4) * cap) == cudaSuccess) {
+                c.pinned_fold_n = cap;
+            } else {
+                cudaGetLastError();
+                c.pinned_fold = nullptr;
+                pageable.resize(cap);
             }
-            c.pinned_fold_n = cap;
         }
+        int4 *const fold = pageable.empty() ? c.pinned_fold : pageable.data();
         std::vector<int> zl(n), at(nz + 1, 0);
         for (int m = 0; m < n; ++m) {
             const int k = find_interval0(c.lzv.data(), nz, h_sfh[(size_t)SFH_NCOL * m + SFH_LOGZSOL]) + 1;
@@ -2237,9 +2241,9 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
             ++at[zl[m] + 1];
         }
         for (int z = 0; z < nz; ++z) at[z + 1] += at[z];
-        int2 *rz = reinterpret_cast<int2 *>(c.pinned_fold);
+        int2 *rz = reinterpret_cast<int2 *>(fold);
         for (int m = 0; m < n; ++m) rz[at[zl[m]]++] = make_int2(m, zl[m]);
-        int4 *mt = c.pinned_fold + (n + 1) / 2;
+        int4 *mt = fold + (n + 1) / 2;
         int nt_all = 0;
         for (int k = 0; k < nchunk; ++k) {
             tile0[k] = nt_all;
@@ -2254,7 +2258,8 @@ static int run_ops_interp(Context &c, int n, const double *d_wz, const double *d
         tile0[nchunk] = nt_all;
         const size_t used = (size_t)(n + 1) / 2 + nt_all;
         if ((e = c.d_fold.reserve(cap)) != cudaSuccess ||
-            (e = cudaMemcpyAsync(c.d_fold.p, c.pinned_fold, sizeof(int4) * used, cudaMemcpyHostToDevice, st)) != cudaSuccess) {
+            (e = cudaMemcpyAsync(c.d_fold.p, fold, sizeof(int4) * used, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
+            (!pageable.empty() && (e = cudaStreamSynchronize(st)) != cudaSuccess)) {
             err = cmsg("fold tiles", e);
             return ST_DATA_MISSING;
         }

@@ -1,5 +1,5 @@
 """Where a batch's magnitudes may go: pageable, page-locked and device memory give the same bits (SFH batches and weights
-over ages and metallicities)."""
+over ages and metallicities), and so do batches whose magnitudes come down in more than one piece of 4 Mi doubles."""
 import ctypes as C
 
 import numpy as np
@@ -50,3 +50,19 @@ def test_any_memory(data, built_lib, weights):
     c.close()
     assert np.isfinite(host).all() and host.all()
     assert np.array_equal(host, pinned.numpy()) and np.array_equal(host, dev.cpu().numpy())
+
+
+def test_magnitudes_in_pieces(data, built_lib):
+    import torch
+    from libopensps_gb300.capi import Context
+    c = Context()
+    c.set_int("sfh", 4)
+    n = (4 << 20) // c.nbands + 1000
+    params = _params(n)
+    host = np.zeros((n, c.nbands))
+    pinned = torch.zeros((n, c.nbands), dtype=torch.float64).pin_memory()
+    for ptr in (host.ctypes.data, pinned.data_ptr()):
+        _mags(c, params, n, ptr)
+    c.close()
+    assert np.isfinite(host).all() and host.all()
+    assert np.array_equal(host, pinned.numpy())
