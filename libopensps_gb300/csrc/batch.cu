@@ -633,7 +633,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     // the weights over ages (the SFH's, or the caller's) and their blend at logzsol, formed on the device: queued here,
     // so that they run beside the checks that follow
     std::vector<double> sfh_pageable, sfhout_pageable;
-    struct SfhInFlight {   // (a batch refused after this point waits: the next one reuses the staging buffer)
+    struct SfhInFlight {   // (a batch that ends early after this point waits: the next one reuses the staging buffer)
         cudaStream_t st = nullptr;
         ~SfhInFlight() { if (st) cudaStreamSynchronize(st); }
     } sfh_in_flight;
@@ -926,7 +926,6 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
     // ---- scratch
     const int kpad = ops ? 64 : bop->kpad;
     const size_t nwz = (size_t)n * nt * nz;
-    sfh_in_flight.st = nullptr;   // (every check has passed)
     if ((!io.dev_inputs && (e = c.d_wz.reserve(nwz)) != cudaSuccess) ||
         (e = c.d_params.reserve((size_t)PAR_DEVICE * n)) != cudaSuccess ||
         (e = c.d_whi.reserve((size_t)n * kpad)) != cudaSuccess || (e = c.d_wlo.reserve((size_t)n * kpad)) != cudaSuccess ||
@@ -1397,6 +1396,7 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
         err = cuda_msg("batch", e);
         return ST_DATA_MISSING;
     }
+    sfh_in_flight.st = nullptr;
     if (kstatus != 0) {
         char buf[96];
         std::snprintf(buf, sizeof buf, "a device wait gave up (code 0x%x)", kstatus);
