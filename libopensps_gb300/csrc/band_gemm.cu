@@ -322,20 +322,33 @@ band_gemm_kernel(const __grid_constant__ CUtensorMap tm_c_hi, const __grid_const
 int band_gemm_npad(int nbands) { return (nbands + 15) / 16 * 16 < 32 ? 32 : (nbands + 15) / 16 * 16; }
 
 // Splits of the pixel blocks over a cluster's CTAs. Few tiles (at most 4096 models): up to two CTAs per SM. More: the
-// split with the least time on the busiest SM, whose CTAs run two at a time: a pair takes 3.1 us a pixel block, a CTA
-// alone 2.3 (a builder warp's own latencies bound it, and two CTAs hide part of them), and every CTA takes BG_SETUP
-// blocks' time besides (its setup, the pipeline's fill, its magnitudes). Measured, us at splits
-// of 1 .. 6: 113, 64, 60, 49, 68, 67 at 9001 models; 145, 132, 111, 114, 110, 116 at 20001; 120 and 90 at 1 and 2 at 16384.
+// split with the least time on the busiest SM, where every CTA takes BG_SETUP blocks' time besides its blocks' (its setup,
+// the pipeline's fill, its magnitudes).
+// Up to 80 bands an SM's CTAs run two at a time: a pair takes 3.1 us a pixel block, a CTA alone 2.3 (a builder warp's own
+// latencies bound it, and two CTAs hide part of them). Measured, us at splits of 1 .. 6: 113, 64, 60, 49, 68, 67 at 9001
+// models; 145, 132, 111, 114, 110, 116 at 20001; 120 and 90 at 1 and 2 at 16384.
+// Above 80 bands one CTA fills an SM: 1, 2 or 4 CTAs by the waves of clusters (of four, one in twenty's places is lost to
+// the GPCs' sizes; other sizes lose more). 100 bands, us at splits of 1 .. 8: 124, 76, 61, 52, 72, 66, 84, 76 at 4500 models;
+// 146, 89, 115, 97, 117, 133, 151, 136 at 9001; 150, 158, 166, 174 .. at 16384; 278, 295, 311, 294 .. at 30000; 543, 517,
+// 612, 613 .. at 65536 (priced as pairs of CTAs: 77, 97, 159, 279, 518).
 static int band_gemm_ksplit(int n_models, int nkb, int npad, int num_sms) {
     const int tiles = (n_models + BG_M - 1) / BG_M;
     // (clusters beyond the portable eight only where two of their CTAs share an SM)
-    const int most = std::max(1, std::min(nkb / BG_MIN_BLOCKS, BandGemmSmem::two_ctas(npad) ? BG_MAX_SPLIT : 8));
+    const bool two = BandGemmSmem::two_ctas(npad);
+    const int most = std::max(1, std::min(nkb / BG_MIN_BLOCKS, two ? BG_MAX_SPLIT : 8));
     if (tiles <= BG_FEW_TILES) return std::min((2 * num_sms + tiles - 1) / tiles, most);
     int best = 1;
     long long best_cost = 0;
-    for (int ks = 1; ks <= std::min(most, 8); ++ks) {
-        const long long ctas = ((long long)tiles * ks + num_sms - 1) / num_sms;     // of the busiest SM
-        const long long cost = (ctas / 2 * 31 + ctas % 2 * 23) * ((nkb + ks - 1) / ks + BG_SETUP);
+    for (int ks = 1; ks <= std::min(most, two ? 8 : 4); ks = two ? ks + 1 : 2 * ks) {
+        const long long blocks = (nkb + ks - 1) / ks + BG_SETUP;
+        long long cost;
+        if (two) {
+            const long long ctas = ((long long)tiles * ks + num_sms - 1) / num_sms;     // of the busiest SM
+            cost = (ctas / 2 * 31 + ctas % 2 * 23) * blocks;
+        } else {
+            const int at_once = std::max(1, (ks == 4 ? num_sms * 19 / 20 : num_sms) / ks);   // clusters
+            cost = (tiles + at_once - 1) / at_once * blocks;
+        }
         if (ks == 1 || cost < best_cost) { best = ks; best_cost = cost; }
     }
     return best;
