@@ -464,20 +464,25 @@ __global__ void __launch_bounds__(128) sfh_moments_kernel(SfhArgs a) {
     SfhT<double> s;
     sfh_setup(a.sfh, p, s);
     const double tlo = smax(s.tq, 1.0), thi = smax(s.tage, 1.0);
-    double t, lt;
-    bool need = true;
+    double t, lt = 0.0;
+    bool need = true, end = false;
     const double tj = j < a.nt ? __ldg(a.t10 + j) : 0.0;
     if (j == a.nt || tj <= tlo) {
         t = fmin(tlo, thi);
-        lt = t == 1.0 ? 0.0 : log10(t);
         need = j == a.nt || __ldg(a.t10 + min(j + 1, a.nt - 1)) * (1.0 + 1e-9) > tlo;
+        end = need && t != 1.0;
     } else if (tj >= thi) {
         t = thi;
-        need = j == 0 || __ldg(a.t10 + j - 1) < thi * (1.0 + 1e-9);
-        lt = need ? log10(thi) : 0.0;
+        end = need = j == 0 || __ldg(a.t10 + j - 1) < thi * (1.0 + 1e-9);
     } else {
         t = tj;
         lt = __ldg(a.tf + j);
+    }
+    if (end) {
+        // (the time of the rounded logarithm, as at the grid's ages: with the end itself the first moment's logarithm is off
+        // by its last place, and masses stand half as far again from the exact ones)
+        lt = log10(t);
+        t = exp10(lt);
     }
     double2 r = make_double2(0.0, 0.0);
     if (need && !(s.tau <= SAFE_FLOOR)) {
