@@ -1,5 +1,4 @@
-// Band fluxes and AB magnitudes as a tensor-core GEMM: fband(m, b) = sum_j Fobs(m, j) C(j, b); with, beside them,
-// the FP64 mass and L_bol sums of the same models.
+// Band fluxes and AB magnitudes as a tensor-core GEMM: fband(m, b) = sum_j Fobs(m, j) C(j, b).
 //
 // compute_magnitudes_columns (OpenSPS src/spectra/opensps_batch_photometry.f90:53-180): each model's rest-frame
 // spectrum resampled to the observed frame at its redshift, divided by lambda (observed_frame_z :819-903), then the
@@ -9,9 +8,9 @@
 // host), so the A operand is the resampled spectrum itself.
 //
 // Per CTA: 128 models (MMA M). K = the pixels that any band reaches, 64 per stage. The A operand (observed frame
-// of 128 models x 64 pixels) is built by warps 0..7 in shared memory from the spectra, in the 128-byte swizzled
+// of 128 models x 64 pixels) is built by warps 0..15 in shared memory from the spectra, in the 128-byte swizzled
 // K-major layout, split into bf16 hi and lo; the B operand (band matrix, hi and lo, bands x pixels) comes by TMA.
-// fband = A_hi B_hi + A_hi B_lo + A_lo B_hi in f32 in tensor memory; the epilogue forms the magnitudes.
+// fband = A_hi B_hi + A_hi B_lo + A_lo B_hi in f32 in tensor memory; all the warps form the magnitudes.
 // Warp roles: warps 0..15 build the A operand (8 model rows each: two CTAs of 17 warps per SM at 56 registers, against
 // 9 warps of 16 rows at 92), warp 16 issues the band matrix's TMA and the MMAs.
 // Two stages with mbarriers: a builder warp signals its rows of stage s on full_a[s] and goes on to the next stage as

@@ -1009,8 +1009,8 @@ int run_batch(Context &c, const BatchIO &io, std::string &err) {
             if ((e = chunk_copy(k)) != cudaSuccess) { err = cuda_msg("weights copy", e); return ST_DATA_MISSING; }
     cudaMemsetAsync(c.d_status.p, 0, sizeof(int), st);
 
-    // ---- the per-model parameters, then the weight operand (one stream: run side by side they took longer than in
-    // turn)
+    // ---- the per-model parameters and the weight operand (above FORK_MODELS models on streams of their own, below
+    // in turn: run_range)
     prof_mark(c, 0);
     // per-model parameters of models [off, off + nk)
     auto model_params = [&](int off, int nk) -> cudaError_t {

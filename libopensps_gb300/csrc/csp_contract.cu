@@ -12,13 +12,14 @@
 // lo parts (x = x_hi + x_lo); D = A_hi B_hi + A_hi B_lo + A_lo B_hi, accumulated in f32 in tensor memory. Tile: 128
 // pixels x BN models x 64 K per stage; the 128 pixel rows of a tile are 120 output pixels with a halo of 4 on each
 // side for the smoothing; BN is the largest tile (256 models, 128 with two accumulators) or a narrower one of a smaller
-// batch, with the stages that fit (contract_tile); a CTA pair takes two pixel tiles by BN models in one MMA. The 16-column K steps past a range's last column are left out
-// (81 steps of 84 for 107 ages x 12 metallicities). One CTA per SM, persistent over tiles (model tile outer, pixel tile inner, so that the
-// CTAs running together share the weights of a model tile in L2). Warp roles: warp 0 = TMA producer, warp 1 = MMA
-// issuer (and TMEM owner; in a pair CTA 0's), the others = epilogue in groups of four (group g takes the models of the
-// g-th part of the columns; in a group, warp w reads TMEM lanes 32 (w % 4) ..): four groups (with two the epilogue was
-// the longer part of a pair's tile, 1820 us at 65536 models against 1591). Accumulators are double-buffered in TMEM so that the
-// epilogue of a tile overlaps the MMAs of the next.
+// batch, with the stages that fit (contract_tile); a CTA pair takes two pixel tiles by BN models in one MMA (with an odd
+// count of pixel tiles the last pair's second CTA multiplies zeros and stores nothing). The 16-column K steps past a
+// range's last column are left out (81 steps of 84 for 107 ages x 12 metallicities). One CTA per SM, persistent over
+// tiles (model tile outer, pixel tile inner, so that the CTAs running together share the weights of a model tile in L2).
+// Warp roles: warp 0 = TMA producer, warp 1 = MMA issuer (and TMEM owner; in a pair CTA 0's), the others = epilogue in
+// groups of four (group g takes the models of the g-th part of the columns; in a group, warp w reads TMEM lanes
+// 32 (w % 4) ..): four groups (with two the epilogue was the longer part of a pair's tile, 1820 us at 65536 models
+// against 1591). Accumulators are double-buffered in TMEM so that the epilogue of a tile overlaps the MMAs of the next.
 //
 // Epilogue of a chunk of 8 models, per group: phase 1, thread = pixel row: the attenuated, IGM-absorbed spectrum
 // of the chunk's models into a staging tile; phase 2, thread = 4 consecutive output pixels of one model: the velocity
@@ -449,7 +450,8 @@ static cudaError_t launch_contract(const ContractPlan &pl, const ContractArgs &a
 // models against 429. The widest tile is not always the cheapest: a batch may fill its last wave badly, or hold fewer
 // models than a tile.
 // Measured, one CTA per 256 (128) models and eight epilogue warps -> with the rule and sixteen: 38.7 -> 20 us at one
-// model, 80 -> 51 at 1000, 317 -> 239 at 9001, 1951 -> 1591 at 65536 (2.0 PFLOP/s executed). Every tile gives the same
+// model, 80 -> 51 at 1000, 317 -> 239 at 9001, 1951 -> 1591 at 65536 (1.90 PFLOP/s of the
+// pixels' products, 2.0 with the halo rows'). The costs are those of 1296 columns of K. Every tile gives the same
 // bits: an output's products are summed in the same order.
 ContractTile contract_tile(int nacc, int n_models, int n_ptiles, int num_sms) {
     struct Shape { int nacc, ctas, bn0; double first0, first1; double further[8]; };

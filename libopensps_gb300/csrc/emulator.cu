@@ -23,7 +23,8 @@
 //
 // A batch of few tiles leaves most SMs without one (four CTAs took 220 us for 500 models): there a CTA takes one member
 // of a tile at a time (SPLIT), its outputs go to the tile's place in the scratch, and emu_reduce_kernel forms the
-// ensemble's results from them: 224 -> 47 us at 500 models, 441 -> 227 at 20000.
+// ensemble's results from them: 224 -> 47 us at 500 models, 441 -> 227 at 20000. So do batches whose members take fewer
+// rounds over the SMs than whole tiles would (emu_split: on 152 SMs up to 121 tiles, and from 153 to 273).
 //
 // Every mbarrier wait is bounded (status word, no hang); drains wait for the copies and MMAs in flight.
 #include <cuda_runtime.h>
@@ -204,8 +205,7 @@ __device__ __forceinline__ void emu_epilogue(const EmuInferArgs &a, uint8_t *S, 
     const int iters = Work::iters(ntiles);
     int *status = a.status;
     // per CTA, two slots x 128 rows x 16 words of tile inputs (the input row's 12 f16 words, zred, the flags, the
-    // distance term); this
-    // row's outputs of each member: scratch[cta][step][row][128], with SPLIT scratch[unit][row][128]
+    // distance term); this row's outputs of each member: scratch[cta][step][row][128], with SPLIT scratch[unit][row][128]
     uint4 *in_row = reinterpret_cast<uint4 *>(a.scratch + (size_t)blockIdx.x * EMU_SCRATCH_IN) + (size_t)r * 4;
     float *scr_row = a.scratch + (size_t)gridDim.x * EMU_SCRATCH_IN +
                      (SPLIT ? 0 : (size_t)blockIdx.x * EMU_MEMBERS * 128 * EMU_NOUT) + (size_t)r * EMU_NOUT;

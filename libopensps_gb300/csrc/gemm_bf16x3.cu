@@ -82,7 +82,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a_hi, const __grid_const
     const int rank = CTAS == 2 ? (int)cluster_ctarank() : 0, tile0 = blockIdx.x / CTAS, tile_step = gridDim.x / CTAS;
     const int mt_n = SLABS ? g.n_mtiles : (g.M + CTAS * G_BM - 1) / (CTAS * G_BM), nt_n = (g.N + G_BN - 1) / G_BN;
     const int n_tiles = mt_n * nt_n * g.ksplit * g.groups;
-    // (SLABS: K blocks of an age's two slabs, kpa of them, the last with ktail columns)
+    // (SLABS: K blocks of an age's two slabs, kpa of them, the last of tail_steps steps of 16 columns)
     const int kpa = SLABS ? (g.slab2 + G_BK - 1) / G_BK : 1, nkb = SLABS ? g.ages * kpa : (g.K + G_BK - 1) / G_BK;
     const int tail_steps = SLABS ? (g.slab2 - (kpa - 1) * G_BK + 15) / 16 : G_BK / 16;
     int *status = g.status;

@@ -447,7 +447,7 @@ __device__ __forceinline__ void zinterval(const double *lz, int nz, double x, in
 // log10 years, whose rounding may leave an interval that ends at tq, up to the oldest age's, a width). t10 = 10^(log age) from the host. After them one thread per
 // model for the SFR, which one lane of a warp per model would take as long for as 32.
 // Bound by the FP64 pipe: about 110 instructions per limit, 612 with the series term by term, pow and logarithms per
-// limit: 116 us at 4001 models, 454 before (sfh_forward_kernel 116, 526 before).
+// limit: 125 us at 4001 models, 454 before (sfh_forward_kernel 116, 526 before).
 __device__ double sfh_sfr(const double *tf, int nt, int sfh, const double *p);
 
 __global__ void __launch_bounds__(128) sfh_moments_kernel(SfhArgs a) {

@@ -180,7 +180,7 @@ __device__ __forceinline__ float ops_g2(float x) {
 // P = c lo^em expm1(em dl) / em (em = 2 - alpha, dl = ln(hi / lo)) has dP/dem = c lo^em dl (ln lo g1 + dl g2)(em dl)
 // and c2 the factor 2^(alpha1 - alpha2).
 __device__ inline void kroupa_setup(const double *al3, double lim_lo, double lim_hi, KroupaSeg &k, float &inv_total,
-                                    double *dlnT, double *total_out = nullptr) {
+                                    double *dlnT) {
     const double a1 = al3[0], a2 = al3[1], a3 = al3[2];
     const double c2 = pow(0.5, -a1 + a2);
     const double al[3] = {a1, a2, a3}, cs[3] = {1.0, c2, c2};
@@ -206,7 +206,6 @@ __device__ inline void kroupa_setup(const double *al3, double lim_lo, double lim
         }
     }
     inv_total = total > 0.0 ? (float)(1.0 / total) : 1.f;
-    if (total_out) *total_out = total;
     k.generic = 0;
     k.logn = 0;
     k.la = k.u0 = k.zs = 0.f;
@@ -224,7 +223,7 @@ __device__ inline void kroupa_setup(const double *al3, double lim_lo, double lim
 // (imf_integral case 4); 1 / T and, with dlnT, d ln T / d(alpha1, alpha2, mdave) (imf_integral_dp case 4: the
 // moving break's edge terms cancel, the IMF being continuous there).
 __device__ inline void dave_setup(const double *p, double lim_lo, double lim_hi, KroupaSeg &k, float &inv_total,
-                                  double *dlnT, double *total_out = nullptr) {
+                                  double *dlnT) {
     const double a1 = p[0], a2 = p[1], md = p[2];
     const double c2 = pow(md, -a1 + a2);
     const double al[2] = {a1, a2}, cs[2] = {1.0, c2}, slo[2] = {0.08, md}, shi[2] = {md, 1.0e30};
@@ -249,7 +248,6 @@ __device__ inline void dave_setup(const double *p, double lim_lo, double lim_hi,
     k.e[2] = k.c[2] = k.ce[2] = 0.f;
     k.lo[2] = k.hi[2] = 1.0e30f;
     inv_total = total > 0.0 ? (float)(1.0 / total) : 1.f;
-    if (total_out) *total_out = total;
     k.generic = 1;
     k.logn = 0;
     k.la = k.u0 = k.zs = 0.f;
@@ -269,7 +267,7 @@ __device__ inline void dave_setup(const double *p, double lim_lo, double lim_hi,
 // c_hi = exp(-u0^2 / (2 0.69^2))). 1 / T with the lognormal's mass in closed form (its centre shifted by
 // ln 10 sigma^2). No parameters in the reverse pass (imf_integral_dp has none for either): dlnT zero.
 __device__ inline void logn_setup(double A, double u0, double br, double c_hi, double lim_lo, double lim_hi,
-                                  KroupaSeg &k, float &inv_total, double *dlnT, double *total_out = nullptr) {
+                                  KroupaSeg &k, float &inv_total, double *dlnT) {
     const double s2 = 0.69 * 0.69, sig = 0.69, K = 2.302585092994046;
     double total = 0.0;
     // the lognormal's mass over [lim_lo, min(lim_hi, br)]: A e^(K u0 + K^2 sigma^2 / 2) K sigma sqrt(pi / 2)
@@ -295,7 +293,6 @@ __device__ inline void logn_setup(double A, double u0, double br, double c_hi, d
     k.e[2] = k.c[2] = k.ce[2] = 0.f;
     k.lo[2] = k.hi[2] = 1.0e30f;
     inv_total = total > 0.0 ? (float)(1.0 / total) : 1.f;
-    if (total_out) *total_out = total;
     k.generic = 1;
     k.logn = 1;
     k.la = (float)(A * K * sig * 1.4142135623730951);
